@@ -1433,11 +1433,12 @@ __global__ void __launch_bounds__(kNopivPanelThreads) panel_nopiv_kernel(int m, 
                                                                          int col, const int32_t* __restrict__ rowmap,
                                                                          int32_t* __restrict__ ipiv, int ipiv_base,
                                                                          int* __restrict__ info,
-                                                                         int* __restrict__ vflag, R_t<C> tau) {
+                                                                         int* __restrict__ vflag, R_t<C> tau,
+                                                                         int* __restrict__ arrived) {
   // D is one row taller than the block: the rotated reads D[j][j + c] stay inside
   __shared__ C D[kPanelNB + 1][kPanelNB + 1];
   __shared__ C rinv[kPanelNB], prow[kPanelNB];
-  __shared__ int zfirst, viol;
+  __shared__ int zfirst, viol, last;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if (tid == 0) {
     zfirst = INT_MAX;
@@ -1457,6 +1458,14 @@ __global__ void __launch_bounds__(kNopivPanelThreads) panel_nopiv_kernel(int m, 
     for (int c = 0; c < kPanelNB; ++c) x[c] = (row && c < w) ? row[c] : czero<C>();
   }
   __syncthreads();
+  // Every CTA needs the unfactored diagonal block, and not all CTAs need run
+  // at once: the factored block is written back by the CTA whose read of it
+  // was the last (it holds the same factors as every other), never before.
+  if (tid == 0) {
+    __threadfence();
+    last = atomicAdd(arrived, 1) == (int)gridDim.x - 1;
+    if (last) atomicExch(arrived, 0);  // for the next panel
+  }
   // Both parts keep the current column in register 0: every step shifts the
   // row left by one (updating the columns still open) and appends the new
   // multiplier, so register indices stay static in a rolled loop; after the
@@ -1525,7 +1534,7 @@ __global__ void __launch_bounds__(kNopivPanelThreads) panel_nopiv_kernel(int m, 
       if (c < w) row[c] = x[c];
     if (bad) viol = 1;
   }
-  if (blockIdx.x == 0) {
+  if (last) {  // (written before the __syncthreads between the two parts)
     for (int idx = tid; idx < w * w; idx += kNopivPanelThreads) {
       const int i = idx / w, c = idx % w;
       A[(long long)rowmap[i] * ld + col + c] = D[i][c];
@@ -1546,7 +1555,7 @@ static int panel_lu(const LaContext& ctx, int m, int w, C* A, long long ld, int 
     const int grid = max(1, ceil_div(m - w, kNopivPanelThreads));
     panel_nopiv_kernel<C><<<grid, kNopivPanelThreads, 0, ctx.stream>>>(m, w, A, ld, col, rowmap, ipiv, ipiv_base,
                                                                         ctx.dinfo, ctx.vflag,
-                                                                        (R_t<C>)ctx.pivot_tau);
+                                                                        (R_t<C>)ctx.pivot_tau, ctx.vflag + 1);
     BEM_LAUNCH_CHECK();
     count_launch();
     return BEM200_OK;
@@ -2355,7 +2364,7 @@ int getrf(const LaContext& ctx, int n, C* A, long long ld, int32_t* rowmap, int3
   LaContext c = ctx;
   c.vflag = reinterpret_cast<int*>(reinterpret_cast<char*>(scratch) +
                                    (((size_t)2 * n * sizeof(int32_t) + 255) & ~size_t(255)));
-  BEM_CUDA_CHECK(cudaMemsetAsync(c.vflag, 0, sizeof(int), ctx.stream));
+  BEM_CUDA_CHECK(cudaMemsetAsync(c.vflag, 0, 2 * sizeof(int), ctx.stream));  // the flag and the panels' arrival counter
   int st = getrf_dispatch<C>(c, n, A, ld, rowmap, ipiv, scratch);
   if (st) return st;
   nopiv_finish_kernel<<<1, 1, 0, ctx.stream>>>(c.vflag, ctx.dinfo);

@@ -335,6 +335,29 @@ def test_getrf_diagonal_pivots_report_needed_exchange(cuda, dt, where, off):
     assert int(info.item()) == -nat.ERR_PIVOTING
 
 
+@pytest.mark.parametrize("n", [1000, 5000])
+def test_getrf_diagonal_pivots_reproducible_beside_other_work(cuda, n):
+    """The checked no-pivot panels read the diagonal block in every CTA and one
+    CTA writes it back: with the GPU busy on another stream (so that the CTAs
+    of a panel do not all start at once) the factors stay bit-identical."""
+    import torch
+    A = torch.randn((n, n), dtype=torch.complex128, device="cuda", generator=torch.Generator("cuda").manual_seed(n))
+    A = A / n ** 0.5 + 4 * torch.eye(n, dtype=A.dtype, device="cuda")
+    ref = A.clone()
+    assert int(_getrf_ws(ref, 0, flags=4)[2].item()) == 0
+    load = torch.randn((4096, 4096), dtype=torch.float64, device="cuda")
+    side = torch.cuda.Stream()
+    for _ in range(3):
+        B = A.clone()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            for _ in range(6):
+                load @ load
+        assert int(_getrf_ws(B, 0, flags=4)[2].item()) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(torch.view_as_real(B), torch.view_as_real(ref))
+
+
 @pytest.mark.parametrize("dt", [np.complex128, np.complex64])
 def test_getrf_diagonal_pivots_zero_column(cuda, dt):
     """An all-zero column needs no exchange under partial pivoting either:
