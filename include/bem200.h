@@ -294,8 +294,8 @@ int bem200_getrs_noalloc(int dtype, int n, int nrhs, const void* LU, int64_t ld,
  * precision 1 = mixed: complex64 factors (GEMMs on `engine`) with FP64
  * residuals and iterative refinement (bem200_bem_solve_ir).
  * precision 2 = mixed with explicit complex64 inverses G1^-1, G2^-1,
- * Delta^-1, Sigma^-1 (block Schur complement without pivoting, each checked
- * by a probe M^-1 (M v) = v): every solve and refinement sweep is then a
+ * Delta^-1, Sigma^-1 (block Schur complement without pivoting, multipliers of
+ * at most 16 in the leaves, each checked by a probe M^-1 (M v) = v): every solve and refinement sweep is then a
  * few matrix products.  bem200_bem_init returns BEM200_ERR_PIVOTING when a
  * probe fails; write the slots again and initialise with precision 1.  The
  * same workspace serves precisions 1 and 2; pass the precision the
@@ -321,9 +321,15 @@ int bem200_bem_init(int precision, int engine, int n, void* ws, int eps_per_face
  * and the caller writes the slots again and repeats the call without the
  * flag), lookahead_nb the block width of the
  * look-ahead LU schedule (a multiple of 32 in [64, 1024]; 0 = 128).
+ * BEM200_INIT_REPAIR (with DIAGONAL_PIVOTS, precision 0 or 1, info_host given):
+ * when G1 and G2 passed their checks and only Delta or Sigma needs row
+ * exchanges, that part alone is built again with partial pivoting inside the
+ * call, which then returns BEM200_OK with *info_host = -BEM200_ERR_PIVOTING
+ * (the factors are partial pivoting's throughout).
  * phase_ms (HOST, 4 floats, or NULL): stage timer (CUDA events on the
  * stream; the call then synchronises): LU(G1) || LU(G2) with Sigma1 || Sigma2,
  * LU(Delta), Delta^-1, Sigma build + LU(Sigma). */
+#define BEM200_INIT_REPAIR 8
 int bem200_bem_init_ex(int precision, int engine, int n, void* ws, int eps_per_face, const double* eps1,
                        const double* eps2, const double* nvec, double k0, void* gemm_ws, size_t gemm_ws_bytes,
                        int lu_flags, int lookahead_nb, float* phase_ms, int32_t* info_host, void* stream);

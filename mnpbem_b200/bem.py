@@ -76,6 +76,7 @@ def _excitation_rhs(p, exc, enei):
 
 
 _DIAGONAL_PIVOTS = 4  # BEM200_GETRF_DIAGONAL_PIVOTS
+_REPAIR = 8           # BEM200_INIT_REPAIR
 
 
 class BEMRet:
@@ -210,12 +211,13 @@ class BEMRet:
             st = nat.lib().bem200_bem_init_ex(
                 cprec, _ENGINES[self.engine], n, nat.ptr(self._ws), self._eps_mode, self._e1p, self._e2p,
                 nat.ptr(self._nvec), self.k, nat.ptr(self._gws), self._gws_bytes,
-                0 if mode == "partial" else _DIAGONAL_PIVOTS, self._lookahead(), self._phase_buf,
+                0 if mode == "partial" else _DIAGONAL_PIVOTS | _REPAIR, self._lookahead(), self._phase_buf,
                 ctypes.byref(info), s)
             if st == nat.ERR_PIVOTING and mode != "partial":
                 continue  # a factor matrix needs row exchanges: the next, more general factorisation
             nat.check(st, "bem200_bem_init_ex")
-            self.last_pivoting = mode
+            # Delta or Sigma needed exchanges and was factored again inside the call
+            self.last_pivoting = "partial" if info.value == -nat.ERR_PIVOTING else mode
             self._cprec = cprec
             break
         if self._phase_buf is not None:

@@ -29,8 +29,9 @@ struct BemState {
   int32_t* ipiv[4];  // LAPACK swap sequences of the same factors
   int32_t* snap[2];  // look-ahead LU scratch (2 n row-map snapshots + grid-panel slots), one per chain
   C* dinv[6];        // diagonal-block inverses (L, U) of LU(G1), LU(G2), LU(Sigma) for the blocked solves
-  int* info;
+  int* info;      // verdict of the init: 0, first zero pivot, or -BEM200_ERR_*
   int* status;
+  int* verdict;   // the same of each factorisation: G1, G2, Delta, Sigma
 };
 
 static size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
@@ -67,6 +68,7 @@ static BemState<C> state_view(int n, void* ws) {
   }
   s.info = reinterpret_cast<int*>(p);
   s.status = s.info + 1;
+  s.verdict = s.info + 2;
   return s;
 }
 
@@ -119,10 +121,27 @@ __global__ void flag_to_info_kernel(const int* __restrict__ vflag, int* __restri
   if (*vflag) atomicExch(info, -BEM200_ERR_PIVOTING);
 }
 
+// info = the first verdict that is not 0, an unmet pivoting check before a zero pivot
+__global__ void verdict_kernel(const int* __restrict__ verdict, int* __restrict__ info) {
+  int v = 0;
+  for (int i = 0; i < 4; ++i) {
+    const int w = verdict[i];
+    if (w && (v == 0 || (w < 0 && v > 0))) v = w;
+  }
+  *info = v;
+}
+
 // probe tolerances of the complex64 inverses (relative to max|v|): the
 // factors only precondition the FP64 refinement
 constexpr double kDeltaProbeTol = 1e-2;
 constexpr double kInverseProbeTol = 1e-2;
+// Pivot threshold of the explicit inverses' leaves: multipliers up to this are
+// accepted.  The inverses only precondition the FP64 refinement and are
+// probe-checked, so threshold pivoting suffices: with 1 (partial pivoting's
+// choice) Sigma failed at most wavelengths of small meshes (1 - 5 exchanges),
+// and every failure costs the whole chain a second and third time
+// (1325-face rod: 40 ms instead of 8).
+constexpr float kInversePivotTau = 16.0f;
 
 // the verdict flag of a checked factorisation: the first int of the LU
 // scratch after its row-map snapshots (as getrf places it)
@@ -171,6 +190,51 @@ struct StageTimer {
   }
 };
 
+// Delta = Sigma1 - Sigma2 and Delta^-1
+template <typename C, typename Mark>
+static int delta_stage(const LaContext& ctx, int n, const BemState<C>& s, Mark mark) {
+  const long long nn = (long long)n * n;
+  LaContext c = ctx;
+  c.dinfo = s.verdict + 2;
+  int st;
+  if constexpr (sizeof(C) == 8) {
+    if (ctx.diag_pivots && inverse_nopiv_scratch_elems<C>(n) <= (size_t)n * n) {
+      // complex64 with checked diagonal pivots: Delta^-1 by the block Schur
+      // complement (GEMMs) instead of LU(Delta) + two n-column triangular
+      // solves; a failed probe raises the pivoting flag (-> partial pivoting)
+      int* vflag = lu_flag_of(s.snap[0], n);
+      BEM_CUDA_CHECK(cudaMemsetAsync(vflag, 0, sizeof(int), ctx.stream));
+      delta_kernel<C><<<ceil_div(nn, 256), 256, 0, ctx.stream>>>(nn, s.M[2], s.M[3], s.M[5]);
+      BEM_LAUNCH_CHECK();
+      if ((st = mark(2))) return st;
+      if ((st = inverse_nopiv<C>(c, n, s.M[5], n, s.M[4], vflag, kDeltaProbeTol))) return st;
+      flag_to_info_kernel<<<1, 1, 0, ctx.stream>>>(vflag, c.dinfo);
+      BEM_LAUNCH_CHECK();
+      return BEM200_OK;
+    }
+  }
+  delta_kernel<C><<<ceil_div(nn, 256), 256, 0, ctx.stream>>>(nn, s.M[2], s.M[3], s.M[4]);
+  BEM_LAUNCH_CHECK();
+  if ((st = getrf<C>(c, n, s.M[4], n, s.map[2], s.ipiv[2], s.snap[0]))) return st;
+  if ((st = mark(2))) return st;
+  return inverse<C>(c, n, s.M[4], n, s.map[2], s.M[5], n);
+}
+
+// Sigma and LU(Sigma)
+template <typename C>
+static int sigma_stage(const LaContext& ctx, int n, const BemState<C>& s, const EpsArg& eps, const double* nvec,
+                       double k0) {
+  const long long nn = (long long)n * n;
+  LaContext c = ctx;
+  c.dinfo = s.verdict + 3;
+  int st;
+  sigma_kernel<C><<<ceil_div(nn, 256), 256, 0, ctx.stream>>>(n, s.M[2], s.M[3], s.M[5], nvec, eps, k0 * k0, s.M[6]);
+  BEM_LAUNCH_CHECK();
+  if ((st = getrf<C>(c, n, s.M[6], n, s.map[3], s.ipiv[3], s.snap[0]))) return st;
+  if constexpr (sizeof(C) == 8) return trsv_diag_inverse<C>(c, n, s.M[6], n, s.map[3], s.dinv[4], s.dinv[5]);
+  return BEM200_OK;
+}
+
 template <typename C>
 static int bem_init_t(const LaContext& ctx, int n, void* ws, const EpsArg& eps, const double* nvec, double k0,
                       StageTimer* tm = nullptr, bool inv = false) {
@@ -181,9 +245,10 @@ static int bem_init_t(const LaContext& ctx, int n, void* ws, const EpsArg& eps, 
   };
   const long long nn = (long long)n * n;
   LaContext c = ctx;
-  c.dinfo = s.info;
+  c.dinfo = s.verdict;
   c.dstatus = s.status;
-  BEM_CUDA_CHECK(cudaMemsetAsync(s.info, 0, 2 * sizeof(int), ctx.stream));
+  if (inv) c.pivot_tau = kInversePivotTau;
+  BEM_CUDA_CHECK(cudaMemsetAsync(s.info, 0, 6 * sizeof(int), ctx.stream));
   int* vf[2] = {lu_flag_of(s.snap[0], n), lu_flag_of(s.snap[1], n)};  // verdicts of the checked factorisations
   BEM_CUDA_CHECK(cudaMemsetAsync(vf[0], 0, sizeof(int), ctx.stream));
   BEM_CUDA_CHECK(cudaMemsetAsync(vf[1], 0, sizeof(int), ctx.stream));
@@ -196,6 +261,7 @@ static int bem_init_t(const LaContext& ctx, int n, void* ws, const EpsArg& eps, 
   const bool fork = !split_ws || gemm_tc_workspace(n, half, half, ctx.engine) <= ctx.ws_bytes / 2;
   ForkJoin fj;
   LaContext c2 = c;
+  c2.dinfo = s.verdict + 1;
   if (fork) {
     BEM_CUDA_CHECK(cudaStreamCreateWithFlags(&fj.side, cudaStreamNonBlocking));
     BEM_CUDA_CHECK(cudaEventCreateWithFlags(&fj.fork, cudaEventDisableTiming));
@@ -228,8 +294,8 @@ static int bem_init_t(const LaContext& ctx, int n, void* ws, const EpsArg& eps, 
         BEM_CUDA_CHECK(cudaStreamWaitEvent(ctx.stream, fj.join, 0));
         c.ws_bytes = ctx.ws_bytes;
       }
-      flag_to_info_kernel<<<1, 1, 0, ctx.stream>>>(vf[0], s.info);
-      flag_to_info_kernel<<<1, 1, 0, ctx.stream>>>(vf[1], s.info);
+      flag_to_info_kernel<<<1, 1, 0, ctx.stream>>>(vf[0], s.verdict);
+      flag_to_info_kernel<<<1, 1, 0, ctx.stream>>>(vf[1], s.verdict + 1);
       BEM_LAUNCH_CHECK();
       if ((st = mark(1))) return st;
       BEM_CUDA_CHECK(cudaMemsetAsync(vf[0], 0, sizeof(int), ctx.stream));
@@ -242,7 +308,9 @@ static int bem_init_t(const LaContext& ctx, int n, void* ws, const EpsArg& eps, 
                                                                   s.M[6]);
       BEM_LAUNCH_CHECK();
       if ((st = inverse_nopiv<C>(c, n, s.M[6], n, s.M[4], vf[0], kInverseProbeTol))) return st;
-      flag_to_info_kernel<<<1, 1, 0, ctx.stream>>>(vf[0], s.info);
+      flag_to_info_kernel<<<1, 1, 0, ctx.stream>>>(vf[0], s.verdict + 3);
+      BEM_LAUNCH_CHECK();
+      verdict_kernel<<<1, 1, 0, ctx.stream>>>(s.verdict, s.info);
       BEM_LAUNCH_CHECK();
       return mark(4);
     }
@@ -263,40 +331,32 @@ static int bem_init_t(const LaContext& ctx, int n, void* ws, const EpsArg& eps, 
     c.ws_bytes = ctx.ws_bytes;
   }
   if ((st = mark(1))) return st;
-  // Delta = Sigma1 - Sigma2, Delta^-1
-  bool inverted = false;
-  if constexpr (sizeof(C) == 8) {
-    if (ctx.diag_pivots && inverse_nopiv_scratch_elems<C>(n) <= (size_t)n * n) {
-      // complex64 with checked diagonal pivots: Delta^-1 by the block Schur
-      // complement (GEMMs) instead of LU(Delta) + two n-column triangular
-      // solves; a failed probe raises the pivoting flag (-> partial pivoting)
-      int* vflag = vf[0];
-      BEM_CUDA_CHECK(cudaMemsetAsync(vflag, 0, sizeof(int), ctx.stream));
-      delta_kernel<C><<<ceil_div(nn, 256), 256, 0, ctx.stream>>>(nn, s.M[2], s.M[3], s.M[5]);
-      BEM_LAUNCH_CHECK();
-      if ((st = mark(2))) return st;
-      if ((st = inverse_nopiv<C>(c, n, s.M[5], n, s.M[4], vflag, kDeltaProbeTol))) return st;
-      flag_to_info_kernel<<<1, 1, 0, ctx.stream>>>(vflag, s.info);
-      BEM_LAUNCH_CHECK();
-      inverted = true;
-    }
-  }
-  if (!inverted) {
-    delta_kernel<C><<<ceil_div(nn, 256), 256, 0, ctx.stream>>>(nn, s.M[2], s.M[3], s.M[4]);
-    BEM_LAUNCH_CHECK();
-    if ((st = getrf<C>(c, n, s.M[4], n, s.map[2], s.ipiv[2], s.snap[0]))) return st;
-    if ((st = mark(2))) return st;
-    if ((st = inverse<C>(c, n, s.M[4], n, s.map[2], s.M[5], n))) return st;
-  }
+  if ((st = delta_stage<C>(c, n, s, mark))) return st;
   if ((st = mark(3))) return st;
-  // Sigma, LU(Sigma)
-  sigma_kernel<C><<<ceil_div(nn, 256), 256, 0, ctx.stream>>>(n, s.M[2], s.M[3], s.M[5], nvec, eps, k0 * k0, s.M[6]);
+  if ((st = sigma_stage<C>(c, n, s, eps, nvec, k0))) return st;
+  verdict_kernel<<<1, 1, 0, ctx.stream>>>(s.verdict, s.info);
   BEM_LAUNCH_CHECK();
-  if ((st = getrf<C>(c, n, s.M[6], n, s.map[3], s.ipiv[3], s.snap[0]))) return st;
-  if constexpr (sizeof(C) == 8) {
-    if ((st = trsv_diag_inverse<C>(c, n, s.M[6], n, s.map[3], s.dinv[4], s.dinv[5]))) return st;
-  }
   return mark(4);
+}
+
+// Delta (from `delta` on) or Sigma alone once more with partial pivoting, after
+// a checked factorisation without row exchanges failed there: the factors
+// before it passed their checks, so they are partial pivoting's already.
+template <typename C>
+static int bem_init_repair(const LaContext& ctx, int n, void* ws, const EpsArg& eps, const double* nvec, double k0,
+                           bool delta) {
+  BemState<C> s = state_view<C>(n, ws);
+  LaContext c = ctx;
+  c.dstatus = s.status;
+  c.diag_pivots = false;
+  int st;
+  const int first = delta ? 2 : 3;
+  BEM_CUDA_CHECK(cudaMemsetAsync(s.verdict + first, 0, (4 - first) * sizeof(int), ctx.stream));
+  if (delta && (st = delta_stage<C>(c, n, s, [](int) { return BEM200_OK; }))) return st;
+  if ((st = sigma_stage<C>(c, n, s, eps, nvec, k0))) return st;
+  verdict_kernel<<<1, 1, 0, ctx.stream>>>(s.verdict, s.info);
+  BEM_LAUNCH_CHECK();
+  return BEM200_OK;
 }
 
 // ------------------------------------------------------------ solve kernels
@@ -940,7 +1000,7 @@ int bem200_bem_init_ex(int precision, int engine, int n, void* ws, int eps_per_f
                        int lu_flags, int lookahead_nb, float* phase_ms, int32_t* info_host, void* stream) {
   BEM_REQUIRE(n > 0 && ws && eps1 && eps2 && nvec, BEM200_ERR_ARG, "bem_init: bad arguments");
   BEM_REQUIRE((lu_flags & ~(BEM200_GETRF_PARTIAL_PIVOTING | BEM200_GETRF_TOURNAMENT_PIVOTING |
-                             BEM200_GETRF_DIAGONAL_PIVOTS)) == 0,
+                             BEM200_GETRF_DIAGONAL_PIVOTS | BEM200_INIT_REPAIR)) == 0,
               BEM200_ERR_ARG, "bem_init: unknown LU flags 0x%x", lu_flags);
   BEM_REQUIRE(!((lu_flags & BEM200_GETRF_DIAGONAL_PIVOTS) && (lu_flags & BEM200_GETRF_TOURNAMENT_PIVOTING)),
               BEM200_ERR_ARG, "bem_init: diagonal and tournament pivoting exclude each other");
@@ -967,8 +1027,20 @@ int bem200_bem_init_ex(int precision, int engine, int n, void* ws, int eps_per_f
   }
   if (info_host) {
     int* dinfo = precision == 0 ? state_view<double2>(n, ws).info : state_view<float2>(n, ws).info;
-    BEM_CUDA_CHECK(cudaMemcpyAsync(info_host, dinfo, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
+    int h[6];  // info, status, verdicts of G1, G2, Delta, Sigma
+    BEM_CUDA_CHECK(cudaMemcpyAsync(h, dinfo, sizeof(h), cudaMemcpyDeviceToHost, ctx.stream));
     BEM_CUDA_CHECK(cudaStreamSynchronize(ctx.stream));
+    *info_host = h[0];
+    if ((lu_flags & BEM200_INIT_REPAIR) && precision != 2 && h[0] == -BEM200_ERR_PIVOTING && h[2] == 0 && h[3] == 0) {
+      const bool delta = h[4] != 0;
+      st = precision == 0 ? bem_init_repair<double2>(ctx, n, ws, eps, nvec, k0, delta)
+                          : bem_init_repair<float2>(ctx, n, ws, eps, nvec, k0, delta);
+      if (st) return st;
+      BEM_CUDA_CHECK(cudaMemcpyAsync(h, dinfo, sizeof(h), cudaMemcpyDeviceToHost, ctx.stream));
+      BEM_CUDA_CHECK(cudaStreamSynchronize(ctx.stream));
+      if (h[0] == 0) return BEM200_OK;  // *info_host = -BEM200_ERR_PIVOTING: repaired
+      *info_host = h[0];
+    }
     BEM_REQUIRE(*info_host != -BEM200_ERR_PIVOTING, BEM200_ERR_PIVOTING,
                 "bem_init: a factor matrix needs row exchanges (factor it with partial pivoting)");
     BEM_REQUIRE(*info_host != -BEM200_ERR_TIMEOUT, BEM200_ERR_TIMEOUT, "bem_init: a bounded device wait gave up");
