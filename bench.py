@@ -6,7 +6,7 @@ on x, water (eps = 1.77), Drude gold (9.84, 9.0 eV, 0.067 eV), plane wave
 polarised along x travelling along +z, wavelengths 650 + 0.05 s nm (step s).
 A step is one full solve: Green assembly (G1, G2, H1, H2), Sigma / Delta build
 with four LU factorisations, and the Eq. (19, 20) solve; with
---precision mixed the factors are complex64 (tcgen05 bf16x3 GEMMs) and the
+--precision mixed the factors are complex64 (tcgen05 int8 residue GEMMs) and the
 solution is refined against the complex128 operator to max-residual 1e-12.
 The one-time mesh precompute (refinement integrals) is excluded, as the metric
 prescribes.
@@ -318,11 +318,12 @@ def run_ours(args):
 
 
 def roofline_gemm(dev):
-    """Dominant tensor-core kernel: complex64 bf16x3 GEMM of the Sigma / LU
-    updates at the workload's top-level size (m = 5768, n = k = 2884), timed
-    with CUDA events on its own stream.  achieved = 8 m n k algorithmic flops
-    per launch / launch time; peak = measured dense bf16 (the tensor pipe runs 3
-    bf16 products per complex64 product, so frac <= 1/3 by construction)."""
+    """Dominant tensor-core product: the complex64 GEMM in residue arithmetic at
+    the workload's top-level size (m = 5768, n = k = 2884), timed with CUDA
+    events on its own stream.  achieved = 8 m n k algorithmic flops per product
+    / its time (operand split, int8 products, merge); peak = measured dense
+    bf16 (14 int8 products of 2 m n k operations each at twice the bf16 rate,
+    so frac <= 4/7 by construction)."""
     import ctypes
     import torch
     from mnpbem_b200 import _native as nat
@@ -358,12 +359,12 @@ def roofline_gemm(dev):
         peak_s, src_s = float(mp["bf16_tflops_sustained"]), "measured bf16 sustained"
     except Exception:
         pass
-    # DRAM bytes (read + write) of one launch of this GEMM from an ncu capture of the same shape
-    # (profiles/gemm_bf16x3_5768x2884x2884.md): 1.251 GB read + 0.139 GB written
-    traffic = 1.251e9 + 0.139e9
-    return {"kernel": "tc::gemm_bf16x3_kernel (+ operand prep)", "bound": "tensor", "achieved": round(achieved, 2),
+    # bytes the three kernels move once: operands read, 14 residue planes of A, B and C written and
+    # read, C written
+    traffic = 8.0 * (m * k + k * n + m * n) + 28.0 * (m * k + k * n + m * n)
+    return {"kernel": "rns_gemm_kernel (+ rns_split, rns_merge)", "bound": "tensor", "achieved": round(achieved, 2),
             "peak": peak, "peak_source": src, "unit": "TFLOP/s", "frac": round(achieved / peak, 4),
-            "traffic": traffic, "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, one launch",
+            "traffic": traffic, "traffic_source": "operand, residue-plane and result bytes, each written and read once",
             "algorithmic_flops_per_launch": 8.0 * m * n * k, "shape": [m, n, k], "ms_per_launch": round(1e3 * t, 3),
             "peak_sustained": peak_s, "peak_sustained_source": src_s}
 
@@ -371,7 +372,8 @@ def roofline_gemm(dev):
 def fp64_peak(dev):
     """FP64 yardstick of this GPU: cuBLAS DGEMM (torch.matmul, 4096^3) timed
     with CUDA events -- the denominator of the FP64 path's roofline fraction
-    (the FP64 path runs its complex128 GEMMs on CUDA cores)."""
+    (the large complex128 products run on the int8 tensor cores, so the
+    fraction can pass 1)."""
     import torch
     n = 4096
     A = torch.randn(n, n, dtype=torch.float64, device=dev)

@@ -7,7 +7,8 @@ Everything per wavelength runs in libbem200 on the GPU:
 * ``precision='fp64'`` (default): complex128 assembly, LU factors, Sigma /
   Delta build and the Eq. (19, 20) solve -- the drop-in path;
 * ``precision='mixed'``: complex64 factors built with tcgen05 tensor-core
-  GEMMs (``engine='bf16x3'``; ``'simt'`` uses CUDA cores),
+  GEMMs (``engine='bf16x3'``, the name of an earlier operand split, runs
+  the int8 residue products; ``'simt'`` uses CUDA cores),
   then iterative refinement against the complex128 BEM operator until the
   max-norm residual drops below ``ir_tol`` times the right-hand side.
   Refinement whose sweeps stop contracting (the contraction rate of
@@ -155,9 +156,9 @@ class BEMRet:
         slots = [ctypes.c_void_p() for _ in range(4)]
         nat.call("bem200_bem_slots", prec, n, nat.ptr(self._ws), *[ctypes.byref(s) for s in slots])
         self._slots = [s.value for s in slots]
-        # operand space of the largest GEMM plus headroom for the concurrent
-        # halves of the factor chains (each needs about a quarter of it)
-        gbytes = int(L.bem200_gemm_workspace_size(_ENGINES[self.engine], n, n, n) * 5 // 4)
+        # operand space of the largest GEMM for each of the two factor chains
+        # that run beside each other
+        gbytes = int(L.bem200_gemm_workspace_size(_ENGINES[self.engine], n, n, n) * 2)
         self._gws = torch.empty(max(gbytes, 1), dtype=torch.uint8, device=self.dev)
         self._gws_bytes = gbytes
         if prec == 1:

@@ -17,7 +17,7 @@ BUILD = os.path.join(HERE, "_build")
 LIBDIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIBDIR, "libbem200.so")
 
-SOURCES = ["green.cu", "dense.cu", "gemm_tc.cu", "bem.cu", "krylov.cu", "hmat.cu", "planewave.cu", "field.cu",
+SOURCES = ["green.cu", "dense.cu", "gemm_rns.cu", "bem.cu", "krylov.cu", "hmat.cu", "planewave.cu", "field.cu",
            "adjoint.cu", "noalloc.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",

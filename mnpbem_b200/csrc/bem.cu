@@ -32,16 +32,27 @@ struct BemState {
   int* info;      // verdict of the init: 0, first zero pivot, or -BEM200_ERR_*
   int* status;
   int* verdict;   // the same of each factorisation: G1, G2, Delta, Sigma
+  void* gws;         // complex128: operand space of the tensor-core products of the init
+  size_t gws_bytes;
 };
 
 static size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
+
+// complex128 operand space: the two factor chains of the init run
+// concurrently and each solves two halves of its right-hand sides at a time
+template <typename C>
+static size_t state_operand_bytes(int n) {
+  if (sizeof(C) == 8) return 0;  // the caller's GEMM workspace
+  const int half = n / 2 + 64;
+  return align256(4 * gemm_tc_workspace<C>(n, half, half, GemmEngine::kTc) + 4096);
+}
 
 template <typename C>
 static size_t state_bytes(int n) {
   size_t mat = align256(sizeof(C) * (size_t)n * n);
   return kSlots * mat + 8 * align256(sizeof(int32_t) * n) +
          2 * (align256(sizeof(int32_t) * 2 * (size_t)n) + kPanelGridScratch) + 6 * align256(trsv_diag_inverse_bytes<C>(n)) +
-         256;
+         256 + state_operand_bytes<C>(n);
 }
 
 template <typename C>
@@ -69,6 +80,8 @@ static BemState<C> state_view(int n, void* ws) {
   s.info = reinterpret_cast<int*>(p);
   s.status = s.info + 1;
   s.verdict = s.info + 2;
+  s.gws = p + 256;
+  s.gws_bytes = state_operand_bytes<C>(n);
   return s;
 }
 
@@ -147,22 +160,6 @@ constexpr float kInversePivotTau = 16.0f;
 // scratch after its row-map snapshots (as getrf places it)
 static int* lu_flag_of(int32_t* snap, int n) {
   return reinterpret_cast<int*>(reinterpret_cast<char*>(snap) + align256(sizeof(int32_t) * 2 * (size_t)n));
-}
-
-// Out = A B (m x k times k x n, dense row-major), split along k into slices
-// whose tensor-core operand planes fit ctx's workspace
-template <typename C>
-static int gemm_fit(const LaContext& ctx, int m, int n, int k, const C* A, const C* B, C* Out) {
-  int kc = k;
-  if (ctx.engine != GemmEngine::kSimt)
-    while (kc > 64 && gemm_tc_workspace(m, n, kc, ctx.engine) > ctx.ws_bytes) kc = ((kc / 2 + 63) / 64) * 64;
-  const C one = cmake<C>(1.0, 0.0), zero = czero<C>();
-  for (int k0 = 0; k0 < k; k0 += kc) {
-    const int kk = min(kc, k - k0);
-    const int st = gemm<C>(ctx, m, n, kk, one, A + k0, k, B + (long long)k0 * n, n, k0 ? one : zero, Out, n);
-    if (st) return st;
-  }
-  return BEM200_OK;
 }
 
 // The factor chains of G1 and G2 are independent: LU(G2) and Sigma2 run on a
@@ -258,7 +255,7 @@ static int bem_init_t(const LaContext& ctx, int n, void* ws, const EpsArg& eps, 
   // an LU / right solve (n x n/2 x n/2, rounded up)
   const int half = n / 2 + 64;
   const bool split_ws = ctx.engine != GemmEngine::kSimt;
-  const bool fork = !split_ws || gemm_tc_workspace(n, half, half, ctx.engine) <= ctx.ws_bytes / 2;
+  const bool fork = gemm_tc_two_fit<C>(ctx, n, half, half);
   ForkJoin fj;
   LaContext c2 = c;
   c2.dinfo = s.verdict + 1;
@@ -276,6 +273,7 @@ static int bem_init_t(const LaContext& ctx, int n, void* ws, const EpsArg& eps, 
       c2.ws_bytes = h;
     }
   }
+  const C one = cmake<C>(1.0, 0.0), zero = czero<C>();
   if constexpr (sizeof(C) == 8) {
     if (inv) {
       // explicit inverses (complex64): G1^-1 || G2^-1 by the block Schur
@@ -284,10 +282,10 @@ static int bem_init_t(const LaContext& ctx, int n, void* ws, const EpsArg& eps, 
       BEM_REQUIRE(inverse_nopiv_scratch_elems<C>(n) <= (size_t)n * n, BEM200_ERR_UNSUPPORTED,
                   "bem_init: the inverse's scratch does not fit a slot");
       if ((st = inverse_nopiv<C>(c, n, s.M[0], n, s.M[4], vf[0], kInverseProbeTol))) return st;
-      if ((st = gemm_fit<C>(c, n, n, n, s.M[2], s.M[0], s.M[4]))) return st;
+      if ((st = gemm<C>(c, n, n, n, one, s.M[2], n, s.M[0], n, zero, s.M[4], n))) return st;
       BEM_CUDA_CHECK(cudaMemcpyAsync(s.M[2], s.M[4], sizeof(C) * nn, cudaMemcpyDeviceToDevice, c.stream));
       if ((st = inverse_nopiv<C>(c2, n, s.M[1], n, s.M[5], vf[1], kInverseProbeTol))) return st;
-      if ((st = gemm_fit<C>(c2, n, n, n, s.M[3], s.M[1], s.M[5]))) return st;
+      if ((st = gemm<C>(c2, n, n, n, one, s.M[3], n, s.M[1], n, zero, s.M[5], n))) return st;
       BEM_CUDA_CHECK(cudaMemcpyAsync(s.M[3], s.M[5], sizeof(C) * nn, cudaMemcpyDeviceToDevice, c2.stream));
       if (fork) {  // (without a second chain, c2 is c: same stream, whole workspace)
         BEM_CUDA_CHECK(cudaEventRecord(fj.join, fj.side));
@@ -352,7 +350,7 @@ static int bem_init_repair(const LaContext& ctx, int n, void* ws, const EpsArg& 
   int st;
   const int first = delta ? 2 : 3;
   BEM_CUDA_CHECK(cudaMemsetAsync(s.verdict + first, 0, (4 - first) * sizeof(int), ctx.stream));
-  if (delta && (st = delta_stage<C>(c, n, s, [](int) { return BEM200_OK; }))) return st;
+  if (delta && (st = delta_stage<C>(c, n, s, [](int) -> int { return BEM200_OK; }))) return st;
   if ((st = sigma_stage<C>(c, n, s, eps, nvec, k0))) return st;
   verdict_kernel<<<1, 1, 0, ctx.stream>>>(s.verdict, s.info);
   BEM_LAUNCH_CHECK();
@@ -974,7 +972,7 @@ static EpsArg make_eps(int per_face, const double* e1, const double* e2) {
 }
 
 static GemmEngine engine_from(int e) {
-  return e == 1 ? GemmEngine::kTcBf16x3 : (e == 2 ? GemmEngine::kTcTf32 : GemmEngine::kSimt);
+  return e == 1 ? GemmEngine::kTc : (e == 2 ? GemmEngine::kTf32 : GemmEngine::kSimt);
 }
 
 extern "C" {
@@ -1013,6 +1011,12 @@ int bem200_bem_init_ex(int precision, int engine, int n, void* ws, int eps_per_f
   ctx.diag_pivots = (lu_flags & BEM200_GETRF_DIAGONAL_PIVOTS) != 0;
   ctx.la_nb = lookahead_nb;
   EpsArg eps = make_eps(eps_per_face, eps1, eps2);
+  if (precision == 0) {  // complex128 products: the operand space of the workspace itself
+    const BemState<double2> s = state_view<double2>(n, ws);
+    ctx.engine = GemmEngine::kTc;
+    ctx.ws = s.gws;
+    ctx.ws_bytes = s.gws_bytes;
+  }
   StageTimer tm;
   if (phase_ms)
     for (cudaEvent_t& e : tm.ev) BEM_CUDA_CHECK(cudaEventCreate(&e));

@@ -214,18 +214,22 @@ static int gemm_skinny(const LaContext& ctx, int m, int n, int k, C alpha, RowVi
   return BEM200_OK;
 }
 
-constexpr double kTcMinMacs = 67108864.0;  // 2^26
-
 // Whether gemm_v runs an m x n x k product on the tensor cores (the only path
-// that uses the operand workspace ctx.ws).  The tensor-core path pays ~25 us of
-// operand preparation, pipeline fill and launches per call: below ~2^26
-// multiply-adds (about 400^3) the CUDA-core tiles finish first.
+// that uses the operand workspace ctx.ws).  That path pays three launches and
+// 2 N residue bytes written and read per entry of C whatever k is.  Measured
+// against the CUDA-core tiles: complex64 360^3 23 vs 24 us, 512^3 30 vs 44 us
+// (from 2^26 multiply-adds), but with k = 128 only the large updates gain
+// (5768 x 5768 x 128: 451 vs 751 us; updates of 1500 rows slow a sweep on four
+// streams by 4 %); complex128 256^3 25 vs 23 us, 360^3 33 vs 38 us,
+// 5768 x 5768 x 128 1140 vs 1780 us.
 template <typename C>
 static bool gemm_takes_tc(const LaContext& ctx, int m, int n, int k) {
   if (m <= 0 || n <= 0 || (n <= 16 && k >= 256)) return false;  // empty, or the skinny path
-  if constexpr (sizeof(C) == 8)
-    return ctx.engine != GemmEngine::kSimt && k >= 64 && m >= 128 && n >= 64 && (double)m * n * k >= kTcMinMacs;
-  return false;
+  if (ctx.engine == GemmEngine::kSimt || k < 64 || m < 64 || n < 64) return false;
+  const double macs = (double)m * n * k;
+  if (sizeof(C) == 16)  // without room for the operands: CUDA cores
+    return ctx.engine == GemmEngine::kTc && macs >= 33554432.0 && gemm_tc_fits<C>(ctx, m, n, k);
+  return macs >= (k >= 256 ? 67108864.0 : 1073741824.0);
 }
 
 template <typename C>
@@ -239,9 +243,7 @@ int gemm_v(const LaContext& ctx, int m, int n, int k, C alpha, RowView<C> A, Row
     if (n <= 8) return gemm_skinny<C, 8, z ? 1 : 2>(ctx, m, n, k, alpha, A, B, beta, Cv);
     return gemm_skinny<C, 16, 1>(ctx, m, n, k, alpha, A, B, beta, Cv);
   }
-  if constexpr (sizeof(C) == 8) {
-    if (gemm_takes_tc<C>(ctx, m, n, k)) return gemm_tc_c64(ctx, m, n, k, alpha, A, B, beta, Cv);
-  }
+  if (gemm_takes_tc<C>(ctx, m, n, k)) return gemm_tc<C>(ctx, m, n, k, alpha, A, B, beta, Cv);
   constexpr int BK = sizeof(C) == 16 ? 8 : 16;
   if ((long long)ceil_div(n, 32) * ceil_div(m, 32) < 74) {  // 32 x 32 tiles would fill fewer than half the SMs
     dim3 grid(ceil_div(n, 16), ceil_div(m, 16));
@@ -2377,9 +2379,11 @@ static int getrf_dispatch(const LaContext& ctx, int n, C* A, long long ld, int32
                           int32_t* scratch) {
   // look-ahead needs the row-map snapshots (scratch) and, on the tensor-core
   // engines, room for two concurrent GEMMs in the operand workspace
-  const bool ws_ok = ctx.engine == GemmEngine::kSimt ||
-                     gemm_tc_workspace(n, n, la_width(ctx), ctx.engine) <= ((ctx.ws_bytes / 2) & ~size_t(255));
-  if (scratch && n > 2 * la_width(ctx) && ws_ok) return getrf_lookahead<C>(ctx, n, A, ld, rowmap, ipiv, scratch);
+  const bool ws_ok = gemm_tc_two_fit<C>(ctx, n, n, la_width(ctx));
+  // (complex64 panels and updates below n = 512 are so short that the two
+  // streams' events cost more than the overlap gains: 7.7 vs 7.0 ms for the
+  // fallback chain of a 284-face solve)
+  if (scratch && n > max(2 * la_width(ctx), sizeof(C) == 8 ? 512 : 0) && ws_ok) return getrf_lookahead<C>(ctx, n, A, ld, rowmap, ipiv, scratch);
   iota_kernel<<<ceil_div(n, 256), 256, 0, ctx.stream>>>(n, rowmap);
   BEM_LAUNCH_CHECK();
   return getrf_rec(ctx, n, A, ld, rowmap, ipiv, 0, n);
@@ -2568,8 +2572,7 @@ template <typename C>
 int solve_right(const LaContext& ctx, int n, int m, const C* LU, long long ld, const int32_t* rowmap, C* X,
                 long long ldx, C* tmp) {
   const int h = m / 2;
-  const bool split = m >= 1024 && (ctx.engine == GemmEngine::kSimt ||
-                                   gemm_tc_workspace(m - h, n / 2 + 64, n / 2 + 64, ctx.engine) <= ctx.ws_bytes / 2);
+  const bool split = m >= 1024 && gemm_tc_two_fit<C>(ctx, m - h, n / 2 + 64, n / 2 + 64);
   if (!split) return solve_right_rows<C>(ctx, n, m, LU, ld, rowmap, X, ldx, tmp);
   LaContext c1 = ctx, c2;
   SideStream ss;
@@ -2617,8 +2620,7 @@ int inverse(const LaContext& ctx, int n, const C* LU, long long ld, const int32_
   // the columns of the inverse are independent: with enough workspace the
   // second half of them is solved on a forked stream
   const int h = n / 2;
-  const bool split = n >= 1024 && (ctx.engine == GemmEngine::kSimt ||
-                                   gemm_tc_workspace(n, n - h + 64, n, ctx.engine) <= ctx.ws_bytes / 2);
+  const bool split = n >= 1024 && gemm_tc_two_fit<C>(ctx, n, n - h + 64, n);
   if (!split) {
     int st = trsm_llu<C>(ctx, n, n, T, plain(Inv, ldi));
     if (st) return st;
@@ -3079,7 +3081,7 @@ BEM_INST(float2)
 using namespace bem200;
 
 static GemmEngine engine_of(int e) {
-  return e == 1 ? GemmEngine::kTcBf16x3 : (e == 2 ? GemmEngine::kTcTf32 : GemmEngine::kSimt);
+  return e == 1 ? GemmEngine::kTc : (e == 2 ? GemmEngine::kTf32 : GemmEngine::kSimt);
 }
 
 extern "C" {
@@ -3104,7 +3106,7 @@ int bem200_gemm(int dtype, int engine, int m, int n, int k, const double* alpha,
 }
 
 size_t bem200_gemm_workspace_size(int engine, int m, int n, int k) {
-  return gemm_tc_workspace(m, n, k, engine_of(engine));
+  return gemm_tc_workspace<float2>(m, n, k, engine_of(engine));
 }
 
 // ws layout for getrf: [tensor-core operand space | 2 n int32 row-map snapshots]
@@ -3112,10 +3114,17 @@ static size_t getrf_snap_bytes(int n) {
   return (((size_t)2 * n * sizeof(int32_t) + 255) & ~size_t(255)) + kPanelGridScratch;
 }
 
+// operand space of getrf: complex64 for any product of the factorisation,
+// complex128 for the two concurrent updates of the look-ahead schedule
+static size_t getrf_operand_bytes(int dtype, int engine, int n) {
+  const size_t b = dtype == BEM200_C128 ? 2 * gemm_tc_workspace<double2>(n, n, min(n, 512), GemmEngine::kTc) + 512
+                                        : gemm_tc_workspace<float2>(n, n, n, engine_of(engine));
+  return (b + 255) & ~size_t(255);
+}
+
 size_t bem200_getrf_workspace_size(int dtype, int engine, int n) {
-  (void)dtype;
   if (n <= 0) return 0;
-  return ((gemm_tc_workspace(n, n, n, engine_of(engine)) + 255) & ~size_t(255)) + getrf_snap_bytes(n);
+  return getrf_operand_bytes(dtype, engine, n) + getrf_snap_bytes(n);
 }
 
 int bem200_getrf_ex(int dtype, int engine, int n, void* A, int64_t ld, int32_t* rowmap, int32_t* ipiv, int32_t* info,
@@ -3135,11 +3144,15 @@ int bem200_getrf_ex(int dtype, int engine, int n, void* A, int64_t ld, int32_t* 
   ctx.diag_pivots = (flags & BEM200_GETRF_DIAGONAL_PIVOTS) != 0;
   ctx.la_nb = lookahead_nb;
   int32_t* snap = nullptr;
-  if (ws && n > 0 && ws_bytes >= bem200_getrf_workspace_size(dtype, engine, n)) {
-    const size_t sb = getrf_snap_bytes(n);
+  // complex128 needs only the snapshots for the look-ahead schedule; its
+  // products go to the tensor cores when the operand space is there too
+  const bool z = dtype == BEM200_C128;
+  const size_t sb = n > 0 ? getrf_snap_bytes(n) : 0;
+  if (ws && n > 0 && ws_bytes >= (z ? sb : bem200_getrf_workspace_size(dtype, engine, n))) {
     ctx.ws_bytes = (ws_bytes - sb) & ~size_t(255);
     snap = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(ws) + ctx.ws_bytes);
   }
+  if (z) ctx.engine = snap && ctx.ws_bytes >= getrf_operand_bytes(dtype, engine, n) ? GemmEngine::kTc : GemmEngine::kSimt;
   if (dtype == BEM200_C128) return getrf<double2>(ctx, n, (double2*)A, ld, rowmap, ipiv, snap);
   if (dtype == BEM200_C64) return getrf<float2>(ctx, n, (float2*)A, ld, rowmap, ipiv, snap);
   set_error("getrf: bad dtype %d", dtype);

@@ -11,17 +11,17 @@
 //   inverse      : A^-1
 //   gemm         : C <- alpha A B + beta C on row views
 // Element types: double2 (complex128, FP64 arithmetic) and float2 (complex64).
-// The complex64 GEMM runs on tcgen05 tensor cores when a tensor-core engine
-// is selected (gemm_tc.cu), otherwise on CUDA cores.
+// Large GEMMs run on the tcgen05 tensor cores when that engine is selected
+// and a workspace is at hand (gemm_rns.cu), otherwise on CUDA cores.
 #pragma once
 #include "common.cuh"
 
 namespace bem200 {
 
 enum class GemmEngine : int {
-  kSimt = 0,      // CUDA-core FMA (FP64 for complex128, FP32 for complex64)
-  kTcBf16x3 = 1,  // complex64 on tcgen05: bf16 hi/lo split, 3 products, FP32 accumulate
-  kTcTf32 = 2,    // reserved (complex64 on tcgen05 with TF32 inputs): not built, rejected by gemm_tc_c64
+  kSimt = 0,  // CUDA-core FMA (FP64 for complex128, FP32 for complex64)
+  kTc = 1,    // large products on the int8 tensor cores (residue arithmetic, gemm_rns.cu)
+  kTf32 = 2,  // reserved (complex64 on tcgen05 with TF32 inputs): not built, rejected by gemm_tc
 };
 
 // Row-addressed matrix view: element (i, j) lives at
@@ -176,9 +176,23 @@ size_t inverse_nopiv_scratch_elems(int n);
 template <typename C>
 int inverse_nopiv(const LaContext& ctx, int n, C* M, long long ld, C* ws, int* vflag, double tol);
 
-// bytes of scratch the tensor-core GEMM needs for an m x n x k product
+// Tensor-core product (gemm_rns.cu).  gemm_tc_workspace: bytes for one pass
+// of an m x n x k product (blocks of at most 6144 (complex64) or 3072
+// (complex128) per extent); a smaller ctx.ws is used in smaller blocks,
+// gemm_tc_fits tells whether any fit.
+template <typename C>
 size_t gemm_tc_workspace(int m, int n, int k, GemmEngine e);
-int gemm_tc_c64(const LaContext& ctx, int m, int n, int k, float2 alpha, RowView<float2> A, RowView<float2> B,
-                float2 beta, RowView<float2> Cv);
+template <typename C>
+bool gemm_tc_fits(const LaContext& ctx, int m, int n, int k);
+// Whether two chains of products up to m x n x k may run beside each other in
+// the two halves of ctx.ws: a half holds at least two thirds of one pass (the
+// product then runs in two or three blocks, whose repeated operand splits cost
+// less than serialising the chains).
+template <typename C>
+bool gemm_tc_two_fit(const LaContext& ctx, int m, int n, int k) {
+  return ctx.engine == GemmEngine::kSimt || gemm_tc_workspace<C>(m, n, k, ctx.engine) / 4 <= ctx.ws_bytes / 3;
+}
+template <typename C>
+int gemm_tc(const LaContext& ctx, int m, int n, int k, C alpha, RowView<C> A, RowView<C> B, C beta, RowView<C> Cv);
 
 }  // namespace bem200
