@@ -427,7 +427,7 @@ int bem200_bem_apply_T(int n, int npol, const void* G1, const void* G2, const vo
  * 4.  Far pairs are differentiated analytically and swept by rows and by
  * columns without storing any n x n matrix; refined pairs through their
  * phase, normals and coefficients, whose derivatives with respect to the
- * face nodes and the observation frame are exact (forward-mode dual numbers
+ * face nodes and the observation frame are exact (reverse mode
  * over the refinement quadrature); the closed-surface correction is chained
  * through its column sums.  Inputs: the assembly tables of
  * bem200_green_assemble (pid, blk_mat, kmat_host), the refinement inputs of

@@ -18,7 +18,7 @@
 //   phi(d) = (ik - 1/d) e^{ikd} / d^2,  phi'(d) = e^{ikd} / d^2 (3/d^2 - 3ik/d - k^2)
 // refined pairs: G = sum_m g_m (ik)^m e^{ikd}, Gp = sum_m f_m (ik)^m e^{ikd},
 // whose coefficients g, f depend on the face nodes through the refinement
-// quadrature: their derivatives are exact (dual numbers, dual.cuh).
+// quadrature: their derivatives are exact (reverse mode through the quadrature).
 //
 // Nothing n x n (x 3) is stored: the far pairs are swept by one warp per row
 // (row-side gradients: pos_i, nvec_i) and one warp per column (pos_j, area_j),
@@ -27,7 +27,7 @@
 // Output: complex cotangents (c = sum of lambda^T dA x contributions) for
 // pos (n, 3), nvec (n, 3), area (n), tvec1 (n, 3), tvec2 (n, 3) and the face
 // nodes (n, 9, 3); the caller chains them to the vertices.
-#include "dual.cuh"
+#include "common.cuh"
 #include "green_entry.cuh"
 
 namespace bem200 {
@@ -485,161 +485,322 @@ __global__ void refined_closed_kernel(Args A) {
 
 // ------------------------------------------------------------ refinement coefficients
 // Derivatives of the refinement coefficients g_m, f_cm of entry e with respect
-// to its inputs, contracted with their cotangents: one warp per entry, one
-// dual-number evaluation of the entry's quadrature per input coordinate.
-// Inputs: self terms (kind 2): pos_i, n_i, t1_i, t2_i and the nodes of face
-// j; others: pos_i, pos_j and the nodes of face j.
-using ad::Dual;
-using ad::V3;
+// to its inputs, contracted with their cotangents: reverse mode through the
+// refinement quadrature (the reference's _refine_diagonal / _refine_offdiagonal,
+// mnpbem/greenfun/greenret_refined.py:122-516, with the rules of
+// refine_integrals_kernel in green.cu).  Inputs: self terms (kind 2): pos_i, n_i,
+// t1_i, t2_i and the nodes of face j; others: pos_i, pos_j and the nodes of
+// face j.
+//
+// A quadrature point x = sum_c N_c node_c has the weight wf |px x py|, px and
+// py the sums with the derivatives Dx_c, Dy_c of its shape functions (flat
+// triangles: the two edges).  Its contribution to the contraction is w phi(v, ..),
+// v = pos_i - x; the point's cotangents are -w dphi/dv for x and phi wf times the
+// gradient of |px x py| for px, py.
+//
+// One warp per entry, one point per lane; the points' cotangents and shape
+// functions go through shared memory, and lane 3 c + x then sums node c's
+// component x over the points.  One evaluation of the quadrature replaces one
+// dual-number evaluation per input coordinate (24 - 39 of them): FP64 bound.
+constexpr int kPtVals = 18;    // complex cotangents of x, px, py
+constexpr int kPtBasis = 27;   // N, Dx, Dy of up to 9 nodes
+constexpr int kCoefWarps = 4;
 
-template <typename T>
-__device__ __forceinline__ T wsumT(T v);
-template <>
-__device__ __forceinline__ Dual wsumT<Dual>(Dual v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v.v += __shfl_xor_sync(0xffffffffu, v.v, o);
-    v.d += __shfl_xor_sync(0xffffffffu, v.d, o);
-  }
-  return v;
+struct Vec { double x, y, z; };
+__device__ __forceinline__ Vec vsub(Vec a, Vec b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
+__device__ __forceinline__ Vec vcross(Vec a, Vec b) {
+  return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
+__device__ __forceinline__ double vdot(Vec a, Vec b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ Vec vload(const double* p) { return {p[0], p[1], p[2]}; }
+__device__ __forceinline__ double2 cfma(double2 a, double s, double2 c) {
+  return make_double2(fma(a.x, s, c.x), fma(a.y, s, c.y));
+}
+
+// node of the face behind shape function c of the current (sub-)element
+__device__ __forceinline__ int sub_node(int fk, bool self, int s, int c) {
+  if (self || fk == 0 || fk == 2) return c;
+  if (fk == 1) return c == 0 ? 0 : c + s;                 // flat quad: triangles 0 1 2 and 0 2 3
+  const unsigned m = s == 0 ? 0x854210u : 0x876032u;      // curved quad: 0 1 2 4 5 8 and 2 3 0 6 7 8
+  return (m >> (4 * c)) & 15;
+}
+
+// shape functions at rule point q: number of nodes, weight factor; B[3 c .. 3 c + 2] = N, Dx, Dy
+__device__ __forceinline__ double shape_at(const Args& A, int fk, bool self, int q, double* B, int stride) {
+  const double* x3 = A.rules + 3 * A.n28;
+  const double* x4 = x3 + 3 * A.n3;
+  auto put = [&](int c, double N, double Dx, double Dy) {
+    B[(3 * c) * stride] = N;
+    B[(3 * c + 1) * stride] = Dx;
+    B[(3 * c + 2) * stride] = Dy;
+  };
+  if (self && (fk == 1 || fk == 3)) {
+    const double x = x4[q], y = x4[A.n4 + q], w = x4[2 * A.n4 + q];
+    if (fk == 1) {
+      put(0, 0.25 * (1 - x) * (1 - y), -0.25 * (1 - y), -0.25 * (1 - x));
+      put(1, 0.25 * (1 + x) * (1 - y), 0.25 * (1 - y), -0.25 * (1 + x));
+      put(2, 0.25 * (1 + x) * (1 + y), 0.25 * (1 + y), 0.25 * (1 + x));
+      put(3, 0.25 * (1 - x) * (1 + y), -0.25 * (1 + y), 0.25 * (1 - x));
+    } else {
+      put(0, 0.25 * x * (x - 1) * y * (y - 1), 0.25 * (2 * x - 1) * y * (y - 1), 0.25 * x * (x - 1) * (2 * y - 1));
+      put(1, 0.25 * x * (x + 1) * y * (y - 1), 0.25 * (2 * x + 1) * y * (y - 1), 0.25 * x * (x + 1) * (2 * y - 1));
+      put(2, 0.25 * x * (x + 1) * y * (y + 1), 0.25 * (2 * x + 1) * y * (y + 1), 0.25 * x * (x + 1) * (2 * y + 1));
+      put(3, 0.25 * x * (x - 1) * y * (y + 1), 0.25 * (2 * x - 1) * y * (y + 1), 0.25 * x * (x - 1) * (2 * y + 1));
+      put(4, 0.5 * (1 - x * x) * y * (y - 1), -x * y * (y - 1), 0.5 * (1 - x * x) * (2 * y - 1));
+      put(5, 0.5 * x * (x + 1) * (1 - y * y), 0.5 * (2 * x + 1) * (1 - y * y), -x * (x + 1) * y);
+      put(6, 0.5 * (1 - x * x) * y * (y + 1), -x * y * (y + 1), 0.5 * (1 - x * x) * (2 * y + 1));
+      put(7, 0.5 * x * (x - 1) * (1 - y * y), 0.5 * (2 * x - 1) * (1 - y * y), -x * (x - 1) * y);
+      put(8, (1 - x * x) * (1 - y * y), -2 * x * (1 - y * y), -2 * (1 - x * x) * y);
+    }
+    return w;
+  }
+  const double* r = self ? x3 : A.rules;
+  const int np = self ? A.n3 : A.n28;
+  const double x = r[q], y = r[np + q], z = 1.0 - x - y;
+  double w = 0.5 * r[2 * np + q];
+  if (fk >= 2) {
+    put(0, x * (2 * x - 1), 4 * x - 1, 0.0);
+    put(1, y * (2 * y - 1), 0.0, 4 * y - 1);
+    put(2, z * (2 * z - 1), -4 * z + 1, -4 * z + 1);
+    put(3, 4 * x * y, 4 * y, 4 * x);
+    put(4, 4 * y * z, -4 * y, 4 * (z - y));
+    put(5, 4 * z * x, 4 * (z - x), -4 * x);
+  } else {
+    put(0, x, -1.0, -1.0);
+    put(1, y, 1.0, 0.0);
+    put(2, z, 0.0, 1.0);
+  }
+  return w;
+}
+
 __device__ __forceinline__ double wmax(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
 
-__device__ __forceinline__ V3<Dual> seed3(const double* p, int dir, int first) {
-  V3<Dual> v = ad::mk3<Dual>(Dual(p[0]), Dual(p[1]), Dual(p[2]));
-  if (dir == first) v.x.d = 1.0;
-  if (dir == first + 1) v.y.d = 1.0;
-  if (dir == first + 2) v.z.d = 1.0;
-  return v;
-}
-
-__global__ void refine_coef_grad_kernel(Args A) {
-  const long long e = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(32 * kCoefWarps) refine_coef_grad_kernel(Args A) {
+  extern __shared__ double coef_smem[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const long long e = (long long)blockIdx.x * kCoefWarps + wid;
   if (e >= A.nref) return;
+  constexpr int P = 33;  // pitch of a value over the lanes
+  double* pv = coef_smem + wid * (kPtVals + kPtBasis) * P;  // [kPtVals][P] cotangents of this chunk's points
+  double* pb = pv + kPtVals * P;                             // [kPtBasis][P] shape functions
   const int i = A.ref_row[e], j = A.ref_col[e], kind = A.ref_kind[e];
   const int no = A.order + 1;
   const int fk = A.face_kind[j];
-  const int nn = fk == 0 ? 3 : (fk == 1 ? 4 : (fk == 2 ? 6 : 9));
   const bool self = (kind == 2);
-  // directions: self: pos_i (0-2), n_i (3-5), t1 (6-8), t2 (9-11), nodes (12 + 3c + x)
-  //             near: pos_i (0-2), pos_j (3-5), nodes (6 + 3c + x)
-  const int nbase = self ? 12 : 6;
-  const int ndir = nbase + 3 * nn;
+  const bool quad = fk == 1 || fk == 3;
+  const int nsub = !self && quad ? 2 : 1;
+  const int nb = self ? (fk == 0 ? 3 : fk == 1 ? 4 : fk == 2 ? 6 : 9) : (fk >= 2 ? 6 : 3);
+  const int npts = self ? (quad ? A.n4 : A.n3) : A.n28;
   const double* nodes = A.nodes + 27LL * j;
-  for (int dir = 0; dir < ndir; ++dir) {
-    ad::Face<Dual> fc;
-    fc.kind = fk;
-    for (int c = 0; c < nn; ++c) fc.node[c] = seed3(nodes + 3 * c, dir, nbase + 3 * c);
-    const V3<Dual> pi = seed3(A.pos + 3 * i, dir, 0);
-    Dual sg[kMaxOrder + 1], s1[kMaxOrder + 1], s2[kMaxOrder + 1], s3[kMaxOrder + 1];
-    for (int m = 0; m <= kMaxOrder; ++m) sg[m] = s1[m] = s2[m] = s3[m] = Dual(0.0);
-    double2 acc = make_double2(0, 0);
-    if (self) {
-      const V3<Dual> ni = seed3(A.nvec + 3 * i, dir, 3);
-      const V3<Dual> t1 = seed3(A.tvec1 + 3 * i, dir, 6);
-      const V3<Dual> t2 = seed3(A.tvec2 + 3 * i, dir, 9);
-      const int npts = (fk == 0 || fk == 2) ? A.n3 : A.n4;
-      double rmax = 0.0;
-      for (int q = lane; q < npts; q += 32) {
-        V3<Dual> pt;
-        Dual w;
-        ad::polar_pt<Dual>(fc, A.rules, A.n28, A.n3, A.n4, q, pt, w);
-        rmax = fmax(rmax, fmax(ad::val(ad::norm(ad::sub(pi, pt))), kEps));
-      }
-      rmax = wmax(rmax);
-      const double rfloor = 1e-4 * rmax;
-      for (int q = lane; q < npts; q += 32) {
-        V3<Dual> pt;
-        Dual w;
-        ad::polar_pt<Dual>(fc, A.rules, A.n28, A.n3, A.n4, q, pt, w);
-        const V3<Dual> v = ad::sub(pi, pt);
-        const Dual r = ad::dmax(ad::norm(v), kEps);
-        const Dual ndr = ad::dot(ni, v), in1 = ad::dot(t1, v), in2 = ad::dot(t2, v);
-        const Dual rr = ad::dmax(r, rfloor);
-        const Dual irr3 = Dual(1.0) / (rr * rr * rr);
-        const Dual ir = Dual(1.0) / r;
-        Dual rp_m1 = ir, rp_m3 = ir * ir * ir, rp_m = Dual(1.0);
-        for (int m = 0; m < no; ++m) {
-          sg[m] += w * rp_m1;
-          s1[m] += w * ndr * rp_m3;
-          s2[m] += w * in1 * rp_m * irr3;
-          s3[m] += w * in2 * rp_m * irr3;
-          rp_m1 *= r;
-          rp_m3 *= r;
-          rp_m *= r;
-        }
-      }
-      double fact = 1.0;
-      for (int m = 0; m < no; ++m) {
-        if (m > 0) fact *= m;
-        const Dual a = wsumT(sg[m]), b = wsumT(s1[m]), c = wsumT(s2[m]), dd = wsumT(s3[m]);
-        // g_m = a / m!;  f_m = n (m-1) b / m! + t1 (m-1) c / m! + t2 (m-1) dd / m!
-        const double gd = a.d / fact;
-        acc = ca(acc, cs(A.ghat[e * no + m], gd));
-        const double cf = (m - 1) / fact;
-        const Dual fx = (ni.x * b + t1.x * c + t2.x * dd) * cf;
-        const Dual fy = (ni.y * b + t1.y * c + t2.y * dd) * cf;
-        const Dual fz = (ni.z * b + t1.z * c + t2.z * dd) * cf;
-        acc = ca(acc, cs(A.fhat[(e * 3 + 0) * no + m], fx.d));
-        acc = ca(acc, cs(A.fhat[(e * 3 + 1) * no + m], fy.d));
-        acc = ca(acc, cs(A.fhat[(e * 3 + 2) * no + m], fz.d));
-      }
-    } else {
-      const V3<Dual> pj = seed3(A.pos + 3 * j, dir, 3);
-      const Dual r0 = ad::norm(ad::sub(pj, pi));
-      const int nsub = (fk == 1 || fk == 3) ? 2 : 1;
-      for (int t = lane; t < nsub * A.n28; t += 32) {
-        const int s = t / A.n28, q = t - s * A.n28;
-        V3<Dual> pt;
-        Dual w;
-        ad::tri_pt<Dual>(fc, A.rules, A.n28, s, q, pt, w);
-        const V3<Dual> v = ad::sub(pi, pt);
-        const Dual r = ad::dmax(ad::norm(v), kEps);
-        const Dual ir = Dual(1.0) / r;
-        const Dual ir2 = ir * ir, ir3 = ir2 * ir;
-        const Dual dl = r - r0;
-        Dual dpow = Dual(1.0), dprev = Dual(0.0);
-        double fm = 1.0, fm1 = 1.0;
-        for (int m = 0; m < no; ++m) {
-          sg[m] += w * dpow * ir * (1.0 / fm);
-          const Dual fs = (m == 0) ? -ir3 : (-(dpow * ir3) * (1.0 / fm) + dprev * ir2 * (1.0 / fm1));
-          s1[m] += w * v.x * fs;
-          s2[m] += w * v.y * fs;
-          s3[m] += w * v.z * fs;
-          dprev = dpow;
-          dpow *= dl;
-          fm1 = fm;
-          fm *= (m + 1);
-        }
-      }
-      for (int m = 0; m < no; ++m) {
-        const Dual a = wsumT(sg[m]), b = wsumT(s1[m]), c = wsumT(s2[m]), dd = wsumT(s3[m]);
-        acc = ca(acc, cs(A.ghat[e * no + m], a.d));
-        acc = ca(acc, cs(A.fhat[(e * 3 + 0) * no + m], b.d));
-        acc = ca(acc, cs(A.fhat[(e * 3 + 1) * no + m], c.d));
-        acc = ca(acc, cs(A.fhat[(e * 3 + 2) * no + m], dd.d));
-      }
+  const double2* gh = A.ghat + e * no;
+  const double2* fh = A.fhat + e * 3 * no;
+  const Vec pi = vload(A.pos + 3 * i);
+  Vec pj{0, 0, 0}, ni{0, 0, 0}, t1{0, 0, 0}, t2{0, 0, 0}, u0{0, 0, 0};
+  double r0 = 0.0, rfloor = 0.0;
+  // point q of sub-element s: shape functions to shared memory, position, px, py
+  auto point = [&](int s, int q, Vec& x, Vec& px, Vec& py) -> double {
+    const double wf = shape_at(A, fk, self, q, pb + lane, P);
+    x = px = py = Vec{0, 0, 0};
+    for (int c = 0; c < nb; ++c) {
+      const double* nd = nodes + 3 * sub_node(fk, self, s, c);
+      const double N = pb[(3 * c) * P + lane], Dx = pb[(3 * c + 1) * P + lane], Dy = pb[(3 * c + 2) * P + lane];
+      x = {fma(N, nd[0], x.x), fma(N, nd[1], x.y), fma(N, nd[2], x.z)};
+      px = {fma(Dx, nd[0], px.x), fma(Dx, nd[1], px.y), fma(Dx, nd[2], px.z)};
+      py = {fma(Dy, nd[0], py.x), fma(Dy, nd[1], py.y), fma(Dy, nd[2], py.z)};
     }
+    return wf;
+  };
+  if (self) {
+    ni = vload(A.nvec + 3 * i);
+    t1 = vload(A.tvec1 + 3 * i);
+    t2 = vload(A.tvec2 + 3 * i);
+    double rmax = 0.0;
+    for (int q = lane; q < npts; q += 32) {
+      Vec x, px, py;
+      point(0, q, x, px, py);
+      const Vec v = vsub(pi, x);
+      rmax = fmax(rmax, fmax(sqrt(vdot(v, v)), kEps));
+    }
+    rfloor = 1e-4 * wmax(rmax);
+  } else {
+    pj = vload(A.pos + 3 * j);
+    const Vec d = vsub(pj, pi);
+    r0 = sqrt(vdot(d, d));
+    const double ir0 = r0 > 0 ? 1.0 / r0 : 0.0;
+    u0 = {d.x * ir0, d.y * ir0, d.z * ir0};
+  }
+  const double2 zero = make_double2(0, 0);
+  double2 gpi[3] = {zero, zero, zero};  // pos_i
+  double2 gr0 = zero;                   // r0
+  double2 gn[3] = {zero, zero, zero}, g1[3] = {zero, zero, zero}, g2[3] = {zero, zero, zero};  // n, t1, t2 (self)
+  double2 gnode[2] = {zero, zero};      // lane 3 c + x: node of shape function c, per sub-element
+  for (int s = 0; s < nsub; ++s) {
+    for (int q0 = 0; q0 < npts; q0 += 32) {
+      const int q = q0 + lane;
+      double2 ct[9];
+#pragma unroll
+      for (int c = 0; c < 9; ++c) ct[c] = zero;
+      if (q < npts) {
+        Vec x, px, py;
+        const double wf = point(s, q, x, px, py);
+        const Vec nn = vcross(px, py);
+        const double J = sqrt(vdot(nn, nn)), w = J * wf;
+        const Vec v = vsub(pi, x);
+        const double rv = sqrt(vdot(v, v));
+        const double r = fmax(rv, kEps), ir = 1.0 / r;
+        const double act = rv >= kEps ? ir : 0.0;  // dr / dv = v act
+        double2 phi, dv[3];
+        if (!self) {
+          // phi = G ir - ir^3 v.P + ir^2 v.P', polynomials in dl = r - r0:
+          // G = sum ghat_m dl^m / m!, P_c = sum fhat_cm dl^m / m!
+          const double dl = r - r0, ir2 = ir * ir, ir3 = ir2 * ir;
+          double2 G = zero, G1 = zero, p0[3], p1[3], p2[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) p0[c] = p1[c] = p2[c] = zero;
+          double t0 = 1.0, tm1 = 0.0, tm2 = 0.0;  // dl^m / m!, and one and two orders lower
+          for (int m = 0; m < no; ++m) {
+            const double2 a = gh[m];
+            G = cfma(a, t0, G);
+            G1 = cfma(a, tm1, G1);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              const double2 f = fh[c * no + m];
+              p0[c] = cfma(f, t0, p0[c]);
+              p1[c] = cfma(f, tm1, p1[c]);
+              p2[c] = cfma(f, tm2, p2[c]);
+            }
+            tm2 = tm1;
+            tm1 = t0;
+            t0 *= dl / (m + 1);
+          }
+          double2 s0 = zero, s1 = zero, s2 = zero;
+          const double vv[3] = {v.x, v.y, v.z};
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            s0 = cfma(p0[c], vv[c], s0);
+            s1 = cfma(p1[c], vv[c], s1);
+            s2 = cfma(p2[c], vv[c], s2);
+          }
+          phi = ca(ca(cs(G, ir), cs(s0, -ir3)), cs(s1, ir2));
+          const double2 pdl = ca(ca(cs(G1, ir), cs(s1, -ir3)), cs(s2, ir2));
+          const double2 pr = ca(ca(cs(G, -ir2), cs(s0, 3.0 * ir2 * ir2)), cs(s1, -2.0 * ir3));
+          const double2 rad = cs(ca(pdl, pr), act);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) dv[c] = cfma(rad, vv[c], ca(cs(p0[c], -ir3), cs(p1[c], ir2)));
+          gr0 = cfma(pdl, -w, gr0);
+        } else {
+          // phi = A + ndr n.FB + irr3 (in1 t1.FC + in2 t2.FC),  A = sum ghat_m r^(m-1) / m!,
+          // FB = sum fhat_m (m-1) / m! r^(m-3),  FC = r^3 FB
+          const double rr = fmax(r, rfloor), irr = 1.0 / rr, irr3 = irr * irr * irr;
+          double2 a0 = zero, a1 = zero, b0[3], b1[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) b0[c] = b1[c] = zero;
+          double rm = 1.0, fact = 1.0;  // r^m, m!
+          for (int m = 0; m < no; ++m) {
+            if (m > 0) fact *= m;
+            const double2 a = gh[m];
+            a0 = cfma(a, rm * ir / fact, a0);
+            a1 = cfma(a, (m - 1) * rm * ir * ir / fact, a1);
+            const double cf = (m - 1) / fact;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {  // FC and its derivative
+              const double2 f = fh[c * no + m];
+              b0[c] = cfma(f, cf * rm, b0[c]);
+              b1[c] = cfma(f, cf * m * rm * ir, b1[c]);
+            }
+            rm *= r;
+          }
+          const double ir3 = ir * ir * ir;
+          const double nvv[3] = {ni.x, ni.y, ni.z}, t1v[3] = {t1.x, t1.y, t1.z}, t2v[3] = {t2.x, t2.y, t2.z};
+          const double vv[3] = {v.x, v.y, v.z};
+          const double ndr = vdot(ni, v), in1 = vdot(t1, v), in2 = vdot(t2, v);
+          double2 B = zero, B1 = zero, C = zero, C1 = zero, D = zero, D1 = zero;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const double2 fb = cs(b0[c], ir3);                               // FB
+            const double2 fb1 = ca(cs(b1[c], ir3), cs(b0[c], -3.0 * ir3 * ir));  // FB'
+            B = cfma(fb, nvv[c], B);
+            B1 = cfma(fb1, nvv[c], B1);
+            C = cfma(b0[c], t1v[c], C);
+            C1 = cfma(b1[c], t1v[c], C1);
+            D = cfma(b0[c], t2v[c], D);
+            D1 = cfma(b1[c], t2v[c], D1);
+          }
+          const double2 tcd = ca(cs(C, in1), cs(D, in2));
+          phi = ca(ca(a0, cs(B, ndr)), cs(tcd, irr3));
+          double2 pr = ca(ca(a1, cs(B1, ndr)), cs(ca(cs(C1, in1), cs(D1, in2)), irr3));
+          if (r >= rfloor) pr = cfma(tcd, -3.0 * irr3 * irr, pr);
+          const double2 rad = cs(pr, act);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            dv[c] = cfma(rad, vv[c], ca(cs(B, nvv[c]), cs(ca(cs(C, t1v[c]), cs(D, t2v[c])), irr3)));
+            gn[c] = ca(gn[c], cs(ca(cs(B, vv[c]), cs(b0[c], ndr * ir3)), w));
+            g1[c] = ca(g1[c], cs(ca(cs(C, vv[c]), cs(b0[c], in1)), w * irr3));
+            g2[c] = ca(g2[c], cs(ca(cs(D, vv[c]), cs(b0[c], in2)), w * irr3));
+          }
+        }
+        // cotangents of x, px, py
+        const double iJ = J > 0 ? 1.0 / J : 0.0;
+        const Vec un{nn.x * iJ, nn.y * iJ, nn.z * iJ};
+        const Vec jx = vcross(py, un), jy = vcross(un, px);
+        const double2 pj_ = cs(phi, wf);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          gpi[c] = cfma(dv[c], w, gpi[c]);
+          ct[c] = cs(dv[c], -w);
+        }
+        ct[3] = cs(pj_, jx.x);
+        ct[4] = cs(pj_, jx.y);
+        ct[5] = cs(pj_, jx.z);
+        ct[6] = cs(pj_, jy.x);
+        ct[7] = cs(pj_, jy.y);
+        ct[8] = cs(pj_, jy.z);
+      }
+#pragma unroll
+      for (int c = 0; c < 9; ++c) {
+        pv[(2 * c) * P + lane] = ct[c].x;
+        pv[(2 * c + 1) * P + lane] = ct[c].y;
+      }
+      __syncwarp();
+      if (lane < 3 * nb) {
+        const int c = lane / 3, x = lane - 3 * c;
+        const int np = min(32, npts - q0);
+        double2 acc = gnode[s];
+        for (int k = 0; k < np; ++k) {
+          const double N = pb[(3 * c) * P + k], Dx = pb[(3 * c + 1) * P + k], Dy = pb[(3 * c + 2) * P + k];
+          acc.x = fma(N, pv[(2 * x) * P + k], fma(Dx, pv[(2 * x + 6) * P + k], fma(Dy, pv[(2 * x + 12) * P + k], acc.x)));
+          acc.y = fma(N, pv[(2 * x + 1) * P + k],
+                      fma(Dx, pv[(2 * x + 7) * P + k], fma(Dy, pv[(2 * x + 13) * P + k], acc.y)));
+        }
+        gnode[s] = acc;
+      }
+      __syncwarp();
+    }
+  }
+  if (lane < 3 * nb) {
+    const int c = lane / 3, x = lane - 3 * c;
+    for (int s = 0; s < nsub; ++s) atomic_c(&A.gnodes[27LL * j + 3 * sub_node(fk, self, s, c) + x], gnode[s]);
+  }
+  const double uu[3] = {u0.x, u0.y, u0.z};
+  if (!self) gr0 = wsum2(gr0);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double2 g = wsum2(gpi[c]);
     if (lane == 0) {
-      double2* dst;
-      if (dir < 3)
-        dst = &A.gpos[3 * i + dir];
-      else if (self && dir < 6)
-        dst = &A.gnv[3 * i + dir - 3];
-      else if (self && dir < 9)
-        dst = &A.gt1[3 * i + dir - 6];
-      else if (self && dir < 12)
-        dst = &A.gt2[3 * i + dir - 9];
-      else if (!self && dir < 6)
-        dst = &A.gpos[3 * j + dir - 3];
-      else
-        dst = &A.gnodes[27LL * j + (dir - nbase)];
-      atomic_c(dst, acc);
+      atomic_c(&A.gpos[3 * i + c], self ? g : cfma(gr0, -uu[c], g));  // d r0 / d pos_i = -u0
+      if (!self) atomic_c(&A.gpos[3 * j + c], cs(gr0, uu[c]));
+    }
+    if (self) {
+      const double2 a = wsum2(gn[c]), b = wsum2(g1[c]), d = wsum2(g2[c]);
+      if (lane == 0) {
+        atomic_c(&A.gnv[3 * i + c], a);
+        atomic_c(&A.gt1[3 * i + c], b);
+        atomic_c(&A.gt2[3 * i + c], d);
+      }
     }
   }
 }
@@ -758,7 +919,8 @@ int bem200_shape_gradient(int n, int npol, int npart, const int32_t* pid, const 
   BEM_LAUNCH_CHECK();
   refined_closed_kernel<<<ceil_div(nref, 128), 128, 0, s>>>(A);
   BEM_LAUNCH_CHECK();
-  refine_coef_grad_kernel<<<ceil_div(nref * 32, 128), 128, 0, s>>>(A);
+  const int csm = kCoefWarps * (kPtVals + kPtBasis) * 33 * (int)sizeof(double);
+  refine_coef_grad_kernel<<<ceil_div(nref, kCoefWarps), 32 * kCoefWarps, csm, s>>>(A);
   BEM_LAUNCH_CHECK();
   return BEM200_OK;
 }
