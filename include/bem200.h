@@ -223,7 +223,8 @@ size_t bem200_gemm_workspace_size(int engine, int m, int n, int k);
  * pivots that may differ from LAPACK's (measured slower than partial
  * pivoting at n = 5768 on B200, so off by default).  BEM200_GETRF_PARTIAL_
  * PIVOTING (the default) is accepted and wins over it.  lookahead_nb = block
- * width of the look-ahead schedule (multiple of 32 in [64, 1024]; 0 = 128). */
+ * width of the look-ahead schedule (multiple of 32 in [64, 1024]; 0 = 128, for
+ * large complex128 matrices 256 or 512). */
 #define BEM200_GETRF_PARTIAL_PIVOTING 1
 #define BEM200_GETRF_TOURNAMENT_PIVOTING 2
 /* BEM200_GETRF_DIAGONAL_PIVOTS: factor without the pivot search (blocked,
@@ -324,7 +325,7 @@ int bem200_bem_init(int precision, int engine, int n, void* ws, int eps_per_face
  * BEM200_ERR_PIVOTING when one of G1, G2, Delta, Sigma needs row exchanges,
  * and the caller writes the slots again and repeats the call without the
  * flag), lookahead_nb the block width of the
- * look-ahead LU schedule (a multiple of 32 in [64, 1024]; 0 = 128).
+ * look-ahead LU schedule (a multiple of 32 in [64, 1024]; 0 = the default).
  * BEM200_INIT_REPAIR (with DIAGONAL_PIVOTS, precision 0 or 1, info_host given):
  * when G1 and G2 passed their checks and only Delta or Sigma needs row
  * exchanges, that part alone is built again with partial pivoting inside the

@@ -1408,14 +1408,14 @@ __global__ void __launch_bounds__(kCaluThreads, 1) panel_calu_kernel(int m, int 
 // the diagonal element is the first largest |re| + |im| of its column; the
 // factor matrices of the retarded BEM (G1, G2, Delta, mostly Sigma) have
 // that property, so their panels can skip the column-wide pivot search that
-// bounds the pivoted panels.  Every CTA factors the w x w diagonal block in
-// registers (warp 0, a lane per row), then each thread takes one row
-// below it through x U11 = a (forward substitution in registers, the
-// triangle fully unrolled).  Column j fails the check when some row has
-// |a_ij^(j)|_1 > tau |a_jj^(j)|_1; a failing panel raises ctx.vflag and the
-// caller factors the matrix again with partial pivoting.  With tau = 1 a
-// passing matrix gets LAPACK's partial-pivoting factors (no exchanges).
-constexpr int kNopivPanelThreads = 64;
+// bounds the pivoted panels.  Two launches per 64 columns: one CTA factors the
+// 64 x 64 diagonal block in registers (panel_diag_kernel), then the rows below
+// it are multiplied by U11^-1 (trsm_leaf with the check).  Column j fails the
+// check when some row has |a_ij^(j)|_1 > tau |a_jj^(j)|_1; a failing panel
+// raises ctx.vflag and the caller factors the matrix again with partial
+// pivoting.  With tau = 1 a passing matrix gets LAPACK's partial-pivoting
+// factors (no exchanges).
+constexpr int kDiagNB = 64;
 
 // 1 / p for p != 0 (0 for p = 0), scaled by max(|re|, |im|) so that |p|^2
 // neither overflows nor underflows: two real divisions, no branches
@@ -1430,137 +1430,131 @@ __device__ __forceinline__ C crecip_scaled(C p) {
   return cmake<C>(px * f, -py * f);
 }
 
+// 1 / p in FP64: p scaled by a power of two, one approximate reciprocal of
+// |p|^2 and two Newton steps (relative error below 2^-51).  The two divisions of
+// crecip_scaled are a chain of about 400 cycles in every elimination step.
+// p = 0 gives NaN, or 0 with kZeroSafe.
+template <bool kZeroSafe>
+__device__ __forceinline__ double2 crecip_newton(double2 p) {
+  const double m = fmax(fabs(p.x), fabs(p.y));
+  if (kZeroSafe && !(m > 0.0)) return make_double2(0.0, 0.0);
+  const double s = __hiloint2double(min(2046, 2046 - ((__double2hiint(m) >> 20) & 0x7ff)) << 20, 0);
+  const double px = p.x * s, py = p.y * s, d = fma(px, px, py * py);
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  r = fma(r, fma(-d, r, 1.0), r);
+  r = fma(r, fma(-d, r, 1.0), r);
+  const double f = r * s;
+  return make_double2(px * f, -py * f);
+}
+__device__ __forceinline__ double2 crecip_pivot(double2 p) { return crecip_newton<true>(p); }
+__device__ __forceinline__ float2 crecip_pivot(float2 p) { return crecip_scaled(p); }
+
+// acc +- a b, four FMAs
 template <typename C>
-__global__ void __launch_bounds__(kNopivPanelThreads) panel_nopiv_kernel(int m, int w, C* __restrict__ A, long long ld,
-                                                                         int col, const int32_t* __restrict__ rowmap,
-                                                                         int32_t* __restrict__ ipiv, int ipiv_base,
-                                                                         int* __restrict__ info,
-                                                                         int* __restrict__ vflag, R_t<C> tau,
-                                                                         int* __restrict__ arrived) {
-  // D is one row taller than the block: the rotated reads D[j][j + c] stay inside
-  __shared__ C D[kPanelNB + 1][kPanelNB + 1];
-  __shared__ C rinv[kPanelNB], prow[kPanelNB];
-  __shared__ int zfirst, viol, last;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+__device__ __forceinline__ void cmac(C& acc, C a, C b) {
+  acc.x = fma(-a.y, b.y, fma(a.x, b.x, acc.x));
+  acc.y = fma(a.y, b.x, fma(a.x, b.y, acc.y));
+}
+template <typename C>
+__device__ __forceinline__ void cmsub(C& acc, C a, C b) {
+  acc.x = fma(a.y, b.y, fma(-a.x, b.x, acc.x));
+  acc.y = fma(-a.y, b.x, fma(-a.x, b.y, acc.y));
+}
+
+// L U of the w x w (w <= 64) diagonal block, no row exchanges.  Thread (ty, tx)
+// of the 16 x 16 grid holds rows ty + 16 p and columns tx + 16 q of the block
+// (padded with the identity); step k publishes row k, column k and the
+// reciprocal of the pivot in double-buffered shared memory: one barrier per
+// step.  Latency bound (one CTA, 64 dependent steps).
+template <typename C>
+__global__ void __launch_bounds__(256) panel_diag_kernel(int w, C* __restrict__ A, long long ld, int col,
+                                                         const int32_t* __restrict__ rowmap,
+                                                         int32_t* __restrict__ ipiv, int ipiv_base,
+                                                         int* __restrict__ info, int* __restrict__ vflag, R_t<C> tau) {
+  using R = R_t<C>;
+  constexpr int N = kDiagNB, G = 16, PQ = N / G;
+  __shared__ C rowb[2][N], colb[2][N], rinv[2];
+  __shared__ int zfirst, viol;
+  const int tid = threadIdx.x, ty = tid / G, tx = tid % G;
   if (tid == 0) {
     zfirst = INT_MAX;
     viol = 0;
   }
-  for (int idx = tid; idx < w * w; idx += kNopivPanelThreads) {
-    const int i = idx / w, c = idx % w;
-    D[i][c] = A[(long long)rowmap[i] * ld + col + c];
-  }
-  // this thread's row below the diagonal block (complex64: loaded while warp
-  // 0 factors the block; complex128 registers hold one row at a time)
-  const int r = w + blockIdx.x * kNopivPanelThreads + tid;
-  C* row = r < m ? A + (long long)rowmap[r] * ld + col : nullptr;
-  C x[kPanelNB];
-  if constexpr (sizeof(C) == 8) {
+  C a[PQ][PQ];
 #pragma unroll
-    for (int c = 0; c < kPanelNB; ++c) x[c] = (row && c < w) ? row[c] : czero<C>();
-  }
-  __syncthreads();
-  // Every CTA needs the unfactored diagonal block, and not all CTAs need run
-  // at once: the factored block is written back by the CTA whose read of it
-  // was the last (it holds the same factors as every other), never before.
-  if (tid == 0) {
-    __threadfence();
-    last = atomicAdd(arrived, 1) == (int)gridDim.x - 1;
-    if (last) atomicExch(arrived, 0);  // for the next panel
-  }
-  // Both parts keep the current column in register 0: every step shifts the
-  // row left by one (updating the columns still open) and appends the new
-  // multiplier, so register indices stay static in a rolled loop; after the
-  // 32 steps of a full cycle the row is back in column order.
-  if (wid == 0) {  // the diagonal block, lane i owning row i (padded with the identity)
-    C v[kPanelNB];
+  for (int p = 0; p < PQ; ++p)
 #pragma unroll
-    for (int c = 0; c < kPanelNB; ++c)
-      v[c] = (lane < w && c < w) ? D[lane][c] : (lane == c ? cmake<C>(1.0, 0.0) : czero<C>());
-    bool bad = false;
+    for (int q = 0; q < PQ; ++q) {
+      const int i = ty + G * p, j = tx + G * q;
+      a[p][q] = (i < w && j < w) ? A[(long long)rowmap[i] * ld + col + j] : (i == j ? cmake<C>(1.0, 0.0) : czero<C>());
+    }
+  bool bad = false;
+#pragma unroll
+  for (int kp = 0; kp < PQ; ++kp) {
+    if (G * kp >= w) break;
 #pragma unroll 1
-    for (int j = 0; j < kPanelNB; ++j) {
-      if (lane == j) {
+    for (int kr = 0; kr < G; ++kr) {
+      const int k = G * kp + kr, b = k & 1;
+      if (tx == kr) {
 #pragma unroll
-        for (int c = 0; c < kPanelNB; ++c) prow[c] = v[c];
+        for (int p = kp; p < PQ; ++p) colb[b][ty + G * p] = a[p][kp];
+        if (ty == kr) rinv[b] = crecip_pivot(a[kp][kp]);
       }
-      __syncwarp();
-      const C piv = prow[0];
-      const R_t<C> pm = pmag(piv);
-      const C inv = crecip_scaled(piv);
-      const bool act = lane > j;
-      if (act && pmag(v[0]) > tau * pm) bad = true;
-      const C l = cmul(v[0], inv);
-      const C first = v[0];
-      const int lim = kPanelNB - 1 - j;
+      if (ty == kr) {
 #pragma unroll
-      for (int c = 1; c < kPanelNB; ++c) {
-        const C u = csub(v[c], cmul(l, prow[c]));
-        v[c - 1] = (act && c <= lim) ? u : v[c];
+        for (int q = kp; q < PQ; ++q) rowb[b][tx + G * q] = a[kp][q];
       }
-      v[kPanelNB - 1] = act ? l : first;
-      if (lane == 0 && j < w && !(pm > 0) && zfirst == INT_MAX) zfirst = j;
-      __syncwarp();
-    }
+      __syncthreads();
+      const R pm = pmag(rowb[b][k]);
+      const C inv = rinv[b];
+      if (tid == 0 && k < w && !(pm > 0) && zfirst == INT_MAX) zfirst = k;
+      C u[PQ];
 #pragma unroll
-    for (int c = 0; c < kPanelNB; ++c) D[lane][c] = v[c];
-    C d = v[0];
+      for (int q = kp; q < PQ; ++q) u[q] = rowb[b][tx + G * q];
 #pragma unroll
-    for (int c = 1; c < kPanelNB; ++c)
-      if (c == lane) d = v[c];
-    rinv[lane] = crecip_scaled(d);
-    if (__any_sync(0xffffffffu, bad) && lane == 0) viol = 1;
-  }
-  __syncthreads();
-  if constexpr (sizeof(C) == 16) {
+      for (int p = kp; p < PQ; ++p) {
+        if (p == kp && ty <= kr) continue;
+        const C c = colb[b][ty + G * p];
+        if (pmag(c) > tau * pm) bad = true;
+        const C l = cmul(c, inv);
 #pragma unroll
-    for (int c = 0; c < kPanelNB; ++c) x[c] = (row && c < w) ? row[c] : czero<C>();
-  }
-  if (row) {  // x U11 = a; padded steps j >= w see an identity pivot and leave x alone
-    bool bad = false;
-#pragma unroll 1
-    for (int j = 0; j < kPanelNB; ++j) {
-      const C* Dj = &D[j][j];
-      if (pmag(x[0]) > tau * pmag(Dj[0])) bad = true;  // x[0] = a_rj^(j) here
-      const C l = cmul(x[0], rinv[j]);
-      const int lim = kPanelNB - 1 - j;
-#pragma unroll
-      for (int c = 1; c < kPanelNB; ++c) {
-        const C u = csub(x[c], cmul(l, Dj[c]));
-        x[c - 1] = c <= lim ? u : x[c];
+        for (int q = kp; q < PQ; ++q) {
+          if (q == kp && tx <= kr) continue;
+          cmsub(a[p][q], l, u[q]);
+        }
+        if (tx == kr) a[p][kp] = l;
       }
-      x[kPanelNB - 1] = l;
     }
+  }
 #pragma unroll
-    for (int c = 0; c < kPanelNB; ++c)
-      if (c < w) row[c] = x[c];
-    if (bad) viol = 1;
-  }
-  if (last) {  // (written before the __syncthreads between the two parts)
-    for (int idx = tid; idx < w * w; idx += kNopivPanelThreads) {
-      const int i = idx / w, c = idx % w;
-      A[(long long)rowmap[i] * ld + col + c] = D[i][c];
+  for (int p = 0; p < PQ; ++p)
+#pragma unroll
+    for (int q = 0; q < PQ; ++q) {
+      const int i = ty + G * p, j = tx + G * q;
+      if (i < w && j < w) A[(long long)rowmap[i] * ld + col + j] = a[p][q];
     }
-    if (tid < w) ipiv[tid] = ipiv_base + tid;
-  }
+  if (tid < w) ipiv[tid] = ipiv_base + tid;
+  if (bad) viol = 1;
   __syncthreads();
   if (tid == 0) {
     if (viol && vflag) atomicExch(vflag, 1);
-    if (blockIdx.x == 0 && zfirst != INT_MAX && info) atomicCAS(info, 0, ipiv_base + zfirst + 1);
+    if (zfirst != INT_MAX && info) atomicCAS(info, 0, ipiv_base + zfirst + 1);
   }
 }
+
+template <typename C>
+static int trsm_leaf_rows_checked(const LaContext& ctx, int m, int nvec, RowView<C> T, RowView<C> B);
 
 template <typename C>
 static int panel_lu(const LaContext& ctx, int m, int w, C* A, long long ld, int col, int32_t* rowmap, int32_t* ipiv,
                     int ipiv_base) {
   if (ctx.diag_pivots) {
-    const int grid = max(1, ceil_div(m - w, kNopivPanelThreads));
-    panel_nopiv_kernel<C><<<grid, kNopivPanelThreads, 0, ctx.stream>>>(m, w, A, ld, col, rowmap, ipiv, ipiv_base,
-                                                                        ctx.dinfo, ctx.vflag,
-                                                                        (R_t<C>)ctx.pivot_tau, ctx.vflag + 1);
+    panel_diag_kernel<C><<<1, 256, 0, ctx.stream>>>(w, A, ld, col, rowmap, ipiv, ipiv_base, ctx.dinfo, ctx.vflag,
+                                                    (R_t<C>)ctx.pivot_tau);
     BEM_LAUNCH_CHECK();
-    count_launch();
-    return BEM200_OK;
+    const RowView<C> V{A, ld, rowmap, col};
+    return trsm_leaf_rows_checked<C>(ctx, w, m - w, V, V.sub(w, 0));  // L21 = A21 U11^-1
   }
   if constexpr (sizeof(C) == 8) {
     if (ctx.tournament && m > kCaluMinRows && m <= kCaluMaxCluster * kCaluThreads) {
@@ -1707,18 +1701,17 @@ static int panel_lu(const LaContext& ctx, int m, int w, C* A, long long ld, int 
 }
 
 // ===================================================================== TRSM leaves
-// A leaf solves with a triangle of m <= NB = 64 rows held in shared memory
-// (odd pitch); larger triangles recurse, so the work above the leaves runs as
-// GEMMs with k >= 64 (tensor cores for complex64).  Each warp sweeps one
-// right-hand vector at a time -- a column of B for left solves, a row of X for
-// right solves.  Lane l holds elements l + 32 t of the vector in registers;
-// each step of the sweep finishes one element, broadcasts it with a shuffle and
-// updates the elements still open (NB / 32 complex FMAs per lane at most).
-// Divisions by the diagonal use reciprocals computed before the sweep.  A CTA
-// owns kLeafVecs vectors, two per warp.
+// A leaf solves with a triangle of m <= NB = 64 rows; larger triangles recurse,
+// so the work above the leaves runs as GEMMs with k >= 64 (tensor cores for the
+// large ones).  Every CTA holds the triangle in shared memory in a canonical
+// form (lower, the backward kinds with reversed indices), inverts its two 32 x
+// 32 diagonal blocks (8 x 8 by substitution, then block merges) and applies
+// X1 = D1^-1 B1, X2 = D2^-1 (B2 - T21 X1) to NV right-hand vectors (columns of B
+// for left solves, rows of X for right solves) as small products.  The
+// substitution it replaces was a chain of 64 shuffles per vector: complex128
+// 64 x 64 x 2884 vectors 35 us, now about 8.  FP64 (FP32) pipe bound.
 template <typename C> struct LeafNB { static constexpr int value = 64; };
 constexpr int kLeafThreads = 256;
-constexpr int kLeafVecs = 16;
 
 enum LeafKind : int {
   kLeftLowerUnit = 0,   // B <- L^-1 B
@@ -1727,8 +1720,163 @@ enum LeafKind : int {
   kRightLowerUnit = 3,  // X <- X L^-1
 };
 
+// acc[p][v] += sum_{r < 32} M[row0 + ty + 16 p][r0 + r] V[r0 + r][tx + 16 v] for the 2 x NV / 16 block of a thread
+template <int NVT, int MP, int VP>
+__device__ __forceinline__ void leaf_product(const double2* M, const double2* V, int row0, int r0, int ty, int tx,
+                                             double2 (&acc)[2][NVT]) {
+#pragma unroll 8
+  for (int r = 0; r < 32; ++r) {
+    double2 m[2], v[NVT];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) m[p] = M[(row0 + ty + 16 * p) * MP + r0 + r];
+#pragma unroll
+    for (int q = 0; q < NVT; ++q) v[q] = V[(r0 + r) * VP + tx + 16 * q];
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+      for (int q = 0; q < NVT; ++q) cmac(acc[p][q], m[p], v[q]);
+  }
+}
+
+template <typename C, int K, int NV, bool kCheck>
+__global__ void __launch_bounds__(kLeafThreads) trsm_leaf_kernel(int m, int nvec, RowView<C> T, RowView<C> B,
+                                                                 double tau, int* __restrict__ vflag) {
+  constexpr int NB = LeafNB<C>::value, MP = NB + 1, VP = NV + 1, NVT = NV / 16;
+  constexpr bool kLeft = (K == kLeftLowerUnit || K == kLeftUpper);
+  constexpr bool kForward = (K == kLeftLowerUnit || K == kRightUpper);
+  constexpr bool kUnit = (K == kLeftLowerUnit || K == kRightLowerUnit);
+  extern __shared__ __align__(16) unsigned char leaf_smem[];
+  using D = double2;  // both types solve in FP64: the inverses lose nothing against substitution
+  D* M = reinterpret_cast<D*>(leaf_smem);  // [NB][MP]: the triangle, then the inverses of its diagonal blocks
+  D* V = M + NB * MP;                      // [NB][VP]: element e of vector v
+  __shared__ D rinv[NB], diag[NB], tmp[512];
+  const int tid = threadIdx.x;
+  const int v0 = blockIdx.x * NV;
+  const int nv = min(NV, nvec - v0);
+  // canonical lower triangle: element e of a backward kind is row m - 1 - e
+  for (int idx = tid; idx < NB * NB; idx += kLeafThreads) {
+    const int e = kLeft ? idx / NB : idx % NB, r = kLeft ? idx % NB : idx / NB;
+    D t = make_double2(e == r ? 1.0 : 0.0, 0.0);
+    if (e < m && r <= e && !(kUnit && e == r)) {
+      const int fe = kForward ? e : m - 1 - e, fr = kForward ? r : m - 1 - r;
+      const C g = kLeft ? T.at(fe, fr) : T.at(fr, fe);
+      t = make_double2(g.x, g.y);
+    }
+    M[e * MP + r] = t;
+    if (e == r) {
+      diag[e] = t;
+      rinv[e] = kUnit ? t : crecip_newton<kCheck>(t);
+    }
+  }
+  for (int idx = tid; idx < NB * NV; idx += kLeafThreads) {
+    const int e = kLeft ? idx / NV : idx % NB, v = kLeft ? idx % NV : idx / NB;
+    const int fe = kForward ? e : m - 1 - e;
+    const C g = (e < m && v < nv) ? (kLeft ? B.at(fe, v0 + v) : B.at(v0 + v, fe)) : czero<C>();
+    V[e * VP + v] = make_double2(g.x, g.y);
+  }
+  __syncthreads();
+  // inverses of the 8 x 8 diagonal blocks: thread 8 b + c takes column c of block b
+  D x[8];
+  if (tid < NB) {
+    const int b0 = tid & ~7, c = tid & 7;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      D s = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int j = 0; j < i; ++j) cmsub(s, M[(b0 + i) * MP + b0 + j], x[j]);
+      const D ri = rinv[b0 + i];
+      x[i] = i < c ? make_double2(0.0, 0.0) : (i == c ? ri : cmul(s, ri));
+    }
+  }
+  __syncthreads();
+  if (tid < NB) {
+    const int b0 = tid & ~7, c = tid & 7;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i >= c) M[(b0 + i) * MP + b0 + c] = x[i];
+  }
+  __syncthreads();
+  // merges 8 -> 16 -> 32: the off-diagonal block becomes -D2^-1 T21 D1^-1
+#pragma unroll
+  for (int h = 8; h <= 16; h *= 2) {
+    const int per = h * h, total = (NB / (2 * h)) * per;
+    for (int idx = tid; idx < total; idx += kLeafThreads) {
+      const int b = (idx / per) * 2 * h, i = (idx % per) / h, j = idx % h;
+      D s = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int r = 0; r < h; ++r) cmac(s, M[(b + h + i) * MP + b + r], M[(b + r) * MP + b + j]);
+      tmp[idx] = s;
+    }
+    __syncthreads();
+    for (int idx = tid; idx < total; idx += kLeafThreads) {
+      const int b = (idx / per) * 2 * h, i = (idx % per) / h, j = idx % h;
+      D s = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int r = 0; r < h; ++r) cmsub(s, M[(b + h + i) * MP + b + h + r], tmp[(idx / per) * per + r * h + j]);
+      M[(b + h + i) * MP + b + j] = s;
+    }
+    __syncthreads();
+  }
+  const int tx = tid & 15, ty = tid >> 4;
+  auto put = [&](int row0, const D(&acc)[2][NVT]) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+      for (int q = 0; q < NVT; ++q) V[(row0 + ty + 16 * p) * VP + tx + 16 * q] = acc[p][q];
+  };
+  D acc[2][NVT];
+  auto clear = [&]() {
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+      for (int q = 0; q < NVT; ++q) acc[p][q] = make_double2(0.0, 0.0);
+  };
+  clear();
+  leaf_product<NVT, MP, VP>(M, V, 0, 0, ty, tx, acc);  // X1 = D1^-1 B1
+  __syncthreads();
+  put(0, acc);
+  __syncthreads();
+  if (m > 32) {
+    clear();
+    leaf_product<NVT, MP, VP>(M, V, 32, 0, ty, tx, acc);  // T21 X1
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+      for (int q = 0; q < NVT; ++q) acc[p][q] = csub(V[(32 + ty + 16 * p) * VP + tx + 16 * q], acc[p][q]);
+    put(32, acc);  // B2 - T21 X1 (each thread rewrites the entries that it read)
+    __syncthreads();
+    clear();
+    leaf_product<NVT, MP, VP>(M, V, 32, 32, ty, tx, acc);
+    __syncthreads();
+    put(32, acc);
+    __syncthreads();
+  }
+  bool bad = false;
+  for (int idx = tid; idx < NB * NV; idx += kLeafThreads) {
+    const int e = kLeft ? idx / NV : idx % NB, v = kLeft ? idx % NV : idx / NB;
+    if (v >= nv || e >= m) continue;
+    const int fe = kForward ? e : m - 1 - e;
+    const D r = V[e * VP + v];
+    if constexpr (kCheck) {  // the multiplier times the pivot is the eliminated entry a_ie^(e)
+      if (pmag(cmul(r, diag[e])) > tau * pmag(diag[e])) bad = true;
+    }
+    const C g = cmake<C>(r.x, r.y);
+    if constexpr (kLeft) B.at(fe, v0 + v) = g; else B.at(v0 + v, fe) = g;
+  }
+  if constexpr (kCheck) {
+    if (__syncthreads_or(bad) && tid == 0 && vflag) atomicExch(vflag, 1);
+  }
+}
+
+// complex64: one warp sweeps one right-hand vector at a time by substitution
+// (the order of operations of LAPACK's, which the complex64 factors are
+// compared with).  Lane l holds elements l + 32 t of the vector in registers;
+// each step finishes one element, broadcasts it with a shuffle and updates the
+// elements still open.  A CTA owns kLeafVecs vectors, two per warp.
+constexpr int kLeafVecs = 16;
+
 template <typename C, int K>
-__global__ void __launch_bounds__(kLeafThreads) trsm_leaf_kernel(int m, int nvec, RowView<C> T, RowView<C> B) {
+__global__ void __launch_bounds__(kLeafThreads) trsm_leaf_subst_kernel(int m, int nvec, RowView<C> T, RowView<C> B) {
   constexpr int NB = LeafNB<C>::value, NT = NB / 32, P = NB + 1;
   constexpr bool kLeft = (K == kLeftLowerUnit || K == kLeftUpper);
   constexpr bool kForward = (K == kLeftLowerUnit || K == kRightUpper);
@@ -1815,25 +1963,46 @@ __global__ void __launch_bounds__(kLeafThreads) trsm_leaf_kernel(int m, int nvec
   }
 }
 
+template <typename C, int NV>
+static constexpr size_t leaf_smem_bytes() {
+  return sizeof(double2) * (size_t)LeafNB<C>::value * (LeafNB<C>::value + 1 + NV + 1);
+}
+
+template <typename C, int K, int NV, bool kCheck>
+static int trsm_leaf_launch(const LaContext& ctx, int m, int nvec, RowView<C> T, RowView<C> B) {
+  auto kern = trsm_leaf_kernel<C, K, NV, kCheck>;
+  BEM_CUDA_CHECK(set_kernel_attrs_once(kern, (int)leaf_smem_bytes<C, NV>(), false));
+  kern<<<ceil_div(nvec, NV), kLeafThreads, leaf_smem_bytes<C, NV>(), ctx.stream>>>(m, nvec, T, B, (double)ctx.pivot_tau,
+                                                                                   ctx.vflag);
+  BEM_LAUNCH_CHECK();
+  return BEM200_OK;
+}
+
+// 32 vectors per CTA, 16 while that leaves SMs without work
+template <typename C, int K, bool kCheck = false>
+static int trsm_leaf(const LaContext& ctx, int m, int nvec, RowView<C> T, RowView<C> B) {
+  if constexpr (sizeof(C) == 8 && !kCheck) {
+    constexpr int NB = LeafNB<C>::value;
+    constexpr int smem = (int)(sizeof(C) * (size_t)(NB + kLeafVecs) * (NB + 1));
+    auto kern = trsm_leaf_subst_kernel<C, K>;
+    BEM_CUDA_CHECK(set_kernel_attrs_once(kern, smem, false));
+    kern<<<ceil_div(nvec, kLeafVecs), kLeafThreads, smem, ctx.stream>>>(m, nvec, T, B);
+    BEM_LAUNCH_CHECK();
+    return BEM200_OK;
+  }
+  if (nvec <= 148 * 16) return trsm_leaf_launch<C, K, 16, kCheck>(ctx, m, nvec, T, B);
+  return trsm_leaf_launch<C, K, 32, kCheck>(ctx, m, nvec, T, B);
+}
+
 template <typename C>
-static size_t leaf_smem_bytes() {
-  constexpr int NB = LeafNB<C>::value;
-  return sizeof(C) * (size_t)(NB + kLeafVecs) * (NB + 1);
+static int trsm_leaf_rows_checked(const LaContext& ctx, int m, int nvec, RowView<C> T, RowView<C> B) {
+  if (nvec <= 0) return BEM200_OK;
+  return trsm_leaf<C, kRightUpper, true>(ctx, m, nvec, T, B);
 }
 
 template <typename K>
 static int prep_smem(K kern, size_t bytes) {
   BEM_CUDA_CHECK(set_kernel_attrs_once(kern, (int)bytes, false));
-  return BEM200_OK;
-}
-
-template <typename C, int K>
-static int trsm_leaf(const LaContext& ctx, int m, int nvec, RowView<C> T, RowView<C> B) {
-  auto kern = trsm_leaf_kernel<C, K>;
-  int st = prep_smem(kern, leaf_smem_bytes<C>());
-  if (st) return st;
-  kern<<<ceil_div(nvec, kLeafVecs), kLeafThreads, leaf_smem_bytes<C>(), ctx.stream>>>(m, nvec, T, B);
-  BEM_LAUNCH_CHECK();
   return BEM200_OK;
 }
 
@@ -2243,8 +2412,9 @@ __global__ void iota_kernel(int n, int32_t* __restrict__ a) {
 template <typename C>
 static int getrf_rec(const LaContext& ctx, int n, C* A, long long ld, int32_t* rowmap, int32_t* ipiv, int col0,
                      int w) {
-  if (w <= kPanelNB) return panel_lu<C>(ctx, n - col0, w, A, ld, col0, rowmap + col0, ipiv + col0, col0);
-  int w1 = split_point(w, kPanelNB);
+  const int nb = ctx.diag_pivots ? kDiagNB : kPanelNB;
+  if (w <= nb) return panel_lu<C>(ctx, n - col0, w, A, ld, col0, rowmap + col0, ipiv + col0, col0);
+  int w1 = split_point(w, nb);
   int st = getrf_rec(ctx, n, A, ld, rowmap, ipiv, col0, w1);
   if (st) return st;
   RowView<C> V{A, ld, rowmap + col0, col0};  // logical rows from col0, columns from col0
@@ -2269,8 +2439,15 @@ static int getrf_rec(const LaContext& ctx, int n, C* A, long long ld, int32_t* r
 // so wide(j) addresses those rows through a snapshot of the row map taken
 // right after panel(j) (two snapshots alternate).  The rows themselves never
 // move, so both orders give the same matrix.
-static int la_width(const LaContext& ctx) {
-  const int w = ctx.la_nb > 0 ? ctx.la_nb : 128;
+template <typename C>
+static int la_width(const LaContext& ctx, int n) {
+  // complex128 updates on the tensor cores read and write 32 residue bytes per
+  // entry whatever the width: wide blocks pay off as soon as the panels hide
+  // (init at n = 5768: 150 / 126 / 121 ms for 128 / 256 / 512; at 2492 128 and
+  // 256 are equal, at 1016 the narrow ones win)
+  int dflt = 128;
+  if (sizeof(C) == 16 && ctx.engine == GemmEngine::kTc) dflt = n >= 4500 ? 512 : (n >= 3000 ? 256 : 128);
+  const int w = ctx.la_nb > 0 ? ctx.la_nb : dflt;
   return max(64, min(1024, (w / kPanelNB) * kPanelNB));
 }
 
@@ -2312,7 +2489,7 @@ static int getrf_lookahead(const LaContext& ctx, int n, C* A, long long ld, int3
   BEM_LAUNCH_CHECK();
   bool wide_pending = false;
   int st;
-  const int nb = la_width(ctx);
+  const int nb = la_width<C>(ctx, n);
   for (int c0 = 0, j = 0; c0 < n; c0 += nb, ++j) {
     const int w = min(nb, n - c0);
     if ((st = getrf_rec(cm, n, A, ld, rowmap, ipiv, c0, w))) return st;
@@ -2366,7 +2543,7 @@ int getrf(const LaContext& ctx, int n, C* A, long long ld, int32_t* rowmap, int3
   LaContext c = ctx;
   c.vflag = reinterpret_cast<int*>(reinterpret_cast<char*>(scratch) +
                                    (((size_t)2 * n * sizeof(int32_t) + 255) & ~size_t(255)));
-  BEM_CUDA_CHECK(cudaMemsetAsync(c.vflag, 0, 2 * sizeof(int), ctx.stream));  // the flag and the panels' arrival counter
+  BEM_CUDA_CHECK(cudaMemsetAsync(c.vflag, 0, sizeof(int), ctx.stream));
   int st = getrf_dispatch<C>(c, n, A, ld, rowmap, ipiv, scratch);
   if (st) return st;
   nopiv_finish_kernel<<<1, 1, 0, ctx.stream>>>(c.vflag, ctx.dinfo);
@@ -2379,11 +2556,11 @@ static int getrf_dispatch(const LaContext& ctx, int n, C* A, long long ld, int32
                           int32_t* scratch) {
   // look-ahead needs the row-map snapshots (scratch) and, on the tensor-core
   // engines, room for two concurrent GEMMs in the operand workspace
-  const bool ws_ok = gemm_tc_two_fit<C>(ctx, n, n, la_width(ctx));
+  const bool ws_ok = gemm_tc_two_fit<C>(ctx, n, n, la_width<C>(ctx, n));
   // (complex64 panels and updates below n = 512 are so short that the two
   // streams' events cost more than the overlap gains: 7.7 vs 7.0 ms for the
   // fallback chain of a 284-face solve)
-  if (scratch && n > max(2 * la_width(ctx), sizeof(C) == 8 ? 512 : 0) && ws_ok) return getrf_lookahead<C>(ctx, n, A, ld, rowmap, ipiv, scratch);
+  if (scratch && n > max(2 * la_width<C>(ctx, n), sizeof(C) == 8 ? 512 : 0) && ws_ok) return getrf_lookahead<C>(ctx, n, A, ld, rowmap, ipiv, scratch);
   iota_kernel<<<ceil_div(n, 256), 256, 0, ctx.stream>>>(n, rowmap);
   BEM_LAUNCH_CHECK();
   return getrf_rec(ctx, n, A, ld, rowmap, ipiv, 0, n);

@@ -68,7 +68,7 @@ struct LaContext {
 
 // LU scratch beyond the row-map snapshots: the grid-wide panel's candidate
 // slots (2 x up to 160 CTAs x (32 + 1) complex128); with checked diagonal
-// pivots its first two ints are the panels' verdict flag and arrival counter
+// pivots its first int is the panels' verdict flag
 constexpr size_t kPanelGridScratch = 176u * 1024u;
 
 // A non-blocking side stream forked from ctx.stream (fork()) and joined back

@@ -1,0 +1,42 @@
+"""Block edges of the complex128 LU without row exchanges (64-column diagonal
+blocks, rows below multiplied by U11^-1) and of the 64-row triangular leaves
+(32 x 32 inverses, 16 or 32 vectors per CTA), against numpy.  Tolerances: a
+well-conditioned matrix (cond ~ 3), n eps growth: 1e-13 relative."""
+import numpy as np
+import pytest
+
+from mnpbem_b200 import _native as nat
+
+pytestmark = pytest.mark.gpu
+
+
+def _dominant(n, seed):
+    rng = np.random.default_rng(seed)
+    A = (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) / np.sqrt(n)
+    return A + 4 * np.eye(n)
+
+
+# one ragged block, exact blocks, one column over, several blocks; few
+# vectors, a ragged CTA of vectors, more than 148 x 16 (32 per CTA)
+@pytest.mark.parametrize("n,nrhs", [(17, 33), (64, 17), (65, 40), (96, 2400), (129, 31), (200, 18), (321, 64)])
+def test_checked_lu_and_triangular_leaves_c128(cuda, n, nrhs):
+    import torch
+    A = _dominant(n, n)
+    B = np.random.default_rng(n + 1).standard_normal((n, nrhs)) + 1j
+    L = nat.lib()
+    At, Bt = torch.as_tensor(A, device="cuda"), torch.as_tensor(B, device="cuda")
+    rowmap, ipiv = (torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2))
+    info, status = (torch.zeros(1, dtype=torch.int32, device="cuda") for _ in range(2))
+    wsb = int(L.bem200_getrf_workspace_size(nat.C128, 0, n))
+    ws = torch.empty(wsb, dtype=torch.uint8, device="cuda")
+    nat.call("bem200_getrf_ex", nat.C128, 0, n, nat.ptr(At), n, nat.ptr(rowmap), nat.ptr(ipiv), nat.ptr(info),
+             nat.ptr(ws), wsb, 4, 0, nat.stream_ptr())
+    assert int(info.item()) == 0
+    F = At.cpu().numpy()
+    P = (np.tril(F, -1) + np.eye(n)) @ np.triu(F)
+    assert np.max(np.abs(P - A)) <= 1e-13 * np.max(np.abs(A)) * np.sqrt(n)
+    scr = torch.empty(int(L.bem200_getrs_workspace_size(nat.C128, n, nrhs)), dtype=torch.uint8, device="cuda")
+    nat.call("bem200_getrs", nat.C128, 0, n, nrhs, nat.ptr(At), n, nat.ptr(rowmap), nat.ptr(Bt), nrhs, nat.ptr(ws), wsb,
+             nat.ptr(scr), nat.ptr(status), nat.stream_ptr())
+    X = np.linalg.solve(A, B)
+    assert np.max(np.abs(Bt.cpu().numpy() - X)) <= 1e-13 * np.max(np.abs(X)) * np.sqrt(n)
