@@ -508,6 +508,26 @@ int bem200_hmat_matvec_items(int n, int w, const void* x, int nl, const int32_t*
                              const int64_t* doff, const void* D, int nvitems, const int32_t* vitems, int nbitems,
                              const int32_t* bitems, void* y, void* stream);
 
+/* bem200_hmat_operator: the BEM operator of bem200_bem_apply, out = A x (b
+ * NULL) or b - A x for x = [W1 | W2] (npol <= 2), with G1, G2, H1, H2 as four
+ * H-matrices on one block structure (lblk .. doff as above).  D, U, V, rank:
+ * HOST arrays of the four matrices' device pointers (in that order); t_len =
+ * 8 npol sum kcap.  c2p / p2c: cluster <-> particle order.  vitems as in
+ * bem200_hmat_matvec_items; tiles: (first row, rows <= 32, begin, end)
+ * quadruples in cluster order, covering with list[begin .. end) (dense block b
+ * or nd + low-rank block; end - begin <= 128) every row of every block exactly
+ * once.  The sums over
+ * tiles use atomics, as bem200_hmat_matvec_items.  Replaces BEMRetIter._afun
+ * (mnpbem/bem/bem_ret_iter.py:1362-1501) on the H-matrix products. */
+size_t bem200_hmat_operator_workspace_size(int n, int npol, int64_t t_len);
+int bem200_hmat_operator(int n, int npol, const void* x, int eps_per_face, const double* eps1, const double* eps2,
+                         const double* nvec, double k0, const int32_t* c2p, const int32_t* p2c, int nl,
+                         const int32_t* lblk, const int64_t* voff, const int64_t* uoff, const int64_t* toff,
+                         const int32_t* kcap, int64_t t_len, int nd, const int32_t* dblk, const int64_t* doff,
+                         const void* const* D, const void* const* U, const void* const* V, const int32_t* const* rank,
+                         int nvitems, const int32_t* vitems, int ntiles, const int32_t* tiles, const int32_t* list,
+                         void* scratch, const void* b, void* out, void* stream);
+
 /* bem200_hmat_compress_green: the dense leaves and the ACA of the low-rank
  * blocks of BEM matrix `which` (0 = G1, 1 = G2, 2 = H1, 3 = H2) with every
  * entry computed on demand from the Green function, so no n x n matrix is

@@ -845,7 +845,21 @@ __global__ void op_prep_kernel(int n, int p, const double2* __restrict__ W, EpsA
   U[idx] = (c < 4 * p) ? w : cmul(eps_at(eps, i, second), w);
 }
 
-// r = b - A x with GU1 = G1 U1, GU2 = G2 U2, HU1 = H1 U1, HU2 = H2 U2 (n x 8p):
+// Both sides at once with rows in another order (the H-matrix operator):
+// U[side][i] = [s | h | e s | e h] of row map[i]
+__global__ void op_prep_mapped_kernel(int n, int p, const double2* __restrict__ W, EpsArg eps,
+                                      const int32_t* __restrict__ map, double2* __restrict__ U) {
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long per = (long long)n * 8 * p;
+  if (idx >= 2 * per) return;
+  const bool second = idx >= per;
+  const long long e = second ? idx - per : idx;
+  const int i = map[e / (8 * p)], c = (int)(e % (8 * p));
+  const double2 w = W[(second ? 4LL * n * p : 0LL) + (long long)i * 4 * p + (c % (4 * p))];
+  U[idx] = (c < 4 * p) ? w : cmul(eps_at(eps, i, second), w);
+}
+
+// r = b - A x with GU1 = G1 U1, GU2 = G2 U2, HU1 = H1 U1, HU2 = H2 U2 (n x 8p, row i at map[i] when given):
 //   phi   = G1 s1 - G2 s2                          a  = G1 h1 - G2 h2
 //   alpha = H1 h1 - H2 h2 - ik n (G1 e1 s1 - G2 e2 s2)
 //   De    = H1 e1 s1 - H2 e2 s2 - ik n.(G1 e1 h1 - G2 e2 h2)
@@ -855,15 +869,17 @@ __global__ void op_combine_kernel(int n, int p, const double2* __restrict__ GU1,
                                   const double* __restrict__ nvec, double k0, const double2* __restrict__ bphi,
                                   const double2* __restrict__ ba, const double2* __restrict__ balpha,
                                   const double2* __restrict__ bDe, double2* __restrict__ rphi,
-                                  double2* __restrict__ ra, double2* __restrict__ ralpha, double2* __restrict__ rDe) {
+                                  double2* __restrict__ ra, double2* __restrict__ ralpha, double2* __restrict__ rDe,
+                                  const int32_t* __restrict__ map = nullptr) {
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)n * p) return;
   int i = (int)(idx / p), q = (int)(idx % p);
   const int w8 = 8 * p;
-  const double2* g1 = GU1 + (long long)i * w8;
-  const double2* g2 = GU2 + (long long)i * w8;
-  const double2* h1 = HU1 + (long long)i * w8;
-  const double2* h2 = HU2 + (long long)i * w8;
+  const long long mi = (long long)(map ? map[i] : i) * w8;
+  const double2* g1 = GU1 + mi;
+  const double2* g2 = GU2 + mi;
+  const double2* h1 = HU1 + mi;
+  const double2* h2 = HU2 + mi;
   const double2 ik = make_double2(0.0, k0);
   const double nv[3] = {nvec[3 * i], nvec[3 * i + 1], nvec[3 * i + 2]};
   const double sgn = bphi ? -1.0 : 1.0;
@@ -885,6 +901,41 @@ __global__ void op_combine_kernel(int n, int p, const double2* __restrict__ GU1,
   rphi[idx] = bphi ? csub(bphi[idx], phi) : phi;
   rDe[idx] = bphi ? csub(bDe[idx], De) : De;
   (void)sgn;
+}
+
+// The two ends of the operator for callers whose products are in another row
+// order: U (2 x n x 8p) from x = (W1, W2) at c2p, and r = A x (b null) or b - A x
+// from Y = [G1 U1 | G2 U2 | H1 U1 | H2 U2] (4 x n x 8p) at p2c.
+static EpsArg make_eps(int per_face, const double* e1, const double* e2) {
+  EpsArg e;
+  e.per_face = per_face;
+  e.d1 = nullptr;
+  e.d2 = nullptr;
+  if (per_face) {
+    e.d1 = reinterpret_cast<const double2*>(e1);
+    e.d2 = reinterpret_cast<const double2*>(e2);
+    e.e1 = e.e2 = make_double2(0, 0);
+  } else {
+    e.e1 = make_double2(e1[0], e1[1]);
+    e.e2 = make_double2(e2[0], e2[1]);
+  }
+  return e;
+}
+
+int op_prep_mapped(cudaStream_t st, int n, int p, const double2* x, int eps_per_face, const double* eps1,
+                   const double* eps2, const int32_t* c2p, double2* U) {
+  op_prep_mapped_kernel<<<ceil_div(16LL * n * p, 256), 256, 0, st>>>(n, p, x, make_eps(eps_per_face, eps1, eps2), c2p, U);
+  BEM_LAUNCH_CHECK();
+  return BEM200_OK;
+}
+int op_combine_mapped(cudaStream_t st, int n, int p, const double2* Y, const double* nvec, double k0, const double2* b,
+                      const int32_t* p2c, double2* r) {
+  const long long np = (long long)n * p, per = 8 * np;
+  op_combine_kernel<<<ceil_div(np, 256), 256, 0, st>>>(n, p, Y, Y + per, Y + 2 * per, Y + 3 * per, nvec, k0, b,
+                                                       b ? b + np : nullptr, b ? b + 4 * np : nullptr,
+                                                       b ? b + 7 * np : nullptr, r, r + np, r + 4 * np, r + 7 * np, p2c);
+  BEM_LAUNCH_CHECK();
+  return BEM200_OK;
 }
 
 // A x (or b - A x) for x = (W1 = [s1|h1], W2 = [s2|h2]); scratch: 40 n p complex128
@@ -954,22 +1005,6 @@ static int absmax_host(cudaStream_t s, long long n, const double2* x, unsigned l
 }  // namespace bem200
 
 using namespace bem200;
-
-static EpsArg make_eps(int per_face, const double* e1, const double* e2) {
-  EpsArg e;
-  e.per_face = per_face;
-  e.d1 = nullptr;
-  e.d2 = nullptr;
-  if (per_face) {
-    e.d1 = reinterpret_cast<const double2*>(e1);
-    e.d2 = reinterpret_cast<const double2*>(e2);
-    e.e1 = e.e2 = make_double2(0, 0);
-  } else {
-    e.e1 = make_double2(e1[0], e1[1]);
-    e.e2 = make_double2(e2[0], e2[1]);
-  }
-  return e;
-}
 
 static GemmEngine engine_from(int e) {
   return e == 1 ? GemmEngine::kTc : (e == 2 ? GemmEngine::kTf32 : GemmEngine::kSimt);

@@ -458,6 +458,218 @@ __global__ void __launch_bounds__(kHThreads) hmat_block_items_kernel(
   }
 }
 
+// ------------------------------------------------------- four matrices at once
+// The BEM operator multiplies G1, G2, H1, H2 -- four H-matrices on one block
+// structure -- with the w = 8 npol columns of two sides (G1, H1: side 0; G2, H2:
+// side 1).  One launch per phase covers all four (blockIdx.y): a single
+// matrix's items cannot fill the GPU (65 - 72 us per phase and matrix at 3600
+// faces, for 13 us of memory traffic).
+//   phase A (hmat_vt4_kernel): item (l, j0), rows [j0, j0 + kVtRows) of V_l; warps
+//     own 32 outputs (i, q) of T_l each and split the rows when there are fewer
+//     outputs than threads; partial sums are added into T_l with atomics.
+//   phase B (hmat_rows4_kernel): item = up to 32 rows of one leaf cluster and a
+//     run of the blocks that cover them.  The rows' sums over all blocks of the
+//     run stay in registers and go into y with one atomic per item instead of
+//     one per block (about 40 blocks cover a row).
+struct HMat4 {
+  const double2* D[4];
+  const double2* U[4];
+  const double2* V[4];
+  const int32_t* rank[4];
+};
+
+template <int W>
+__global__ void __launch_bounds__(kHThreads) hmat_vt4_kernel(
+    const int32_t* __restrict__ items, int n, int w, const int32_t* __restrict__ blk, const int64_t* __restrict__ voff,
+    const int64_t* __restrict__ toff, const int32_t* __restrict__ kcap_arr, const __grid_constant__ HMat4 H,
+    const double2* __restrict__ X, double2* __restrict__ Tall, long long t_len) {
+  __shared__ double2 xs[kVtRows][W + 1];
+  __shared__ double2 red[kHThreads / 32][32];
+  const int mat = blockIdx.y;
+  const int l = items[2 * blockIdx.x], j0 = items[2 * blockIdx.x + 1];
+  const int c0 = blk[4 * l + 2], nb = blk[4 * l + 3];
+  const int kc = kcap_arr[l], rw = H.rank[mat][l] * w;
+  const int jn = min(kVtRows, nb - j0);
+  const double2* V = H.V[mat] + voff[l] + (long long)j0 * kc;
+  const double2* x = X + (mat & 1) * (long long)n * w + (long long)(c0 + j0) * w;
+  double2* Tb = Tall + mat * t_len + toff[l] * w;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  for (int e = tid; e < jn * w; e += kHThreads) xs[e / w][e % w] = x[e];
+  __syncthreads();
+  constexpr int NW = kHThreads / 32;
+  const int tiles = (rw + 31) / 32;
+  int split = 1;  // warps per output tile
+  while (2 * split * tiles <= NW) split *= 2;
+  const int rounds = (tiles + NW / split - 1) / (NW / split);
+  for (int t0 = 0; t0 < rounds; ++t0) {
+    const int t = t0 * (NW / split) + wid / split, part = wid % split;
+    const int o = 32 * t + lane;
+    double2 acc = make_double2(0, 0);
+    if (o < rw) {
+      const int lo = o / w, q = o - lo * w;
+      const double2* v = V + lo;
+#pragma unroll 8
+      for (int jj = part; jj < jn; jj += split) {
+        const double2 a = v[(long long)jj * kc], b = xs[jj][q];
+        acc.x = fma(-a.y, b.y, fma(a.x, b.x, acc.x));
+        acc.y = fma(a.y, b.x, fma(a.x, b.y, acc.y));
+      }
+    }
+    if (split > 1) {
+      red[wid][lane] = acc;
+      __syncthreads();
+      if (part == 0)
+        for (int k = 1; k < split; ++k) acc = cadd(acc, red[wid + k][lane]);
+      __syncthreads();
+    }
+    if (part == 0 && o < rw) {
+      double* out = reinterpret_cast<double*>(Tb + o);
+      atomicAdd(out, acc.x);
+      atomicAdd(out + 1, acc.y);
+    }
+  }
+}
+
+constexpr int kRunBlocks = 128;  // blocks of a run at most
+
+template <int W>
+__global__ void __launch_bounds__(kHThreads) hmat_rows4_kernel(
+    const int32_t* __restrict__ items, const int32_t* __restrict__ list, int nd, int n,
+    const int32_t* __restrict__ lblk, const int64_t* __restrict__ uoff, const int64_t* __restrict__ toff,
+    const int32_t* __restrict__ kcap_arr, const int32_t* __restrict__ dblk, const int64_t* __restrict__ doff,
+    const __grid_constant__ HMat4 H, const double2* __restrict__ X, const double2* __restrict__ Tall, long long t_len,
+    double2* __restrict__ Y) {
+  // The columns of the run's blocks (dense columns, low-rank terms) are taken as
+  // one sequence, staged kSChunk at a time: the right-hand rows, and where
+  // column j's matrix entries of row 0 are and how far apart rows lie.
+  __shared__ double2 Ss[kSChunk][W + 1];
+  __shared__ const double2* colp[kSChunk];
+  __shared__ int cold[kSChunk];
+  __shared__ const double2* bM[kRunBlocks];
+  __shared__ const double2* bS[kRunBlocks];
+  __shared__ int bld[kRunBlocks], bend[kRunBlocks];
+  const int mat = blockIdx.y;
+  const int row0 = items[4 * blockIdx.x], nrow = items[4 * blockIdx.x + 1];
+  const int l0 = items[4 * blockIdx.x + 2], nblk = items[4 * blockIdx.x + 3] - l0;
+  const double2* x = X + (mat & 1) * (long long)n * W;
+  const double2* T = Tall + mat * t_len;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (tid < nblk) {
+    const int b = list[l0 + tid];
+    if (b < nd) {
+      const int K = dblk[4 * b + 3];
+      bld[tid] = K;
+      bend[tid] = K;
+      bM[tid] = H.D[mat] + doff[b] + (long long)(row0 - dblk[4 * b]) * K;
+      bS[tid] = x + (long long)dblk[4 * b + 2] * W;
+    } else {
+      const int l = b - nd, ld = kcap_arr[l];
+      bld[tid] = ld;
+      bend[tid] = H.rank[mat][l];
+      bM[tid] = H.U[mat] + uoff[l] + (long long)(row0 - lblk[4 * l]) * ld;
+      bS[tid] = T + toff[l] * W;
+    }
+  }
+  __syncthreads();
+  if (wid == 0) {  // inclusive prefix sums of the column counts
+    int carry = 0;
+    for (int k = 0; k < nblk; k += 32) {
+      int v = k + lane < nblk ? bend[k + lane] : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+      }
+      v += carry;
+      if (k + lane < nblk) bend[k + lane] = v;
+      carry = __shfl_sync(0xffffffffu, v, 31);
+    }
+  }
+  __syncthreads();
+  const int total = nblk ? bend[nblk - 1] : 0;
+  const int js = lane & 7, rs = lane >> 3;  // 8 lanes per row, 4 rows per warp
+  const int rl = 4 * wid + rs;
+  const bool rok = rl < nrow;
+  double2 acc[W];
+#pragma unroll
+  for (int q = 0; q < W; ++q) acc[q] = make_double2(0, 0);
+  for (int k0 = 0; k0 < total; k0 += kSChunk) {
+    const int kn = min(kSChunk, total - k0);
+    if (k0) __syncthreads();
+    for (int e = tid; e < kn * 2; e += kHThreads) {  // two threads per column, half of its W values each
+      const int j = e >> 1, h = e & 1;
+      int lo = 0, hi = nblk - 1;
+      while (lo < hi) {  // first block that ends beyond column k0 + j
+        const int mid = (lo + hi) >> 1;
+        if (bend[mid] > k0 + j) hi = mid; else lo = mid + 1;
+      }
+      const int c = k0 + j - (lo ? bend[lo - 1] : 0);
+      const double2* src = bS[lo] + (long long)c * W;
+#pragma unroll
+      for (int q = 0; q < W / 2; ++q) Ss[j][h * (W / 2) + q] = src[h * (W / 2) + q];
+      if (h == 0) {
+        colp[j] = bM[lo] + c;
+        cold[j] = bld[lo];
+      }
+    }
+    __syncthreads();
+    if (rok) {
+#pragma unroll 4
+      for (int j = js; j < kn; j += 8) {
+        const double2 a = __ldcs(colp[j] + (long long)rl * cold[j]);
+#pragma unroll
+        for (int q = 0; q < W; ++q) {
+          const double2 c = Ss[j][q];
+          acc[q].x = fma(-a.y, c.y, fma(a.x, c.x, acc[q].x));
+          acc[q].y = fma(a.y, c.x, fma(a.x, c.y, acc[q].y));
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < W; ++q) {
+    double2 v = acc[q];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+      v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+    }
+    acc[q] = v;
+  }
+  if (rok) {
+#pragma unroll
+    for (int q = 0; q < W; ++q)
+      if (q % 8 == js) {
+        double* out = reinterpret_cast<double*>(Y + mat * (long long)n * W + (long long)(row0 + rl) * W + q);
+        atomicAdd(out, acc[q].x);
+        atomicAdd(out + 1, acc[q].y);
+      }
+  }
+}
+
+// defined in bem.cu
+int op_prep_mapped(cudaStream_t st, int n, int p, const double2* x, int eps_per_face, const double* eps1,
+                   const double* eps2, const int32_t* c2p, double2* U);
+int op_combine_mapped(cudaStream_t st, int n, int p, const double2* Y, const double* nvec, double k0, const double2* b,
+                      const int32_t* p2c, double2* r);
+
+template <int W>
+static int hmat_apply4(cudaStream_t s, int n, int w, const HMat4& H, int nvitems, const int32_t* vitems, const int32_t* lblk,
+                       const int64_t* voff, const int64_t* uoff, const int64_t* toff, const int32_t* kcap, int nd,
+                       const int32_t* dblk, const int64_t* doff, int ntiles, const int32_t* tiles, const int32_t* list,
+                       const double2* X, double2* T, long long t_len, double2* Y) {
+  if (nvitems > 0) {
+    hmat_vt4_kernel<W><<<dim3(nvitems, 4), kHThreads, 0, s>>>(vitems, n, w, lblk, voff, toff, kcap, H, X, T, t_len);
+    BEM_LAUNCH_CHECK();
+  }
+  if (ntiles > 0) {
+    hmat_rows4_kernel<W><<<dim3(ntiles, 4), kHThreads, 0, s>>>(tiles, list, nd, n, lblk, uoff, toff, kcap, dblk, doff, H, X, T,
+                                                               t_len, Y);
+    BEM_LAUNCH_CHECK();
+  }
+  return BEM200_OK;
+}
+
 }  // namespace bem200
 
 using namespace bem200;
@@ -618,6 +830,48 @@ int bem200_hmat_matvec_items(int n, int w, const void* x, int nl, const int32_t*
                                                               doff, (const double2*)D, (double2*)y);
   BEM_LAUNCH_CHECK();
   return BEM200_OK;
+}
+
+size_t bem200_hmat_operator_workspace_size(int n, int npol, int64_t t_len) {
+  if (n <= 0 || npol <= 0 || t_len < 0) return 0;
+  return sizeof(double2) * ((size_t)6 * n * 8 * npol + 4 * (size_t)t_len);
+}
+
+int bem200_hmat_operator(int n, int npol, const void* x, int eps_per_face, const double* eps1, const double* eps2,
+                         const double* nvec, double k0, const int32_t* c2p, const int32_t* p2c, int nl,
+                         const int32_t* lblk, const int64_t* voff, const int64_t* uoff, const int64_t* toff,
+                         const int32_t* kcap, int64_t t_len, int nd, const int32_t* dblk, const int64_t* doff,
+                         const void* const* D, const void* const* U, const void* const* V, const int32_t* const* rank,
+                         int nvitems, const int32_t* vitems, int ntiles, const int32_t* tiles, const int32_t* list,
+                         void* scratch, const void* b, void* out, void* stream) {
+  BEM_REQUIRE(n > 0 && npol > 0 && x && eps1 && eps2 && nvec && c2p && p2c && D && U && V && rank && scratch && out &&
+                  nl >= 0 && nd >= 0 && t_len >= 0 && nvitems >= 0 && ntiles >= 0,
+              BEM200_ERR_ARG, "hmat_operator: bad arguments");
+  BEM_REQUIRE((nvitems == 0 || (vitems && lblk && voff && uoff && toff && kcap)) && (ntiles == 0 || (tiles && list)) &&
+                  (nd == 0 || (dblk && doff)),
+              BEM200_ERR_ARG, "hmat_operator: block tables missing");
+  BEM_REQUIRE(npol <= 2, BEM200_ERR_UNSUPPORTED, "hmat_operator: at most 2 polarisations (16 columns)");
+  cudaStream_t s = (cudaStream_t)stream;
+  const int w = 8 * npol;
+  double2* X = reinterpret_cast<double2*>(scratch);  // 2 x n x w
+  double2* T = X + 2 * (size_t)n * w;                // 4 x t_len
+  double2* Y = T + 4 * (size_t)t_len;                // 4 x n x w
+  HMat4 H;
+  for (int k = 0; k < 4; ++k) {
+    H.D[k] = (const double2*)D[k];
+    H.U[k] = (const double2*)U[k];
+    H.V[k] = (const double2*)V[k];
+    H.rank[k] = rank[k];
+  }
+  int st = op_prep_mapped(s, n, npol, (const double2*)x, eps_per_face, eps1, eps2, c2p, X);
+  if (st) return st;
+  BEM_CUDA_CHECK(cudaMemsetAsync(T, 0, sizeof(double2) * (4 * (size_t)t_len + 4 * (size_t)n * w), s));
+  st = npol == 1 ? hmat_apply4<8>(s, n, w, H, nvitems, vitems, lblk, voff, uoff, toff, kcap, nd, dblk, doff, ntiles, tiles,
+                                  list, X, T, t_len, Y)
+                 : hmat_apply4<16>(s, n, w, H, nvitems, vitems, lblk, voff, uoff, toff, kcap, nd, dblk, doff, ntiles, tiles,
+                                   list, X, T, t_len, Y);
+  if (st) return st;
+  return op_combine_mapped(s, n, npol, Y, nvec, k0, (const double2*)b, p2c, (double2*)out);
 }
 
 }  // extern "C"

@@ -144,12 +144,20 @@ def make_kaware_fadmiss(k, eta0=2.5):
         if ka * rmin > 1.0 and d < lam:
             return False
         return True
+
+    def many(r1, r2, d):  # the same test on arrays
+        rmin = np.minimum(r1, r2)
+        return ~((eta0 * rmin >= d) | ((ka * rmin > 1.0) & (d < lam)))
+    fadmiss.many = many
     return fadmiss
 
 
 def block_partition(tree, fadmiss):
     """Dense (leaf x leaf) and low-rank (admissible) cluster pairs, in the
     reference's recursion order (clustertree.py:324-376)."""
+    many = getattr(fadmiss, "many", None)
+    if many is not None:
+        return _block_partition_arrays(tree, many)
     dense, lowrank = [], []
 
     def admissible(i1, i2):
@@ -175,7 +183,111 @@ def block_partition(tree, fadmiss):
     return dense, lowrank
 
 
+def _block_partition_arrays(tree, many):
+    """The same recursion, one level of all pairs at a time: a pair is replaced
+    in place by its son pairs, so the sequence stays in recursion order."""
+    leaf = tree.son[:, 0] == -1
+    i1 = i2 = np.zeros(1, dtype=np.int64)
+    kind = np.zeros(1, dtype=np.int8)  # 0 open, 1 low rank, 2 dense
+    while True:
+        o = np.flatnonzero(kind == 0)
+        if len(o) == 0:
+            break
+        a, b = i1[o], i2[o]
+        both = leaf[a] & leaf[b]
+        d = np.sqrt(np.sum((tree.mid[a] - tree.mid[b]) ** 2, axis=1))
+        adm = (tree.ipart[a] != -1) & (tree.ipart[b] != -1) & many(tree.rad[a], tree.rad[b], d)
+        kind[o] = np.where(both, 2, np.where(adm, 1, 0))
+        n1 = np.where(leaf[i1], 1, 2)
+        n2 = np.where(leaf[i2], 1, 2)
+        reps = np.where(kind == 0, n1 * n2, 1)
+        src = np.repeat(np.arange(len(kind)), reps)
+        pos = np.arange(len(src)) - np.repeat(np.cumsum(reps) - reps, reps)  # son pair within its parent
+        grow = kind[src] == 0
+        p1, p2 = pos // n2[src], pos % n2[src]
+        j1 = np.where(grow & ~leaf[i1[src]], tree.son[i1[src], np.minimum(p1, 1)], i1[src])
+        j2 = np.where(grow & ~leaf[i2[src]], tree.son[i2[src], np.minimum(p2, 1)], i2[src])
+        i1, i2, kind = j1, j2, kind[src]
+    pairs = np.stack([i1, i2], axis=1)
+    return ([tuple(v) for v in pairs[kind == 2].tolist()], [tuple(v) for v in pairs[kind == 1].tolist()])
+
+
 # --------------------------------------------------------------------------- device H-matrix
+class _Layout:
+    """Block structure of H-matrices on one partition: block tables, storage
+    offsets and work items, on the host and on the device."""
+
+    _RUN = 512
+
+    def __init__(self, tree, dense, lowrank, kmax, dev):
+        torch = _torch()
+        lo = tree.cind[:, 0].astype(np.int32)
+        ln = (tree.cind[:, 1] - tree.cind[:, 0] + 1).astype(np.int32)
+
+        def table(pairs):
+            p = np.asarray(pairs, dtype=np.int64).reshape(-1, 2)
+            a, b = p[:, 0], p[:, 1]
+            return np.ascontiguousarray(np.stack([lo[a], ln[a], lo[b], ln[b]], axis=1))
+
+        # dense leaves (r0, m, c0, nb) and packed offsets; low-rank blocks,
+        # storage for the maximum rank min(m, nb, kmax)
+        self.db, self.lb = db, lb = table(dense), table(lowrank)
+        self.kcap = kcap = np.minimum(np.minimum(lb[:, 1], lb[:, 3]), kmax).astype(np.int64)
+
+        def offsets(sizes):
+            off = np.zeros(len(sizes) + 1, dtype=np.int64)
+            off[1:] = np.cumsum(sizes)
+            return off
+        self.doff, self.uoff = offsets(db[:, 1].astype(np.int64) * db[:, 3]), offsets(lb[:, 1].astype(np.int64) * kcap)
+        self.voff, self.toff = offsets(lb[:, 3].astype(np.int64) * kcap), offsets(kcap)
+
+        def split(rows, step, first=0):  # (block, first row) for every `step` rows of every block
+            cnt = (rows.astype(np.int64) + step - 1) // step
+            blk = np.repeat(np.arange(len(rows)), cnt)
+            j = np.arange(len(blk)) - np.repeat(np.cumsum(cnt) - cnt, cnt)
+            return np.stack([blk + first, j * step], axis=1).astype(np.int32)
+        vit = split(lb[:, 3], 128)
+        bit = np.concatenate([split(db[:, 1], 32), split(lb[:, 1], 32, first=len(db))])
+        tiles, blist = self._row_tiles(tree, lo, ln)
+        t = lambda a: torch.as_tensor(np.ascontiguousarray(a), device=dev)
+        self.dev = {k: t(v) for k, v in dict(
+            dblk=db.reshape(-1), doff=self.doff, lblk=lb.reshape(-1), uoff=self.uoff, voff=self.voff, toff=self.toff,
+            kcap=kcap.astype(np.int32), c2p=tree.ind[:, 0].astype(np.int32), p2c=tree.ind[:, 1].astype(np.int32),
+            vitems=vit.reshape(-1), bitems=bit.reshape(-1), tiles=tiles.reshape(-1), blist=blist).items()}
+        self.nvitems, self.nbitems, self.ntiles = len(vit), len(bit), len(tiles)
+
+    def _row_tiles(self, tree, lo, ln):
+        """Phase B of the operator product: up to 32 rows of a leaf cluster with
+        a run of at most 128 of the blocks over them (every block's rows are a
+        union of whole leaf clusters), about _RUN matrix columns per run."""
+        leaf = np.flatnonzero(tree.son[:, 0] == -1)
+        leaf = leaf[np.argsort(lo[leaf], kind="stable")]
+        start = lo[leaf]
+        blocks = np.concatenate([self.db, self.lb])
+        cost = np.concatenate([self.db[:, 3].astype(np.int64), np.minimum(self.kcap, 24)]) + 8
+        # leaves covered by each block
+        f = np.searchsorted(start, blocks[:, 0])
+        e = np.searchsorted(start, blocks[:, 0] + blocks[:, 1])
+        cnt = e - f
+        blk = np.repeat(np.arange(len(blocks)), cnt)
+        lf = np.arange(len(blk)) - np.repeat(np.cumsum(cnt) - cnt, cnt) + np.repeat(f, cnt)
+        order = np.lexsort((blk, lf))
+        blk, lf = blk[order].astype(np.int32), lf[order]
+        begin = np.searchsorted(lf, np.arange(len(leaf)))
+        c = np.cumsum(cost[blk]) if len(blk) else np.zeros(0, np.int64)
+        base = np.concatenate([[0], c])[begin] if len(blk) else np.zeros(len(leaf), np.int64)
+        run = (c - cost[blk] - base[lf]) // self._RUN if len(blk) else c
+        head = np.flatnonzero(np.concatenate([[True], (lf[1:] != lf[:-1]) | (run[1:] != run[:-1])])) if len(blk) else \
+            np.zeros(0, np.int64)
+        tail = np.concatenate([head[1:], [len(blk)]]).astype(np.int64) if len(head) else head
+        rows, first = ln[leaf][lf[head]].astype(np.int64), start[lf[head]].astype(np.int64)
+        parts = (rows + 31) // 32
+        src = np.repeat(np.arange(len(head)), parts)
+        k = np.arange(len(src)) - np.repeat(np.cumsum(parts) - parts, parts)
+        tiles = np.stack([first[src] + 32 * k, np.minimum(32, rows[src] - 32 * k), head[src], tail[src]], axis=1)
+        return tiles.astype(np.int32), blk
+
+
 class HMatrixGPU:
     """Compressed n x n complex128 matrix on the device (cluster order).
 
@@ -183,7 +295,7 @@ class HMatrixGPU:
     computes y = H x for n x w row-major device arrays in cluster order.
     """
 
-    def __init__(self, tree, dense, lowrank, htol=1e-6, kmax=100, device="cuda"):
+    def __init__(self, tree, dense, lowrank, htol=1e-6, kmax=100, device="cuda", layout=None):
         torch = _torch()
         self.tree = tree
         self.n = tree.n
@@ -191,46 +303,18 @@ class HMatrixGPU:
         self.kmax = int(kmax)
         dev = torch.device(device)
         self.dev = dev
-        cind = tree.cind
-
-        def rng(i):
-            return int(cind[i, 0]), int(cind[i, 1] - cind[i, 0] + 1)
-
-        # dense leaves: (r0, m, c0, nb) and packed offsets
-        db = np.array([[*rng(a), *rng(b)] for a, b in dense], dtype=np.int32).reshape(-1, 4)
-        doff = np.zeros(len(db) + 1, dtype=np.int64)
-        doff[1:] = np.cumsum(db[:, 1].astype(np.int64) * db[:, 3])
-        # low-rank blocks, storage for the maximum rank min(m, nb, kmax)
-        lb = np.array([[*rng(a), *rng(b)] for a, b in lowrank], dtype=np.int32).reshape(-1, 4)
-        kcap = np.minimum(np.minimum(lb[:, 1], lb[:, 3]), self.kmax).astype(np.int64)
-        uoff = np.zeros(len(lb) + 1, dtype=np.int64)
-        uoff[1:] = np.cumsum(lb[:, 1].astype(np.int64) * kcap)
-        voff = np.zeros(len(lb) + 1, dtype=np.int64)
-        voff[1:] = np.cumsum(lb[:, 3].astype(np.int64) * kcap)
-        toff = np.zeros(len(lb) + 1, dtype=np.int64)
-        toff[1:] = np.cumsum(kcap)
-        self.ndense, self.nlow = len(db), len(lb)
-        self._db, self._lb, self._kcap = db, lb, kcap
-        self._doff_h, self._uoff_h, self._voff_h = doff, uoff, voff
-        t = lambda a: torch.as_tensor(np.ascontiguousarray(a), device=dev)
-        self.dblk, self.doff = t(db.reshape(-1)), t(doff)
-        self.lblk, self.uoff, self.voff, self.toff = t(lb.reshape(-1)), t(uoff), t(voff), t(toff)
-        self.kcap = t(kcap.astype(np.int32))
-        self.D = torch.empty(max(int(doff[-1]), 1), dtype=torch.complex128, device=dev)
-        self.U = torch.empty(max(int(uoff[-1]), 1), dtype=torch.complex128, device=dev)
-        self.V = torch.empty(max(int(voff[-1]), 1), dtype=torch.complex128, device=dev)
-        self.rank = torch.zeros(max(len(lb), 1), dtype=torch.int32, device=dev)
-        self.c2p = t(tree.ind[:, 0].astype(np.int32))
-        self.p2c = t(tree.ind[:, 1].astype(np.int32))
+        self.layout = L = layout if layout is not None else _Layout(tree, dense, lowrank, self.kmax, dev)
+        self.ndense, self.nlow = len(L.db), len(L.lb)
+        self._db, self._lb, self._kcap = L.db, L.lb, L.kcap
+        self._doff_h, self._uoff_h, self._voff_h = L.doff, L.uoff, L.voff
+        for k in ("dblk", "doff", "lblk", "uoff", "voff", "toff", "kcap", "c2p", "p2c", "vitems", "bitems"):
+            setattr(self, k, L.dev[k])
+        self.nvitems, self.nbitems = L.nvitems, L.nbitems
+        self.D = torch.empty(max(int(L.doff[-1]), 1), dtype=torch.complex128, device=dev)
+        self.U = torch.empty(max(int(L.uoff[-1]), 1), dtype=torch.complex128, device=dev)
+        self.V = torch.empty(max(int(L.voff[-1]), 1), dtype=torch.complex128, device=dev)
+        self.rank = torch.zeros(max(self.nlow, 1), dtype=torch.int32, device=dev)
         self.ranks = None
-        # work items of the product: (low-rank block, first V row) per 128 rows
-        # of V, and (block, first row) per 32 rows of every block (dense first)
-        vit = [(l, j0) for l in range(len(lb)) for j0 in range(0, int(lb[l, 3]), 128)]
-        bit = [(b, i0) for b in range(len(db)) for i0 in range(0, int(db[b, 1]), 32)]
-        bit += [(len(db) + l, i0) for l in range(len(lb)) for i0 in range(0, int(lb[l, 1]), 32)]
-        self.nvitems, self.nbitems = len(vit), len(bit)
-        self.vitems = t(np.array(vit, dtype=np.int32).reshape(-1))
-        self.bitems = t(np.array(bit, dtype=np.int32).reshape(-1))
 
     def compress(self, M, scratch=None):
         """Compress the dense n x n complex128 device matrix M (particle order)."""
@@ -252,11 +336,12 @@ class HMatrixGPU:
             self.ranks = np.zeros(0, dtype=np.int32)
         return self
 
-    def compress_green(self, g, enei, which):
+    def compress_green(self, g, enei, which, fetch=True):
         """Compress BEM matrix ``which`` (0 = G1, 1 = G2, 2 = H1, 3 = H2) of the
         Green function ``g`` (a CompGreenRet) at ``enei`` with every entry of the
         dense leaves and of the ACA rows and columns computed on demand: no
-        n x n matrix is formed (bem200_hmat_compress_green)."""
+        n x n matrix is formed (bem200_hmat_compress_green).  fetch=False leaves
+        the ranks on the device (``fetch_ranks`` reads them later)."""
         ks = g.wavenumbers(enei)
         kmat = (ctypes.c_double * (2 * len(ks)))(*[v for k in ks for v in (k.real, k.imag)])
         blk = g._blk_mat([(0, 0), (1, 0), (1, 1), (0, 1)])
@@ -271,6 +356,9 @@ class HMatrixGPU:
                  self.ndense, nat.ptr(self.dblk), nat.ptr(self.doff), nat.ptr(self.D), self.nlow, nat.ptr(self.lblk),
                  nat.ptr(self.uoff), nat.ptr(self.voff), nat.ptr(self.kcap), self.htol, nat.ptr(self.U),
                  nat.ptr(self.V), nat.ptr(self.rank), max_rows, max_kcap, nat.stream_ptr())
+        return self.fetch_ranks() if fetch else self
+
+    def fetch_ranks(self):
         self.ranks = self.rank.cpu().numpy()[:self.nlow].copy() if self.nlow else np.zeros(0, dtype=np.int32)
         return self
 
@@ -350,8 +438,21 @@ class BEMHMatrices:
         dev = self.g.device
         if mats is None and fill == "green":
             self.H = None
-            self.H = [HMatrixGPU(self.tree, dense, low, htol=self.htol, kmax=self.kmax).compress_green(self.g, enei, w)
-                      for w in range(4)]
+            layout = _Layout(self.tree, dense, low, self.kmax, dev)
+            self.H = [HMatrixGPU(self.tree, dense, low, htol=self.htol, kmax=self.kmax, layout=layout)
+                      for _ in range(4)]
+            # the four fills side by side: each is paced by its few largest
+            # blocks (one CTA per block, 1.1 ms at 3600 faces)
+            cur = torch.cuda.current_stream()
+            sides = [torch.cuda.Stream() for _ in range(4)]
+            for w, (h, s) in enumerate(zip(self.H, sides)):
+                s.wait_stream(cur)
+                with torch.cuda.stream(s):
+                    h.compress_green(self.g, enei, w, fetch=False)
+            for s in sides:
+                cur.wait_stream(s)
+            for h in self.H:
+                h.fetch_ranks()
             self.enei = enei
             return self
         if fill not in ("green", "dense"):
@@ -361,7 +462,9 @@ class BEMHMatrices:
             self.g.bem_matrices(enei, dtype="c128", out=mats)
         self.H = None
         scratch = torch.empty((n, n), dtype=torch.complex128, device=dev)
-        self.H = [HMatrixGPU(self.tree, dense, low, htol=self.htol, kmax=self.kmax).compress(M, scratch) for M in mats]
+        layout = _Layout(self.tree, dense, low, self.kmax, dev)
+        self.H = [HMatrixGPU(self.tree, dense, low, htol=self.htol, kmax=self.kmax, layout=layout).compress(M, scratch)
+                  for M in mats]
         del mats, scratch
         self.enei = enei
         return self
@@ -373,26 +476,18 @@ class BEMHMatrices:
         """out = A x (the full BEM operator) for x in the solution layout."""
         torch = _torch()
         n = self.n
-        w = 8 * npol
-        np_ = n * npol
-        dev = x.device
-        key = npol
-        if getattr(self, "_bufkey", None) != key:
-            self._U = [torch.empty((n, w), dtype=torch.complex128, device=dev) for _ in range(2)]
-            self._Uc = [torch.empty((n, w), dtype=torch.complex128, device=dev) for _ in range(2)]
-            self._Yc = torch.empty((n, w), dtype=torch.complex128, device=dev)
-            self._Y = [torch.empty((n, w), dtype=torch.complex128, device=dev) for _ in range(4)]
-            self._bufkey = key
-        s = nat.stream_ptr()
-        base = x.data_ptr()
-        c2p, p2c = self.H[0].c2p, self.H[0].p2c
-        for side in range(2):
-            nat.call("bem200_op_prep", n, npol, ctypes.c_void_p(base + 16 * 4 * np_ * side), eps_mode, e1p, e2p,
-                     side, nat.ptr(self._U[side]), s)
-            nat.call("bem200_hmat_gather_rows", n, w, nat.ptr(self._U[side]), nat.ptr(c2p), nat.ptr(self._Uc[side]), s)
-        # G1 U1, G2 U2, H1 U1, H2 U2 in cluster order, back to particle order
-        for i, (h, side) in enumerate(zip(self.H, (0, 1, 0, 1))):
-            h.matvec(self._Uc[side], self._Yc, w)
-            nat.call("bem200_hmat_gather_rows", n, w, nat.ptr(self._Yc), nat.ptr(p2c), nat.ptr(self._Y[i]), s)
-        nat.call("bem200_op_combine", n, npol, nat.ptr(self._Y[0]), nat.ptr(self._Y[1]), nat.ptr(self._Y[2]),
-                 nat.ptr(self._Y[3]), nat.ptr(nvec), k0, None, nat.ptr(out), s)
+        L = self.H[0].layout
+        d = L.dev
+        t_len = int(L.toff[-1]) * 8 * npol
+        need = int(nat.lib().bem200_hmat_operator_workspace_size(n, npol, t_len))
+        buf = getattr(self, "_opbuf", None)
+        if buf is None or buf.numel() < need:
+            self._opbuf = buf = torch.empty(need, dtype=torch.uint8, device=x.device)
+
+        def four(name):
+            return (ctypes.c_void_p * 4)(*[getattr(h, name).data_ptr() for h in self.H])
+        nat.call("bem200_hmat_operator", n, npol, nat.ptr(x), eps_mode, e1p, e2p, nat.ptr(nvec), k0, nat.ptr(d["c2p"]),
+                 nat.ptr(d["p2c"]), len(L.lb), nat.ptr(d["lblk"]), nat.ptr(d["voff"]), nat.ptr(d["uoff"]),
+                 nat.ptr(d["toff"]), nat.ptr(d["kcap"]), t_len, len(L.db), nat.ptr(d["dblk"]), nat.ptr(d["doff"]),
+                 four("D"), four("U"), four("V"), four("rank"), L.nvitems, nat.ptr(d["vitems"]), L.ntiles,
+                 nat.ptr(d["tiles"]), nat.ptr(d["blist"]), nat.ptr(buf), None, nat.ptr(out), nat.stream_ptr())
