@@ -167,16 +167,6 @@ static int* lu_flag_of(int32_t* snap, int n) {
 // the latency-bound panel factorisations of the two chains overlap.  Each
 // chain gets its own half of the tensor-core operand workspace; Sigma2 uses
 // the Delta slot (free until the join) as its scratch matrix.
-struct ForkJoin {
-  cudaStream_t side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
-  ~ForkJoin() {
-    if (fork) cudaEventDestroy(fork);
-    if (join) cudaEventDestroy(join);
-    if (side) cudaStreamDestroy(side);  // released once its queued work has finished
-  }
-};
-
 // Optional CUDA-event stage timer of the init: events at the start and after
 // each phase, recorded on the caller's stream.
 struct StageTimer {
@@ -256,16 +246,14 @@ static int bem_init_t(const LaContext& ctx, int n, void* ws, const EpsArg& eps, 
   const int half = n / 2 + 64;
   const bool split_ws = ctx.engine != GemmEngine::kSimt;
   const bool fork = gemm_tc_two_fit<C>(ctx, n, half, half);
-  ForkJoin fj;
+  StreamLease fj;
   LaContext c2 = c;
   c2.dinfo = s.verdict + 1;
   if (fork) {
-    BEM_CUDA_CHECK(cudaStreamCreateWithFlags(&fj.side, cudaStreamNonBlocking));
-    BEM_CUDA_CHECK(cudaEventCreateWithFlags(&fj.fork, cudaEventDisableTiming));
-    BEM_CUDA_CHECK(cudaEventCreateWithFlags(&fj.join, cudaEventDisableTiming));
-    BEM_CUDA_CHECK(cudaEventRecord(fj.fork, ctx.stream));
-    BEM_CUDA_CHECK(cudaStreamWaitEvent(fj.side, fj.fork, 0));
-    c2.stream = fj.side;
+    BEM_CUDA_CHECK(fj.acquire(ctx.stream));
+    BEM_CUDA_CHECK(cudaEventRecord(fj.ev[0], ctx.stream));
+    BEM_CUDA_CHECK(cudaStreamWaitEvent(fj.stream, fj.ev[0], 0));
+    c2.stream = fj.stream;
     if (split_ws) {
       const size_t h = (ctx.ws_bytes / 2) & ~size_t(255);
       c.ws_bytes = h;
@@ -288,8 +276,8 @@ static int bem_init_t(const LaContext& ctx, int n, void* ws, const EpsArg& eps, 
       if ((st = gemm<C>(c2, n, n, n, one, s.M[3], n, s.M[1], n, zero, s.M[5], n))) return st;
       BEM_CUDA_CHECK(cudaMemcpyAsync(s.M[3], s.M[5], sizeof(C) * nn, cudaMemcpyDeviceToDevice, c2.stream));
       if (fork) {  // (without a second chain, c2 is c: same stream, whole workspace)
-        BEM_CUDA_CHECK(cudaEventRecord(fj.join, fj.side));
-        BEM_CUDA_CHECK(cudaStreamWaitEvent(ctx.stream, fj.join, 0));
+        BEM_CUDA_CHECK(cudaEventRecord(fj.ev[1], fj.stream));
+        BEM_CUDA_CHECK(cudaStreamWaitEvent(ctx.stream, fj.ev[1], 0));
         c.ws_bytes = ctx.ws_bytes;
       }
       flag_to_info_kernel<<<1, 1, 0, ctx.stream>>>(vf[0], s.verdict);
@@ -324,8 +312,8 @@ static int bem_init_t(const LaContext& ctx, int n, void* ws, const EpsArg& eps, 
     if ((st = trsv_diag_inverse<C>(c2, n, s.M[1], n, s.map[1], s.dinv[2], s.dinv[3]))) return st;
   }
   if (fork) {
-    BEM_CUDA_CHECK(cudaEventRecord(fj.join, fj.side));
-    BEM_CUDA_CHECK(cudaStreamWaitEvent(ctx.stream, fj.join, 0));
+    BEM_CUDA_CHECK(cudaEventRecord(fj.ev[1], fj.stream));
+    BEM_CUDA_CHECK(cudaStreamWaitEvent(ctx.stream, fj.ev[1], 0));
     c.ws_bytes = ctx.ws_bytes;
   }
   if ((st = mark(1))) return st;
@@ -521,14 +509,12 @@ static int bem_solve_core(const LaContext& ctx0, int n, int p, void* ws, const C
   BEM_LAUNCH_CHECK();
   // sig1/h1 = G1^-1 W1 and sig2/h2 = G2^-1 W2 are independent: the second runs
   // on a stream forked from the caller's, with its own triangular-solve scratch
-  ForkJoin fj;
-  BEM_CUDA_CHECK(cudaStreamCreateWithFlags(&fj.side, cudaStreamNonBlocking));
-  BEM_CUDA_CHECK(cudaEventCreateWithFlags(&fj.fork, cudaEventDisableTiming));
-  BEM_CUDA_CHECK(cudaEventCreateWithFlags(&fj.join, cudaEventDisableTiming));
-  BEM_CUDA_CHECK(cudaEventRecord(fj.fork, st_));
-  BEM_CUDA_CHECK(cudaStreamWaitEvent(fj.side, fj.fork, 0));
+  StreamLease fj;
+  BEM_CUDA_CHECK(fj.acquire(st_));
+  BEM_CUDA_CHECK(cudaEventRecord(fj.ev[0], st_));
+  BEM_CUDA_CHECK(cudaStreamWaitEvent(fj.stream, fj.ev[0], 0));
   LaContext c2 = ctx;
-  c2.stream = fj.side;
+  c2.stream = fj.stream;
   void* lscr2 = reinterpret_cast<char*>(lscr) + align256(solve_left_scratch_bytes<C>(n, 4 * p));
   if (inv) {
     if ((st = gemm<C>(ctx, n, 4 * p, n, one, s.M[0], n, P1, 4 * p, zero, W1, 4 * p))) return st;
@@ -541,8 +527,8 @@ static int bem_solve_core(const LaContext& ctx0, int n, int p, void* ws, const C
                             di ? s.dinv[3] : nullptr)))
       return st;
   }
-  BEM_CUDA_CHECK(cudaEventRecord(fj.join, fj.side));
-  BEM_CUDA_CHECK(cudaStreamWaitEvent(st_, fj.join, 0));
+  BEM_CUDA_CHECK(cudaEventRecord(fj.ev[1], fj.stream));
+  BEM_CUDA_CHECK(cudaStreamWaitEvent(st_, fj.ev[1], 0));
   return BEM200_OK;
 }
 
@@ -989,6 +975,38 @@ __global__ void absmax_kernel(long long n, const double2* __restrict__ x, unsign
   if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(m));
 }
 
+// The refinement's bookkeeping stays on the device until the end of a sweep: the
+// scale of the complex64 solve is read from the norm's slot, and the residual's
+// norm, the right-hand side's and the status of the factors come back in one
+// copy per sweep.
+struct IrState {
+  unsigned long long bnorm, rnorm[2];  // bits of non-negative doubles; rnorm alternates
+  int info, status;
+};
+__device__ __forceinline__ double norm_scale(const unsigned long long* norm, bool inverse) {
+  const double v = __longlong_as_double((long long)*norm);
+  return v > 0 && v < 1e300 ? (inverse ? 1.0 / v : v) : 0.0;
+}
+__global__ void c128_to_c64_scaled_kernel(long long n, const double2* __restrict__ x, float2* __restrict__ y,
+                                          const unsigned long long* __restrict__ norm) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const double scale = norm_scale(norm, true);
+  if (i < n) y[i] = make_float2((float)(x[i].x * scale), (float)(x[i].y * scale));
+}
+__global__ void axpy_c64_to_c128_scaled_kernel(long long n, const float2* __restrict__ x,
+                                               const unsigned long long* __restrict__ norm, double2* __restrict__ y,
+                                               bool accumulate) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double scale = norm_scale(norm, false);
+  const double2 v = make_double2((double)x[i].x * scale, (double)x[i].y * scale);
+  y[i] = accumulate ? cadd(y[i], v) : v;
+}
+__global__ void ir_status_kernel(const int* __restrict__ info, IrState* __restrict__ st) {
+  st->info = info[0];
+  st->status = info[1];
+}
+
 static int absmax_host(cudaStream_t s, long long n, const double2* x, unsigned long long* dscratch, double* out) {
   BEM_CUDA_CHECK(cudaMemsetAsync(dscratch, 0, sizeof(unsigned long long), s));
   absmax_kernel<<<296, 256, 0, s>>>(n, x, dscratch);
@@ -1345,45 +1363,51 @@ int bem200_bem_solve_ir_ex(int precision, int engine, int n, int npol, void* ws,
   double2* r = reinterpret_cast<double2*>(p);         p += align256(sizeof(double2) * 8 * np);
   double2* x = reinterpret_cast<double2*>(p);         p += align256(sizeof(double2) * 8 * np);
   double2* opws = reinterpret_cast<double2*>(p);      p += align256(sizeof(double2) * 40 * np);
-  unsigned long long* red = reinterpret_cast<unsigned long long*>(p);
+  IrState* red = reinterpret_cast<IrState*>(p);
   cudaStream_t s = ctx.stream;
   const double2* bb = (const double2*)b;
-  double bnorm = 0;
-  int st = absmax_host(s, 8 * np, bb, red, &bnorm);
-  if (st) return st;
-  BEM_REQUIRE(bnorm > 0 && bnorm < 1e300, BEM200_ERR_ARG, "bem_solve_ir: right-hand side is zero or not finite");
+  BEM_CUDA_CHECK(cudaMemsetAsync(red, 0, sizeof(IrState), s));
+  absmax_kernel<<<296, 256, 0, s>>>(8 * np, bb, &red->bnorm);
+  BEM_LAUNCH_CHECK();
   // x = M b  (mixed solve, scaled to unit magnitude)
   const double2* res = bb;
-  double rnorm = bnorm, prev = bnorm;
-  int it = 0;
+  const unsigned long long* norm = &red->bnorm;
+  double bnorm = 0, rnorm = 0, prev = 0;
+  int it = 0, st;
   bool first = true;
   int outcome = BEM200_OK;
   const BemState<float2> sv = state_view<float2>(n, ws);
   while (true) {
-    double scale = 1.0 / rnorm;
-    c128_to_c64_kernel<<<ceil_div(8 * np, 256), 256, 0, s>>>(8 * np, res, rhs32, scale);
+    c128_to_c64_scaled_kernel<<<ceil_div(8 * np, 256), 256, 0, s>>>(8 * np, res, rhs32, norm);
     BEM_LAUNCH_CHECK();
     // rhs32 = [phi (np) | a (3np) | alpha (3np) | De (np)];  sol32 = [W1 (4np) | W2 (4np)]
     if ((st = bem_solve_core<float2>(ctx, n, npol, ws, rhs32, rhs32 + np, rhs32 + 4 * np, rhs32 + 7 * np, eps, nvec,
                                      k0, sol32, sol32 + 4 * np, core, inv)))
       return st;
-    axpy_c64_to_c128_kernel<<<ceil_div(8 * np, 256), 256, 0, s>>>(8 * np, sol32, rnorm, x, !first);
+    axpy_c64_to_c128_scaled_kernel<<<ceil_div(8 * np, 256), 256, 0, s>>>(8 * np, sol32, norm, x, !first);
     BEM_LAUNCH_CHECK();
     first = false;
     // r = b - A x
     if ((st = bem_apply(ctx, n, npol, (const double2*)G1, (const double2*)G2, (const double2*)H1, (const double2*)H2,
                         eps, nvec, k0, x, x + 4 * np, bb, r, opws)))
       return st;
-    if ((st = absmax_host(s, 8 * np, r, red, &rnorm))) return st;
+    unsigned long long* rn = &red->rnorm[it & 1];
+    if (it > 1) BEM_CUDA_CHECK(cudaMemsetAsync(rn, 0, sizeof(*rn), s));
+    absmax_kernel<<<296, 256, 0, s>>>(8 * np, r, rn);
+    BEM_LAUNCH_CHECK();
+    ir_status_kernel<<<1, 1, 0, s>>>(sv.info, red);
+    BEM_LAUNCH_CHECK();
+    IrState h;
+    BEM_CUDA_CHECK(cudaMemcpyAsync(&h, red, sizeof(h), cudaMemcpyDeviceToHost, s));
+    BEM_CUDA_CHECK(cudaStreamSynchronize(s));
+    memcpy(&bnorm, &h.bnorm, sizeof(double));
+    memcpy(&rnorm, &h.rnorm[it & 1], sizeof(double));
+    BEM_REQUIRE(bnorm > 0 && bnorm < 1e300, BEM200_ERR_ARG, "bem_solve_ir: right-hand side is zero or not finite");
+    if (it == 0) prev = bnorm;
     ++it;
-    {
-      int hs[2] = {0, 0};  // info (first zero pivot of the factors), status (bounded waits)
-      BEM_CUDA_CHECK(cudaMemcpyAsync(hs, sv.info, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-      BEM_CUDA_CHECK(cudaStreamSynchronize(s));
-      BEM_REQUIRE(hs[0] == 0, BEM200_ERR_SINGULAR, "bem_solve_ir: the complex64 factors hold a zero pivot (%d)",
-                  hs[0]);
-      BEM_REQUIRE(hs[1] == 0, BEM200_ERR_TIMEOUT, "bem_solve_ir: a bounded device wait gave up (status %d)", hs[1]);
-    }
+    // info (first zero pivot of the factors), status (bounded waits)
+    BEM_REQUIRE(h.info == 0, BEM200_ERR_SINGULAR, "bem_solve_ir: the complex64 factors hold a zero pivot (%d)", h.info);
+    BEM_REQUIRE(h.status == 0, BEM200_ERR_TIMEOUT, "bem_solve_ir: a bounded device wait gave up (status %d)", h.status);
     if (rnorm <= tol * bnorm) break;
     if (!(rnorm < 1e300)) {  // NaN or overflow
       outcome = BEM200_ERR_NOCONV;
@@ -1404,6 +1428,7 @@ int bem200_bem_solve_ir_ex(int precision, int engine, int n, int npol, void* ws,
     }
     prev = rnorm;
     res = r;
+    norm = rn;
   }
   *iters = it;
   *relres = rnorm / bnorm;

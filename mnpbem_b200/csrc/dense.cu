@@ -26,6 +26,73 @@ namespace cg = cooperative_groups;
 
 namespace bem200 {
 
+// ------------------------------------------------------------- stream pool
+namespace {
+struct PooledBundle {
+  int dev, kind;
+  cudaStream_t stream;
+  cudaEvent_t ev[3];
+};
+constexpr int kPoolCap = 32;  // idle bundles kept per device and kind
+std::mutex g_pool_mu;
+// never destroyed: streams must not be released after the runtime has shut down
+std::vector<PooledBundle>& pool() {
+  static auto* p = new std::vector<PooledBundle>;
+  return *p;
+}
+}  // namespace
+
+cudaError_t StreamLease::acquire(cudaStream_t main, Kind kind) {
+  cudaError_t e = cudaGetDevice(&dev_);
+  if (e != cudaSuccess) return e;
+  kind_ = kind;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(main, &cs) != cudaSuccess) {
+    (void)cudaGetLastError();
+    cs = cudaStreamCaptureStatusActive;
+  }
+  pooled_ = cs == cudaStreamCaptureStatusNone;
+  if (pooled_) {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    std::vector<PooledBundle>& v = pool();
+    for (size_t i = v.size(); i-- > 0;)
+      if (v[i].dev == dev_ && v[i].kind == kind) {
+        stream = v[i].stream;
+        for (int k = 0; k < 3; ++k) ev[k] = v[i].ev[k];
+        v.erase(v.begin() + i);
+        return cudaSuccess;
+      }
+  }
+  int prio = 0, lo = 0, hi = 0;
+  if (kind != kNormal) {
+    if ((e = cudaDeviceGetStreamPriorityRange(&lo, &hi)) != cudaSuccess) return e;
+    prio = kind == kHigh ? hi : lo;
+  }
+  if ((e = cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, prio)) != cudaSuccess) return e;
+  for (cudaEvent_t& x : ev)
+    if ((e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming)) != cudaSuccess) return e;
+  return cudaSuccess;
+}
+
+void StreamLease::release() {
+  if (!stream) return;
+  if (pooled_ && ev[2]) {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    std::vector<PooledBundle>& v = pool();
+    int idle = 0;
+    for (const PooledBundle& b : v) idle += b.dev == dev_ && b.kind == kind_;
+    if (idle < kPoolCap) {
+      v.push_back(PooledBundle{dev_, kind_, stream, {ev[0], ev[1], ev[2]}});
+      stream = nullptr;
+      return;
+    }
+  }
+  for (cudaEvent_t& x : ev)
+    if (x) cudaEventDestroy(x);
+  cudaStreamDestroy(stream);  // released once its queued work has finished
+  stream = nullptr;
+}
+
 template <typename C> using R_t = typename cplx_traits<C>::real;
 
 __device__ __forceinline__ double cabs1(double2 a) { return fabs(a.x) + fabs(a.y); }
@@ -2451,33 +2518,19 @@ static int la_width(const LaContext& ctx, int n) {
   return max(64, min(1024, (w / kPanelNB) * kPanelNB));
 }
 
-struct LaStreams {
-  cudaStream_t hi = nullptr, lo = nullptr;
-  cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // fork, panel, wide, done_hi, done_lo
-  ~LaStreams() {
-    for (cudaEvent_t& e : ev)
-      if (e) cudaEventDestroy(e);
-    if (hi) cudaStreamDestroy(hi);  // released once their queued work has finished
-    if (lo) cudaStreamDestroy(lo);
-  }
-};
-
 template <typename C>
 static int getrf_lookahead(const LaContext& ctx, int n, C* A, long long ld, int32_t* rowmap, int32_t* ipiv,
                            int32_t* snap) {
-  LaStreams ls;
-  int lo_pri = 0, hi_pri = 0;
-  BEM_CUDA_CHECK(cudaDeviceGetStreamPriorityRange(&lo_pri, &hi_pri));
-  BEM_CUDA_CHECK(cudaStreamCreateWithPriority(&ls.hi, cudaStreamNonBlocking, hi_pri));
-  BEM_CUDA_CHECK(cudaStreamCreateWithPriority(&ls.lo, cudaStreamNonBlocking, lo_pri));
-  for (cudaEvent_t& e : ls.ev) BEM_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  cudaEvent_t ev_fork = ls.ev[0], ev_panel = ls.ev[1], ev_wide = ls.ev[2];
+  StreamLease hi, lo;
+  BEM_CUDA_CHECK(hi.acquire(ctx.stream, StreamLease::kHigh));
+  BEM_CUDA_CHECK(lo.acquire(ctx.stream, StreamLease::kLow));
+  cudaEvent_t ev_fork = hi.ev[0], ev_panel = hi.ev[1], ev_wide = lo.ev[0];
   BEM_CUDA_CHECK(cudaEventRecord(ev_fork, ctx.stream));
-  BEM_CUDA_CHECK(cudaStreamWaitEvent(ls.hi, ev_fork, 0));
-  BEM_CUDA_CHECK(cudaStreamWaitEvent(ls.lo, ev_fork, 0));
+  BEM_CUDA_CHECK(cudaStreamWaitEvent(hi.stream, ev_fork, 0));
+  BEM_CUDA_CHECK(cudaStreamWaitEvent(lo.stream, ev_fork, 0));
   LaContext cm = ctx, cw = ctx;
-  cm.stream = ls.hi;
-  cw.stream = ls.lo;
+  cm.stream = hi.stream;
+  cw.stream = lo.stream;
   cm.panel_ws = reinterpret_cast<char*>(snap) + (((size_t)2 * n * sizeof(int32_t) + 255) & ~size_t(255));
   if (ctx.engine != GemmEngine::kSimt) {
     const size_t h = (ctx.ws_bytes / 2) & ~size_t(255);
@@ -2485,7 +2538,7 @@ static int getrf_lookahead(const LaContext& ctx, int n, C* A, long long ld, int3
     cw.ws = reinterpret_cast<char*>(ctx.ws) + h;
     cw.ws_bytes = h;
   }
-  iota_kernel<<<ceil_div(n, 256), 256, 0, ls.hi>>>(n, rowmap);
+  iota_kernel<<<ceil_div(n, 256), 256, 0, hi.stream>>>(n, rowmap);
   BEM_LAUNCH_CHECK();
   bool wide_pending = false;
   int st;
@@ -2498,29 +2551,29 @@ static int getrf_lookahead(const LaContext& ctx, int n, C* A, long long ld, int3
     const int w1 = min(nb, n - c1), c2 = c1 + w1;
     int32_t* sn = snap + (size_t)(j & 1) * n;  // sn[i] = rowmap[c1 + i] as of the end of panel(j)
     if (c2 < n) {
-      BEM_CUDA_CHECK(cudaMemcpyAsync(sn, rowmap + c1, sizeof(int32_t) * (n - c1), cudaMemcpyDeviceToDevice, ls.hi));
-      BEM_CUDA_CHECK(cudaEventRecord(ev_panel, ls.hi));
+      BEM_CUDA_CHECK(cudaMemcpyAsync(sn, rowmap + c1, sizeof(int32_t) * (n - c1), cudaMemcpyDeviceToDevice, hi.stream));
+      BEM_CUDA_CHECK(cudaEventRecord(ev_panel, hi.stream));
     }
     // narrow(j): block column j + 1
-    if (wide_pending) BEM_CUDA_CHECK(cudaStreamWaitEvent(ls.hi, ev_wide, 0));
+    if (wide_pending) BEM_CUDA_CHECK(cudaStreamWaitEvent(hi.stream, ev_wide, 0));
     RowView<C> V{A, ld, rowmap + c0, c0};  // logical rows from c0, columns from c0
     if ((st = trsm_llu<C>(cm, w, w1, V, V.sub(0, w)))) return st;
     if ((st = gemm_v<C>(cm, n - c1, w1, w, neg_one<C>(), V.sub(w, 0), V.sub(0, w), one<C>(), V.sub(w, w)))) return st;
     // wide(j): block columns j + 2 ..
     wide_pending = false;
     if (c2 < n) {
-      BEM_CUDA_CHECK(cudaStreamWaitEvent(ls.lo, ev_panel, 0));
+      BEM_CUDA_CHECK(cudaStreamWaitEvent(lo.stream, ev_panel, 0));
       if ((st = trsm_llu<C>(cw, w, n - c2, V, V.sub(0, c2 - c0)))) return st;
       const RowView<C> L21{A, ld, sn, c0}, A22{A, ld, sn, c2};
       if ((st = gemm_v<C>(cw, n - c1, n - c2, w, neg_one<C>(), L21, V.sub(0, c2 - c0), one<C>(), A22))) return st;
-      BEM_CUDA_CHECK(cudaEventRecord(ev_wide, ls.lo));
+      BEM_CUDA_CHECK(cudaEventRecord(ev_wide, lo.stream));
       wide_pending = true;
     }
   }
-  BEM_CUDA_CHECK(cudaEventRecord(ls.ev[3], ls.hi));
-  BEM_CUDA_CHECK(cudaEventRecord(ls.ev[4], ls.lo));
-  BEM_CUDA_CHECK(cudaStreamWaitEvent(ctx.stream, ls.ev[3], 0));
-  BEM_CUDA_CHECK(cudaStreamWaitEvent(ctx.stream, ls.ev[4], 0));
+  BEM_CUDA_CHECK(cudaEventRecord(hi.ev[2], hi.stream));
+  BEM_CUDA_CHECK(cudaEventRecord(lo.ev[1], lo.stream));
+  BEM_CUDA_CHECK(cudaStreamWaitEvent(ctx.stream, hi.ev[2], 0));
+  BEM_CUDA_CHECK(cudaStreamWaitEvent(ctx.stream, lo.ev[1], 0));
   return BEM200_OK;
 }
 

@@ -71,27 +71,42 @@ struct LaContext {
 // pivots its first int is the panels' verdict flag
 constexpr size_t kPanelGridScratch = 176u * 1024u;
 
-// A non-blocking side stream forked from ctx.stream (fork()) and joined back
-// into it (join()); the destructor releases the stream and events once their
-// queued work has finished.  The side context gets the upper half of the
-// tensor-core operand workspace, the main one keeps the lower half.
+// A side stream with three events, leased from a pool shared by all threads
+// (creating and destroying a stream and its events costs 70 - 180 us per call,
+// more than the work of a small solve).  At most 32 idle bundles per device
+// and kind are kept, the rest is destroyed on return.  A returned stream may
+// still have queued work: the next user's work runs after it, which is an
+// ordering only (every lease is joined into its caller's stream).  While
+// `main` is being captured a bundle is created for the call and destroyed with
+// it, so that no stream of the pool ever belongs to a capture.
+struct StreamLease {
+  enum Kind { kNormal = 0, kHigh = 1, kLow = 2 };  // stream priority
+  cudaStream_t stream = nullptr;
+  cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+  StreamLease() = default;
+  StreamLease(const StreamLease&) = delete;
+  StreamLease& operator=(const StreamLease&) = delete;
+  ~StreamLease() { release(); }
+  cudaError_t acquire(cudaStream_t main, Kind kind = kNormal);
+
+ private:
+  void release();
+  int dev_ = -1, kind_ = 0;
+  bool pooled_ = false;
+};
+
+// A side stream forked from ctx.stream (fork()) and joined back into it
+// (join()).  The side context gets the upper half of the tensor-core operand
+// workspace, the main one keeps the lower half.
 struct SideStream {
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  ~SideStream() {
-    if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_join) cudaEventDestroy(ev_join);
-    if (side) cudaStreamDestroy(side);
-  }
+  StreamLease lease;
   // splits the workspace of `main`; returns false (nothing forked) on failure
   bool fork(LaContext& main, LaContext& aux) {
-    if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) return false;
-    if (cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming) != cudaSuccess) return false;
-    if (cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming) != cudaSuccess) return false;
-    if (cudaEventRecord(ev_fork, main.stream) != cudaSuccess) return false;
-    if (cudaStreamWaitEvent(side, ev_fork, 0) != cudaSuccess) return false;
+    if (lease.acquire(main.stream) != cudaSuccess) return false;
+    if (cudaEventRecord(lease.ev[0], main.stream) != cudaSuccess) return false;
+    if (cudaStreamWaitEvent(lease.stream, lease.ev[0], 0) != cudaSuccess) return false;
     aux = main;
-    aux.stream = side;
+    aux.stream = lease.stream;
     if (main.engine != GemmEngine::kSimt) {
       const size_t h = (main.ws_bytes / 2) & ~size_t(255);
       main.ws_bytes = h;
@@ -101,9 +116,9 @@ struct SideStream {
     return true;
   }
   cudaError_t join(cudaStream_t main_stream) {
-    cudaError_t e = cudaEventRecord(ev_join, side);
+    cudaError_t e = cudaEventRecord(lease.ev[1], lease.stream);
     if (e != cudaSuccess) return e;
-    return cudaStreamWaitEvent(main_stream, ev_join, 0);
+    return cudaStreamWaitEvent(main_stream, lease.ev[1], 0);
   }
 };
 
