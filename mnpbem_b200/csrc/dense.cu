@@ -2874,143 +2874,119 @@ int inverse(const LaContext& ctx, int n, const C* LU, long long ld, const int32_
 //   A^-1 (recursive), T1 = A^-1 B, T2 = C A^-1, S = D - C T1, S^-1 (recursive),
 //   B <- -T1 S^-1, C <- -S^-1 T2, A <- A^-1 - B T2.
 // Nearly all of the 8 n^3 flops land in the large GEMMs of the top levels
-// (tensor cores for complex64); the leaves (<= 128 x 128 complex64, 64 x 64
-// complex128) are inverted by
+// (tensor cores for complex64); the leaves (<= 64 x 64) are inverted by
 // Gauss-Jordan elimination in registers.  No row exchanges means no check
 // of the leaves' pivots can cover the rows outside them, so the caller
 // verifies the result with inverse_probe (M^-1 (M v) = v for a fixed
 // pseudo-random v) and falls back to the pivoted LU when it fails.
-template <typename C> struct InvLeaf { static constexpr int value = 64; };
-template <> struct InvLeaf<double2> { static constexpr int value = 64; };
-constexpr int kInvLeafThreads = 128;
+constexpr int kInvLeaf = 64;
+constexpr int kInvLeafThreads = 256;
 
-// Gauss-Jordan inversion of the nb x nb (nb <= LN = InvLeaf) block at M, in
-// place.  Thread (ty, tx) of the 8 x 16 grid owns the 8 x 4 block of rows
-// ty + 8 p and columns tx + 16 q of an LN x LN tile padded with the identity;
-// the 16 owners of a row are lanes of one warp.  Step k: the owners of row k
-// take a_kk from its lane by a shuffle, scale the row by 1 / a_kk (that is
-// the row's final value) and publish it, each entry beside its product with
-// i so that the update is two packed FMAs; the owners of column k publish it
-// (complex64: negated, each part duplicated for the packed operands).  With
-// 1 + 1 / a_kk published in place of the pivot, every other row takes
-// a_ij -= a_ik r_j, which also turns column k into -a_ik / a_kk.  The
-// buffers are double buffered, so one barrier per step suffices.  A pivot
-// that is zero or not the first largest |re| + |im| among the rows still to
-// be eliminated raises *vflag.
-template <typename C> struct LeafRow { using type = C; };            // complex128: the entry
-template <> struct LeafRow<float2> { using type = float4; };         // complex64: (r_j, i r_j)
-template <typename C> struct LeafCol { using type = C; };            // complex128: a_ik
-template <> struct LeafCol<float2> { using type = float4; };         // complex64: -(x, x, y, y)
-__device__ __forceinline__ void leaf_pub(float4& d, float2 r) { d = make_float4(r.x, r.y, -r.y, r.x); }
-__device__ __forceinline__ void leaf_pub(double2& d, double2 r) { d = r; }
-__device__ __forceinline__ void leaf_pubcol(float4& d, float2 a) { d = make_float4(-a.x, -a.x, -a.y, -a.y); }
-__device__ __forceinline__ void leaf_pubcol(double2& d, double2 a) { d = a; }
-__device__ __forceinline__ float leaf_cmag(float4 c) { return fabsf(c.x) + fabsf(c.z); }
-__device__ __forceinline__ double leaf_cmag(double2 c) { return pmag(c); }
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(f2_bits(a)), "l"(f2_bits(b)), "l"(f2_bits(c)));
-  return bits_f2(d);
-}
-// a_ij - a_ik r_j over the thread's entries of one row
-template <int NQ>
-__device__ __forceinline__ void leaf_row_update(float2 (&a)[NQ], float4 c, const float4 (&rr)[NQ]) {
-  const float2 nx = make_float2(c.x, c.y), ny = make_float2(c.z, c.w);
-#pragma unroll
-  for (int q = 0; q < NQ; ++q)
-    a[q] = ffma2(ny, make_float2(rr[q].z, rr[q].w), ffma2(nx, make_float2(rr[q].x, rr[q].y), a[q]));
-}
-template <int NQ>
-__device__ __forceinline__ void leaf_row_update(double2 (&a)[NQ], double2 c, const double2 (&rr)[NQ]) {
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) a[q] = csub(a[q], cmul(c, rr[q]));
-}
-// 1 / p: approximate reciprocals (two MUFU operations, scaled) for complex64
+// 1 / p in FP32: p scaled by a power of two, one approximate reciprocal of |p|^2
 __device__ __forceinline__ float2 leaf_recip(float2 p) {
-  const float sc = fmaxf(fabsf(p.x), fabsf(p.y));
-  if (!(sc > 0.f)) return make_float2(0.f, 0.f);
-  float rs, f;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(sc));
-  const float px = p.x * rs, py = p.y * rs;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"(px * px + py * py));
-  f *= rs;
-  return make_float2(px * f, -py * f);
+  const float m = fmaxf(fabsf(p.x), fabsf(p.y));
+  const float s = __int_as_float(0x7f000000 - (__float_as_int(m) & 0x7f800000));
+  const float px = p.x * s, py = p.y * s;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaf(px, px, py * py)));
+  r *= s;
+  return make_float2(px * r, -py * r);
 }
-__device__ __forceinline__ double2 leaf_recip(double2 p) { return crecip_scaled(p); }
+__device__ __forceinline__ double2 leaf_recip(double2 p) { return crecip_newton<false>(p); }
 
+// Gauss-Jordan inversion of the nb x nb (nb <= 64) block at M, in place, in
+// registers.  Thread (ty, tx) of the 16 x 16 grid owns rows 4 ty + p and columns
+// 4 tx + q (p, q < 4) of a 64 x 64 tile padded with the identity, so the row and
+// column of pivot k = 4 g + s are entry s of the threads ty = g, tx = g: s is a
+// constant of the unrolled step, and only those entries need a select.  Step k
+// reads row k, column k (published by the step before, double buffered: one
+// barrier per step, columns and rows interleaved to avoid bank conflicts),
+// takes t = row k / a_kk (1 / a_kk in column k) and a_ij -= a_ik t_j everywhere
+// outside row k; every thread forms the reciprocal itself, which is cheaper than
+// a second exchange (and than forming the next reciprocal ahead: 20.5 us).
+// Latency bound: 64 x 64 in 18.5 us for complex64 and 30.8 for complex128 in a
+// back-to-back loop; 128 threads with 8 x 4 entries and the row scaled by its
+// owners before publishing took 28.7 and 47.2.  A pivot that is zero or below 1 / tau of
+// the largest |re| + |im| of the rows still to be eliminated raises *vflag.
 template <typename C>
 __global__ void __launch_bounds__(kInvLeafThreads, 1) inv_leaf_kernel(int nb, C* __restrict__ M, long long ld,
                                                                       R_t<C> tau, int* __restrict__ vflag) {
-  constexpr int LN = InvLeaf<C>::value;
-  constexpr int TY = 8, TX = 16;             // thread grid
-  constexpr int PR = LN / TY, QC = LN / TX;  // rows and columns per thread: 8 x 4
-  using RowE = typename LeafRow<C>::type;
-  using ColE = typename LeafCol<C>::type;
+  constexpr int N = 64, T = 16, PQ = N / T;
   using R = R_t<C>;
-  static_assert(TY * TX == kInvLeafThreads && PR * TY == LN && QC * TX == LN && TX % TY == 0 && 32 % TX == 0,
-                "leaf layout");
-  __shared__ RowE rowb[2][LN];
-  __shared__ ColE colb[2][LN];
-  __shared__ R pmb[2];
-  const int tid = threadIdx.x, ty = tid / TX, tx = tid % TX;
-  const int row_lane = (tid & 31) & ~(TX - 1);  // lane of (ty, 0)
-  C a[PR][QC];
+  __shared__ __align__(16) C rowb[2][N];
+  __shared__ __align__(16) C colb[2][N];
+  const int tid = threadIdx.x, ty = tid / T, tx = tid % T;
+  C a[PQ][PQ];
 #pragma unroll
-  for (int p = 0; p < PR; ++p)
+  for (int p = 0; p < PQ; ++p)
 #pragma unroll
-    for (int q = 0; q < QC; ++q) {
-      const int i = ty + TY * p, c = tx + TX * q;
+    for (int q = 0; q < PQ; ++q) {
+      const int i = PQ * ty + p, c = PQ * tx + q;
       a[p][q] = (i < nb && c < nb) ? M[(long long)i * ld + c] : (i == c ? cmake<C>(1.0, 0.0) : czero<C>());
     }
+  auto publish = [&](int g, int s, int b) {  // row and column 4 g + s
+    if (tx == g) {
+#pragma unroll
+      for (int p = 0; p < PQ; ++p) colb[b][T * p + ty] = a[p][s];
+    }
+    if (ty == g) {
+#pragma unroll
+      for (int q = 0; q < PQ; ++q) rowb[b][T * q + tx] = a[s][q];
+    }
+  };
+  publish(0, 0, 0);
   bool bad = false;
-#pragma unroll
-  for (int kp = 0; kp < PR; ++kp) {   // k = TY kp + kr: row k is row kp of thread row kr
-    const int qk = (TY * kp) / TX;   // column k is column qk of thread column k % TX
-    if (TY * kp >= nb) break;        // the identity padding needs no elimination steps
 #pragma unroll 1
-    for (int kr = 0; kr < TY; ++kr) {
-      const int k = TY * kp + kr, b = k & 1, kx = k % TX;
-      if (k >= nb) break;
-      if (tx == kx) {
+  for (int g = 0; PQ * g < nb; ++g) {
+    const bool mr = ty == g, mc = tx == g, below = ty > g;
 #pragma unroll
-        for (int p = 0; p < PR; ++p) leaf_pubcol(colb[b][ty + TY * p], a[p][qk]);
-      }
-      const C akk = shfl_c(a[kp][qk], row_lane | kx);  // a_{ty + TY kp, k}: a_kk in the lanes of row k
-      if (ty == kr) {
-        const C pinv = leaf_recip(akk);
-#pragma unroll
-        for (int q = 0; q < QC; ++q) {
-          const bool diag = q == qk && tx == kx;
-          const C r = diag ? cadd(cmake<C>(1.0, 0.0), pinv) : cmul(a[kp][q], pinv);
-          leaf_pub(rowb[b][tx + TX * q], r);
-          a[kp][q] = diag ? pinv : r;  // row k is final
-        }
-        if (tx == kx) pmb[b] = pmag(akk);
-      }
+    for (int s = 0; s < PQ; ++s) {
+      const int b = s & 1;
       __syncthreads();
-      const R pm = pmb[b];
-      if (!(pm > 0)) bad = true;
-      RowE rr[QC];
+      const C piv = rowb[b][T * s + g];
+      C r[PQ], c[PQ];
 #pragma unroll
-      for (int q = 0; q < QC; ++q) rr[q] = rowb[b][tx + TX * q];
-      R lower = 0;  // largest |a_ik|_1 among this thread's rows below k
+      for (int q = 0; q < PQ; ++q) r[q] = rowb[b][T * q + tx];
 #pragma unroll
-      for (int p = 0; p < PR; ++p) {
-        const ColE cik = colb[b][ty + TY * p];
-        if (p > kp || (p == kp && ty > kr)) lower = fmax(lower, leaf_cmag(cik));
-        if (!(p == kp && ty == kr)) leaf_row_update(a[p], cik, rr);
+      for (int p = 0; p < PQ; ++p) c[p] = colb[b][T * p + ty];
+      const C pinv = leaf_recip(piv);
+      const R pm = tau * (fabs(piv.x) + fabs(piv.y));
+#pragma unroll
+      for (int q = 0; q < PQ; ++q) {
+        const C t = cmul(r[q], pinv);
+        r[q] = (q == s && mc) ? pinv : t;
       }
-      if (lower > tau * pm) bad = true;
+      R lower = 0, upper = 0;  // largest |a_ik|_1 of this thread's rows beyond s, up to s
+#pragma unroll
+      for (int p = 0; p < PQ; ++p) {
+        const R m = fabs(c[p].x) + fabs(c[p].y);
+        if (p > s) lower = fmax(lower, m); else upper = fmax(upper, m);
+      }
+      lower = below ? fmax(lower, upper) : (mr ? lower : R(0));
+      bad |= !(pm > 0) | (lower > pm);
+      if (mc) {
+#pragma unroll
+        for (int p = 0; p < PQ; ++p) a[p][s] = czero<C>();
+      }
+#pragma unroll
+      for (int p = 0; p < PQ; ++p)
+#pragma unroll
+        for (int q = 0; q < PQ; ++q) cmsub(a[p][q], c[p], r[q]);
+      if (mr) {
+#pragma unroll
+        for (int q = 0; q < PQ; ++q) a[s][q] = r[q];
+      }
+      publish(s == PQ - 1 ? g + 1 : g, (s + 1) % PQ, b ^ 1);
     }
   }
 #pragma unroll
-  for (int p = 0; p < PR; ++p)
+  for (int p = 0; p < PQ; ++p)
 #pragma unroll
-    for (int q = 0; q < QC; ++q) {
-      const int i = ty + TY * p, c = tx + TX * q;
+    for (int q = 0; q < PQ; ++q) {
+      const int i = PQ * ty + p, c = PQ * tx + q;
       if (i < nb && c < nb) M[(long long)i * ld + c] = a[p][q];
     }
-  if (__any_sync(0xffffffffu, bad) && (tid & 31) == 0 && vflag) atomicExch(vflag, 1);
+  if (__syncthreads_or(bad) && tid == 0 && vflag) atomicExch(vflag, 1);
 }
 
 // scratch elements inverse_nopiv needs for an n x n matrix
@@ -3018,7 +2994,6 @@ template <typename C>
 static size_t inverse_nopiv_scratch(int n) {
   // the inverse of A runs first, from the start of the scratch; then T1, T2
   // stay live while the inverse of S uses what follows them
-  constexpr int kInvLeaf = InvLeaf<C>::value;
   if (n <= kInvLeaf) return 0;
   const int n1 = min(n - 1, ceil_div(n / 2, kInvLeaf) * kInvLeaf), n2 = n - n1;
   return max(inverse_nopiv_scratch<C>(n1), 2 * (size_t)n1 * n2 + inverse_nopiv_scratch<C>(n2));
@@ -3056,7 +3031,6 @@ static int gemm_pair(const LaContext& ctx, const RecFork* fk, bool tc, F1 g1, F2
 template <typename C>
 static int inverse_nopiv_rec(const LaContext& ctx, int n, C* M, long long ld, C* ws, int* vflag,
                              const RecFork* fk = nullptr) {
-  constexpr int kInvLeaf = InvLeaf<C>::value;
   if (n <= kInvLeaf) {
     inv_leaf_kernel<C><<<1, kInvLeafThreads, 0, ctx.stream>>>(n, M, ld, (R_t<C>)ctx.pivot_tau, vflag);
     BEM_LAUNCH_CHECK();

@@ -40,3 +40,25 @@ def test_checked_lu_and_triangular_leaves_c128(cuda, n, nrhs):
              nat.ptr(scr), nat.ptr(status), nat.stream_ptr())
     X = np.linalg.solve(A, B)
     assert np.max(np.abs(Bt.cpu().numpy() - X)) <= 1e-13 * np.max(np.abs(X)) * np.sqrt(n)
+
+
+@pytest.mark.parametrize("dt,code,eps", [(np.complex64, nat.C64, 2.0 ** -24), (np.complex128, nat.C128, 2.0 ** -53)],
+                         ids=["c64", "c128"])
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 63, 64, 65, 67])
+def test_inverse_leaf_edges(cuda, n, dt, code, eps):
+    """The register Gauss-Jordan leaf at the edges of its 4 x 4 thread tiles
+    and of the 64 x 64 block.  The matrix is diagonally dominant with condition
+    number below 3, so the residual of the computed inverse stays below
+    16 n eps (a few roundings per step, n steps)."""
+    import torch
+    A = _dominant(n, 40 + n).astype(dt)
+    At = torch.as_tensor(A, device="cuda")
+    scr = torch.empty(int(nat.lib().bem200_inverse_nopiv_workspace_size(code, n)), dtype=torch.uint8, device="cuda")
+    ws = torch.empty(1, dtype=torch.uint8, device="cuda")
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    nat.call("bem200_inverse_nopiv", code, 0, n, nat.ptr(At), n, nat.ptr(ws), 0, nat.ptr(scr), 1e-2,
+             nat.ptr(info), nat.stream_ptr())
+    assert int(info.item()) == 0
+    X = At.cpu().numpy().astype(np.complex128)
+    r = np.abs(X @ A.astype(np.complex128) - np.eye(n)).max()
+    assert r < 16 * n * eps + 16 * eps, r
