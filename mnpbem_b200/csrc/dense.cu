@@ -2908,9 +2908,9 @@ __device__ __forceinline__ double2 leaf_recip(double2 p) { return crecip_newton<
 // back-to-back loop; 128 threads with 8 x 4 entries and the row scaled by its
 // owners before publishing took 28.7 and 47.2.  A pivot that is zero or below 1 / tau of
 // the largest |re| + |im| of the rows still to be eliminated raises *vflag.
-template <typename C>
-__global__ void __launch_bounds__(kInvLeafThreads, 1) inv_leaf_kernel(int nb, C* __restrict__ M, long long ld,
-                                                                      R_t<C> tau, int* __restrict__ vflag) {
+// kPt: the transposed inverse, zero beyond nb, also goes to pt (64 rows of ldt).
+template <typename C, bool kPt>
+__device__ __forceinline__ void inv_leaf(int nb, C* M, long long ld, R_t<C> tau, int* vflag, C* pt, int ldt) {
   constexpr int N = 64, T = 16, PQ = N / T;
   using R = R_t<C>;
   __shared__ __align__(16) C rowb[2][N];
@@ -2985,8 +2985,181 @@ __global__ void __launch_bounds__(kInvLeafThreads, 1) inv_leaf_kernel(int nb, C*
     for (int q = 0; q < PQ; ++q) {
       const int i = PQ * ty + p, c = PQ * tx + q;
       if (i < nb && c < nb) M[(long long)i * ld + c] = a[p][q];
+      if (kPt) pt[(size_t)c * ldt + i] = (i < nb && c < nb) ? a[p][q] : czero<C>();
     }
   if (__syncthreads_or(bad) && tid == 0 && vflag) atomicExch(vflag, 1);
+}
+template <typename C>
+__global__ void __launch_bounds__(kInvLeafThreads, 1) inv_leaf_kernel(int nb, C* __restrict__ M, long long ld,
+                                                                      R_t<C> tau, int* __restrict__ vflag) {
+  inv_leaf<C, false>(nb, M, ld, tau, vflag, nullptr, 0);
+}
+
+// Blocked Gauss-Jordan inversion in place, 64 columns per step, two launches
+// per step (complex64, kGjMin < n <= kGjMax).  With P the inverse of the
+// diagonal block of step k and R = P A_k: ,
+//   A_ij <- A_ij - A_ik R_j,  A_kj <- R_j,  A_ik <- -A_ik P,  A_kk <- P,
+// that is, for the columns of block k, R = P and the old A_ik counts as zero.
+// The diagonal blocks are the same Schur complements as in the recursion, so
+// the pivot checks are too.  gj_pivot_kernel inverts the diagonal block (CTA 0)
+// while its other CTAs copy the old row block (rowk, 64 x nn) and the old column
+// block transposed (colt, 64 x nn) to scratch, P transposed in the place of
+// block k: gj_step_kernel then updates M in place without ordering its CTAs.
+// nn = n rounded up to 64.  A step takes 20 us for the pivot block and 7 us for
+// the update up to n = 512 (17 at 768), against one pivot block and a share of
+// six products, each a launch of 6 us and more, in the recursion.  Whole
+// inverses, recursion -> this: n = 256 128.6 -> 129.5 us, 284 152.6 -> 151.1,
+// 384 203 -> 188, 512 296 -> 244, 704 441 -> 379, 768 483 -> 461, 1024 617 (with
+// two halves by this) -> 697; 1325 1186 -> 901, 2884 2927 -> 2749.
+constexpr int kGjMin = 256, kGjMax = 768;
+template <typename C>
+static bool gj_takes(int n) { return sizeof(C) == 8 && n > kGjMin && n <= kGjMax; }
+static size_t gj_scratch(int n) { return 128 * (size_t)(ceil_div(n, 64) * 64) + 2; }
+
+template <typename C>
+__global__ void __launch_bounds__(kInvLeafThreads, 1) gj_pivot_kernel(int n, int k0, C* __restrict__ M, long long ld,
+                                                                      int nn, C* __restrict__ rowk,
+                                                                      C* __restrict__ colt, R_t<C> tau,
+                                                                      int* __restrict__ vflag) {
+  const int w = min(64, n - k0);
+  if (blockIdx.x == 0) {
+    inv_leaf<C, true>(w, M + (long long)k0 * ld + k0, ld, tau, vflag, colt + k0, nn);
+    return;
+  }
+  const int j0 = 64 * (blockIdx.x - 1);
+  if (j0 == k0) return;
+  for (int e = threadIdx.x; e < 64 * 64; e += kInvLeafThreads) {
+    const int t = e >> 6, c = e & 63;
+    const bool in = t < w && j0 + c < n;
+    rowk[(size_t)t * nn + j0 + c] = in ? M[(long long)(k0 + t) * ld + j0 + c] : czero<C>();
+    colt[(size_t)t * nn + j0 + c] = in ? M[(long long)(j0 + c) * ld + k0 + t] : czero<C>();
+  }
+}
+
+// One 64 x 32 tile per CTA, rows of block i = blockIdx.y.  The four CTAs of a
+// cluster share a strip of columns: each forms 16 rows of its R and hands them
+// to the others through distributed shared memory, then updates its tile.
+// Thread (ty, tx) of 16 x 16 holds 4 x 2 entries.  Bound by latency (launch,
+// loads, one cluster barrier) up to n about 512, beyond by FP32 FMAs.
+constexpr int kGjCluster = 4;
+constexpr int kGjSmem = (64 * 16 + 64 * 64 + 2 * 64 * 32) * (int)sizeof(float2);
+__global__ void __cluster_dims__(1, kGjCluster, 1) __launch_bounds__(256, 3)
+    gj_step_kernel(int n, int k0, float2* __restrict__ M, long long ld, int nn, const float2* __restrict__ rowk,
+                   const float2* __restrict__ colt) {
+  extern __shared__ __align__(16) float2 gj_smem[];
+  float2* P = gj_smem;             // [t][r] = P_(16 rank + r, t)
+  float2* L = P + 64 * 16;         // [t][r] = A_ik (r, t)
+  float2* X = L + 64 * 64;         // [t][c] = A_kj (t, c)
+  float2* R = X + 64 * 32;         // [t][c]
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  const int rank = blockIdx.y % kGjCluster;  // the cluster is a run of blockIdx.y
+  const int i0 = 64 * blockIdx.y, c0 = 32 * blockIdx.x;
+  const bool piv_row = i0 == k0, piv_col = (c0 & ~63) == k0, used = i0 < n;  // piv_col: for the whole cluster
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // its wait: all four CTAs have started
+  if (used && !piv_row)
+    for (int e = tid; e < 64 * 32; e += 256) {
+      const int t = e >> 5, r = 2 * (e & 31);
+      cp_async_elem<16>(L + t * 64 + r, colt + (size_t)t * nn + i0 + r);
+    }
+  if (!piv_col) {
+    for (int e = tid; e < 64 * 16; e += 256) {
+      const int t = e >> 4, c = 2 * (e & 15);
+      cp_async_elem<16>(X + t * 32 + c, rowk + (size_t)t * nn + c0 + c);
+    }
+    for (int e = tid; e < 64 * 8; e += 256) {
+      const int t = e >> 3, r = 2 * (e & 7);
+      cp_async_elem<16>(P + t * 16 + r, colt + (size_t)t * nn + k0 + 16 * rank + r);
+    }
+  } else {
+    for (int e = tid; e < 64 * 32; e += 256) {  // R is a strip of P
+      const int r = e & 63, c = e >> 6;
+      R[r * 32 + c] = colt[(size_t)(c0 - k0 + c) * nn + k0 + r];
+    }
+  }
+  cp_async_commit();
+  float2 a[4][2];
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int i = i0 + 4 * ty + p, c = c0 + 2 * tx + q;
+      a[p][q] = (!piv_row && !piv_col && i < n && c < n) ? M[(long long)i * ld + c] : make_float2(0.f, 0.f);
+    }
+  cp_async_wait<0>();
+  __syncthreads();
+  if (!piv_col) {
+    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int t = 0; t < 64; ++t) {
+      const float2 s = P[t * 16 + ty];
+      const float4 x = *reinterpret_cast<const float4*>(X + t * 32 + 2 * tx);
+      r.x = fmaf(s.x, x.x, fmaf(-s.y, x.y, r.x));
+      r.y = fmaf(s.x, x.y, fmaf(s.y, x.x, r.y));
+      r.z = fmaf(s.x, x.z, fmaf(-s.y, x.w, r.z));
+      r.w = fmaf(s.x, x.w, fmaf(s.y, x.z, r.w));
+    }
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    const uint32_t own = su32(R + (16 * rank + ty) * 32 + 2 * tx);
+#pragma unroll
+    for (int c = 0; c < kGjCluster; ++c) {
+      uint32_t peer;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(peer) : "r"(own), "r"(c));
+      asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(peer), "f"(r.x), "f"(r.y), "f"(r.z), "f"(r.w)
+                   : "memory");
+    }
+    // the last access to a peer's shared memory: a CTA may exit after it
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  } else {
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  }
+  if (!used || (piv_row && piv_col)) return;  // below the matrix; P is in place already
+  if (piv_row) {
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) a[p][q] = R[(4 * ty + p) * 32 + 2 * tx + q];
+  } else {
+#pragma unroll 8
+    for (int t = 0; t < 64; ++t) {
+      const float4 x = *reinterpret_cast<const float4*>(R + t * 32 + 2 * tx);
+      const float2 xv[2] = {make_float2(x.x, x.y), make_float2(x.z, x.w)};
+      const float4 s01 = *reinterpret_cast<const float4*>(L + t * 64 + 4 * ty);
+      const float4 s23 = *reinterpret_cast<const float4*>(L + t * 64 + 4 * ty + 2);
+      const float2 sv[4] = {make_float2(s01.x, s01.y), make_float2(s01.z, s01.w), make_float2(s23.x, s23.y),
+                            make_float2(s23.z, s23.w)};
+#pragma unroll
+      for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          a[p][q].x = fmaf(-sv[p].x, xv[q].x, fmaf(sv[p].y, xv[q].y, a[p][q].x));
+          a[p][q].y = fmaf(-sv[p].x, xv[q].y, fmaf(-sv[p].y, xv[q].x, a[p][q].y));
+        }
+    }
+  }
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int i = i0 + 4 * ty + p, c = c0 + 2 * tx + q;
+      if (i < n && c < n) M[(long long)i * ld + c] = a[p][q];
+    }
+}
+
+static int inverse_gj(const LaContext& ctx, int n, float2* M, long long ld, float2* ws, int* vflag) {
+  const int blocks = ceil_div(n, 64), nn = 64 * blocks;
+  float2* rowk = reinterpret_cast<float2*>((reinterpret_cast<uintptr_t>(ws) + 15) & ~uintptr_t(15));
+  float2* colt = rowk + 64 * (size_t)nn;
+  BEM_CUDA_CHECK(set_kernel_attrs_once(gj_step_kernel, kGjSmem, false));
+  for (int k0 = 0; k0 < n; k0 += 64) {
+    gj_pivot_kernel<float2><<<1 + blocks, kInvLeafThreads, 0, ctx.stream>>>(n, k0, M, ld, nn, rowk, colt,
+                                                                            (float)ctx.pivot_tau, vflag);
+    BEM_LAUNCH_CHECK();
+    gj_step_kernel<<<dim3(2 * blocks, ceil_div(blocks, kGjCluster) * kGjCluster), 256, kGjSmem, ctx.stream>>>(n, k0, M, ld, nn, rowk, colt);
+    BEM_LAUNCH_CHECK();
+    count_launch();
+    count_launch();
+  }
+  return BEM200_OK;
 }
 
 // scratch elements inverse_nopiv needs for an n x n matrix
@@ -2995,6 +3168,7 @@ static size_t inverse_nopiv_scratch(int n) {
   // the inverse of A runs first, from the start of the scratch; then T1, T2
   // stay live while the inverse of S uses what follows them
   if (n <= kInvLeaf) return 0;
+  if (gj_takes<C>(n)) return gj_scratch(n);
   const int n1 = min(n - 1, ceil_div(n / 2, kInvLeaf) * kInvLeaf), n2 = n - n1;
   return max(inverse_nopiv_scratch<C>(n1), 2 * (size_t)n1 * n2 + inverse_nopiv_scratch<C>(n2));
 }
@@ -3037,6 +3211,8 @@ static int inverse_nopiv_rec(const LaContext& ctx, int n, C* M, long long ld, C*
     count_launch();
     return BEM200_OK;
   }
+  if constexpr (sizeof(C) == 8)
+    if (gj_takes<C>(n)) return inverse_gj(ctx, n, M, ld, ws, vflag);
   const int n1 = min(n - 1, ceil_div(n / 2, kInvLeaf) * kInvLeaf), n2 = n - n1;
   C* A = M;
   C* B = M + n1;

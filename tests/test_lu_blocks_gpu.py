@@ -62,3 +62,34 @@ def test_inverse_leaf_edges(cuda, n, dt, code, eps):
     X = At.cpu().numpy().astype(np.complex128)
     r = np.abs(X @ A.astype(np.complex128) - np.eye(n)).max()
     assert r < 16 * n * eps + 16 * eps, r
+
+
+@pytest.mark.parametrize("n", [256, 257, 319, 320, 321, 513, 700, 768, 769, 1100])
+def test_inverse_blocked_gauss_jordan(cuda, n):
+    """Blocked Gauss-Jordan inverse (complex64, 256 < n <= 768): ragged last
+    blocks, 4 to 12 row blocks (clusters of four) and both sides of its range
+    (769, 1100: two or three blocks of the recursion, rows of a larger matrix).
+    Every entry takes n rank-one updates on top of ceil(n / 64) block steps;
+    condition number below 3: residual below 16 sqrt(n) 2^-24 sqrt(n)."""
+    import torch
+    A = _dominant(n, 70 + n).astype(np.complex64)
+    big = torch.full((n + 1, n), 7.0, dtype=torch.complex64, device="cuda")  # a guard row below
+    big[:n] = torch.as_tensor(A, device="cuda")
+    scr = torch.empty(int(nat.lib().bem200_inverse_nopiv_workspace_size(nat.C64, n)), dtype=torch.uint8,
+                      device="cuda")
+    ws = torch.empty(1, dtype=torch.uint8, device="cuda")
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    nat.call("bem200_inverse_nopiv", nat.C64, 0, n, nat.ptr(big), n, nat.ptr(ws), 0, nat.ptr(scr), 1e-2,
+             nat.ptr(info), nat.stream_ptr())
+    assert int(info.item()) == 0
+    X = big[:n].cpu().numpy().astype(np.complex128)
+    r = np.abs(X @ A.astype(np.complex128) - np.eye(n)).max()
+    assert r < 16 * n * 2.0 ** -24, r
+    assert bool((big[n] == 7).all())
+    # a row exchange needed inside a diagonal block is reported
+    B = A.copy()
+    B[[130, 170]] = B[[170, 130]]
+    big[:n] = torch.as_tensor(B, device="cuda")
+    nat.call("bem200_inverse_nopiv", nat.C64, 0, n, nat.ptr(big), n, nat.ptr(ws), 0, nat.ptr(scr), 1e-2,
+             nat.ptr(info), nat.stream_ptr())
+    assert int(info.item()) == 1
