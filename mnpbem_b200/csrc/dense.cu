@@ -310,7 +310,7 @@ int gemm_v(const LaContext& ctx, int m, int n, int k, C alpha, RowView<C> A, Row
     if (n <= 8) return gemm_skinny<C, 8, z ? 1 : 2>(ctx, m, n, k, alpha, A, B, beta, Cv);
     return gemm_skinny<C, 16, 1>(ctx, m, n, k, alpha, A, B, beta, Cv);
   }
-  if (gemm_takes_tc<C>(ctx, m, n, k)) return gemm_tc<C>(ctx, m, n, k, alpha, A, B, beta, Cv);
+  if (gemm_takes_tc<C>(ctx, m, n, k)) return gemm_tc<C>(ctx, m, n, k, alpha, A, B, beta, Cv, n, alpha, beta);
   constexpr int BK = sizeof(C) == 16 ? 8 : 16;
   if ((long long)ceil_div(n, 32) * ceil_div(m, 32) < 74) {  // 32 x 32 tiles would fill fewer than half the SMs
     dim3 grid(ceil_div(n, 16), ceil_div(m, 16));
@@ -3220,10 +3220,24 @@ static int inverse_nopiv_rec(const LaContext& ctx, int n, C* M, long long ld, C*
   C* D = Cm + n1;
   int st;
   if ((st = inverse_nopiv_rec<C>(ctx, n1, A, ld, ws, vflag, fk))) return st;
+  const C one = cmake<C>(1.0, 0.0), mone = cmake<C>(-1.0, 0.0), zero = czero<C>();
+  if (gemm_takes_tc<C>(ctx, n1, n2, n1) && gemm_takes_tc<C>(ctx, n2, n1, n2) && gemm_tc_in_place<C>(ctx, n1, n2, n1) &&
+      gemm_tc_in_place<C>(ctx, n2, n1, n2) && gemm_tc_in_place<C>(ctx, n2, n, n1) &&
+      gemm_tc_in_place<C>(ctx, n1, n, n2)) {
+    // four products that read their operands before they write, so T1 and T2
+    // take the places of B and C: T1 = A^-1 B, [T2 | S] = [0 | D] + C [A^-1 | -T1],
+    // C = -S^-1 T2, [A | B] = [A^-1 | 0] - T1 [C | S^-1].  10 instead of 12 operand
+    // halves are split into residues, and 12 instead of 18 launches.
+    auto at = [&](C* p) { return plain(p, ld); };
+    if ((st = gemm_tc<C>(ctx, n1, n2, n1, one, at(A), at(B), zero, at(B), n2, one, zero))) return st;
+    if ((st = gemm_tc<C>(ctx, n2, n, n1, one, at(Cm), at(A), zero, at(Cm), n1, mone, one))) return st;
+    if ((st = inverse_nopiv_rec<C>(ctx, n2, D, ld, ws, vflag, fk))) return st;
+    if ((st = gemm_tc<C>(ctx, n2, n1, n2, mone, at(D), at(Cm), zero, at(Cm), n1, mone, zero))) return st;
+    return gemm_tc<C>(ctx, n1, n, n2, mone, at(B), at(Cm), one, at(A), n1, mone, zero);
+  }
   C* T1 = ws;                            // n1 x n2
   C* T2 = ws + (size_t)n1 * n2;          // n2 x n1
   C* rest = T2 + (size_t)n2 * n1;
-  const C one = cmake<C>(1.0, 0.0), mone = cmake<C>(-1.0, 0.0), zero = czero<C>();
   // T1 = A^-1 B and T2 = C A^-1 are independent
   const bool tc1 = gemm_takes_tc<C>(ctx, n1, n2, n1) || gemm_takes_tc<C>(ctx, n2, n1, n1);
   if ((st = gemm_pair<C>(

@@ -208,6 +208,12 @@ bool gemm_tc_two_fit(const LaContext& ctx, int m, int n, int k) {
   return ctx.engine == GemmEngine::kSimt || gemm_tc_workspace<C>(m, n, k, ctx.engine) / 4 <= ctx.ws_bytes / 3;
 }
 template <typename C>
-int gemm_tc(const LaContext& ctx, int m, int n, int k, C alpha, RowView<C> A, RowView<C> B, C beta, RowView<C> Cv);
+int gemm_tc(const LaContext& ctx, int m, int n, int k, C alpha, RowView<C> A, RowView<C> B, C beta, RowView<C> Cv,
+            int nsplit, C alpha2, C beta2);
+// Whether an m x n x k gemm_tc reads A and all its rows of B before it writes
+// (one pass over m and k; n in blocks of columns): Cv may then be the same
+// matrix as B, or overlap A.
+template <typename C>
+bool gemm_tc_in_place(const LaContext& ctx, int m, int n, int k);
 
 }  // namespace bem200

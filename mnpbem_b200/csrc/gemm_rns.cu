@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(THREADS, 1) rns_gemm_kernel(const __grid_const
 template <typename C>
 __global__ void __launch_bounds__(256) rns_merge_kernel(int m, int n, int Np, const uint8_t* __restrict__ res,
                                                         const int* __restrict__ sa, const int* __restrict__ sb,
-                                                        C alpha, C beta, RowView<C> Cv,
+                                                        C alpha, C beta, RowView<C> Cv, int nsplit, C alpha2, C beta2,
                                                         const __grid_constant__ MergeTab tab) {
   using T = Traits<C>;
   __shared__ __align__(16) C sh[8][128];
@@ -744,13 +744,14 @@ __global__ void __launch_bounds__(256) rns_merge_kernel(int m, int n, int Np, co
   }
   __syncwarp();
   C* out = &Cv.at(i, q0);
-  const bool use_beta = (beta.x != 0 || beta.y != 0);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int c = lane + 32 * j;
     if (q0 + c >= n) break;
-    C v = cmul(alpha, sh[wid][c]);
-    if (use_beta) v = cadd(v, cmul(beta, out[c]));
+    const bool lo = q0 + c < nsplit;
+    const C be = lo ? beta : beta2;
+    C v = cmul(lo ? alpha : alpha2, sh[wid][c]);
+    if (be.x != 0 || be.y != 0) v = cadd(v, cmul(be, out[c]));
     out[c] = v;
   }
 }
@@ -849,7 +850,14 @@ bool gemm_tc_fits(const LaContext& ctx, int m, int n, int k) {
 }
 
 template <typename C>
-int gemm_tc(const LaContext& ctx, int m, int n, int k, C alpha, RowView<C> A, RowView<C> B, C beta, RowView<C> Cv) {
+bool gemm_tc_in_place(const LaContext& ctx, int m, int n, int k) {
+  int mb, nb, kb;
+  return ctx.ws && rns::fit_blocks<C>(m, n, k, ctx.ws_bytes, mb, nb, kb) && mb == m && kb == k;
+}
+
+template <typename C>
+int gemm_tc(const LaContext& ctx, int m, int n, int k, C alpha, RowView<C> A, RowView<C> B, C beta, RowView<C> Cv,
+            int nsplit, C alpha2, C beta2) {
   using namespace rns;
   using T = Traits<C>;
   BEM_REQUIRE(ctx.engine == GemmEngine::kTc, BEM200_ERR_UNSUPPORTED, "gemm: the TF32 tensor-core engine is not built");
@@ -865,19 +873,20 @@ int gemm_tc(const LaContext& ctx, int m, int n, int k, C alpha, RowView<C> A, Ro
       for (int n0 = 0; n0 < n; n0 += nb) {
         const int mm = std::min(mb, m - m0), nn = std::min(nb, n - n0), kk = std::min(kb, k - k0);
         const Plan p = plan<C>(mm, nn, kk);
-        uint8_t* pa = reinterpret_cast<uint8_t*>(w);
+        // A's scales and planes come first: they stay for the other blocks of n
+        int* sa = reinterpret_cast<int*>(w);
+        uint8_t* pa = reinterpret_cast<uint8_t*>(w) + p.sa;
         uint8_t* pb = pa + p.a;
         uint8_t* pc = pb + p.b;
-        int* sa = reinterpret_cast<int*>(pc + p.c);
-        int* sb = reinterpret_cast<int*>(pc + p.c + p.sa);
+        int* sb = reinterpret_cast<int*>(pc + p.c);
         int* status = ctx.dstatus;
         if (!status) {
-          status = reinterpret_cast<int*>(pc + p.c + p.sa + p.sb);
+          status = reinterpret_cast<int*>(pc + p.c + p.sb);
           BEM_CUDA_CHECK(cudaMemsetAsync(status, 0, sizeof(int), ctx.stream));
         }
         const RowView<C> Ab = A.sub(m0, k0), Bb = B.sub(k0, n0), Cb = Cv.sub(m0, n0);
         const int chunks = p.Kp / 128, wpr = chunks >= 8 ? 8 : (chunks >= 4 ? 4 : (chunks >= 2 ? 2 : 1));
-        const int ablocks = ceil_div(mm, 8 / wpr);
+        const int ablocks = n0 == 0 ? ceil_div(mm, 8 / wpr) : 0;
         rns_split_kernel<C><<<ablocks + ceil_div(nn, 8), 256, 0, ctx.stream>>>(
             mm, nn, kk, Ab, Bb, p.Mp, p.Np, p.Kp, ablocks, wpr, sa, sb, pa, pb, tab.split);
         BEM_LAUNCH_CHECK();
@@ -900,7 +909,8 @@ int gemm_tc(const LaContext& ctx, int m, int n, int k, C alpha, RowView<C> A, Ro
         BEM_LAUNCH_CHECK();
         const C b0 = k0 == 0 ? beta : cmake<C>(1.0, 0.0);
         rns_merge_kernel<C><<<ceil_div((long long)mm * ((nn + 127) / 128), 8), 256, 0, ctx.stream>>>(
-            mm, nn, p.Np, pc, sa, sb, alpha, b0, Cb, tab.merge);
+            mm, nn, p.Np, pc, sa, sb, alpha, b0, Cb, nsplit - n0, alpha2, k0 == 0 ? beta2 : cmake<C>(1.0, 0.0),
+            tab.merge);
         BEM_LAUNCH_CHECK();
       }
   return BEM200_OK;
@@ -909,7 +919,8 @@ int gemm_tc(const LaContext& ctx, int m, int n, int k, C alpha, RowView<C> A, Ro
 #define RNS_INST(C)                                                                                              \
   template size_t gemm_tc_workspace<C>(int, int, int, GemmEngine);                                               \
   template bool gemm_tc_fits<C>(const LaContext&, int, int, int);                                                \
-  template int gemm_tc<C>(const LaContext&, int, int, int, C, RowView<C>, RowView<C>, C, RowView<C>);
+  template bool gemm_tc_in_place<C>(const LaContext&, int, int, int);                                            \
+  template int gemm_tc<C>(const LaContext&, int, int, int, C, RowView<C>, RowView<C>, C, RowView<C>, int, C, C);
 RNS_INST(float2)
 RNS_INST(double2)
 

@@ -93,3 +93,25 @@ def test_inverse_blocked_gauss_jordan(cuda, n):
     nat.call("bem200_inverse_nopiv", nat.C64, 0, n, nat.ptr(big), n, nat.ptr(ws), 0, nat.ptr(scr), 1e-2,
              nat.ptr(info), nat.stream_ptr())
     assert int(info.item()) == 1
+
+
+@pytest.mark.parametrize("n,part", [(830, 1.0), (1001, 1.0), (1500, 1.0), (1500, 0.4), (1500, 0.1)])
+def test_inverse_in_place_products(cuda, n, part):
+    """complex64 inverse whose top products run on the tensor cores in place,
+    with the workspace of one pass, one that splits the columns (0.4) and one
+    too small to keep the operands (0.1: products through scratch).  The
+    operands are rounded to 2^-25 of their row norms: same bound as above."""
+    import torch
+    A = _dominant(n, 90 + n).astype(np.complex64)
+    At = torch.as_tensor(A, device="cuda")
+    L = nat.lib()
+    scr = torch.empty(int(L.bem200_inverse_nopiv_workspace_size(nat.C64, n)), dtype=torch.uint8, device="cuda")
+    wsb = int(part * L.bem200_gemm_workspace_size(1, n, n, n // 2 + 64))
+    ws = torch.empty(wsb, dtype=torch.uint8, device="cuda")
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    nat.call("bem200_inverse_nopiv", nat.C64, 1, n, nat.ptr(At), n, nat.ptr(ws), wsb, nat.ptr(scr), 1e-2,
+             nat.ptr(info), nat.stream_ptr())
+    assert int(info.item()) == 0
+    X = At.cpu().numpy().astype(np.complex128)
+    r = np.abs(X @ A.astype(np.complex128) - np.eye(n)).max()
+    assert r < 16 * n * 2.0 ** -24, r
