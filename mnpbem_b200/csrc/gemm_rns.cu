@@ -233,7 +233,10 @@ __device__ __forceinline__ void residues4(const int4 (&re)[W], const int4 (&im)[
 template <typename C>
 __device__ __forceinline__ void emit(const int4 (&re)[Traits<C>::kWords], const int4 (&im)[Traits<C>::kWords],
                                      uint8_t* out, size_t plane, const SplitTab& tab) {
-#pragma unroll 1
+  // complex64: unrolled, the table's entries become constant operands; the
+  // complex128 body is too long for that (a 5768-face LU loses 0.5 %)
+  constexpr int kUnroll = Traits<C>::N <= 8 ? Traits<C>::N : 1;
+#pragma unroll kUnroll
   for (int t = 0; t < Traits<C>::N; ++t) {
     uint32_t u, v;
     residues4<Traits<C>::kWords>(re, im, tab.mod[t], u, v);
@@ -251,8 +254,10 @@ __device__ __forceinline__ void emit(const int4 (&re)[Traits<C>::kWords], const 
 // ([rows][Kp]; the columns k..Kp are 0).  Blocks beyond: 8 columns of B, read
 // once for the norms and again (from L2) in tiles of 128 rows, written
 // transposed ([columns of B][Kp]; the K padding of B is not written, it meets
-// A's zeros).  Integer issue bounds it: 13 (complex64) / 15 (complex128)
-// instructions per entry and modulus.
+// A's zeros).  Instruction issue (64 % of the slots) and latency at half
+// occupancy bound it: 13 (complex64) / 15 (complex128) instructions per entry
+// and modulus; 2884^3 complex64 operands take 120 us with the moduli unrolled,
+// 133 with a loop over them.  Norms summed in FP32 do not help.
 constexpr int kRowChunks = kBlockK / 128 / 8;  // chunks per warp of the longest row
 template <typename C>
 __global__ void __launch_bounds__(256) rns_split_kernel(int m, int n, int k, RowView<C> A, RowView<C> B, int Mp, int Np,
