@@ -9,8 +9,8 @@
 //   * recursive TRSM with small substitution kernels at the leaves, and a
 //     blocked triangular solve for few right-hand sides in which row blocks
 //     wait on flags of the blocks they depend on (bounded waits).
-//   * GEMM on row views: CUDA-core kernel for complex128 (FP64 FMA) /
-//     complex64, and the tcgen05 tensor-core path for complex64 (gemm_tc.cu).
+//   * GEMM on row views: CUDA-core kernels for small products, the int8
+//     tensor cores for large ones (gemm_rns.cu).
 // Pivot choice follows LAPACK izamax: largest |re| + |im|.
 #include <cooperative_groups.h>
 
@@ -2586,7 +2586,7 @@ static int getrf_dispatch(const LaContext& ctx, int n, C* A, long long ld, int32
                           int32_t* scratch);
 
 // Checked diagonal pivots (ctx.diag_pivots): the same blocked look-ahead LU
-// with panel_nopiv panels; the panels' verdicts collect in a flag in the LU
+// with 64-column panels without exchanges; the panels' verdicts collect in a flag in the LU
 // scratch, turned into *info = -BEM200_ERR_PIVOTING at the end.
 template <typename C>
 int getrf(const LaContext& ctx, int n, C* A, long long ld, int32_t* rowmap, int32_t* ipiv, int32_t* scratch) {
@@ -2874,7 +2874,8 @@ int inverse(const LaContext& ctx, int n, const C* LU, long long ld, const int32_
 //   A^-1 (recursive), T1 = A^-1 B, T2 = C A^-1, S = D - C T1, S^-1 (recursive),
 //   B <- -T1 S^-1, C <- -S^-1 T2, A <- A^-1 - B T2.
 // Nearly all of the 8 n^3 flops land in the large GEMMs of the top levels
-// (tensor cores for complex64); the leaves (<= 64 x 64) are inverted by
+// (tensor cores for complex64, in place); blocks of 257 to 768 rows go by
+// blocked Gauss-Jordan steps (complex64), the leaves (<= 64 x 64) by
 // Gauss-Jordan elimination in registers.  No row exchanges means no check
 // of the leaves' pivots can cover the rows outside them, so the caller
 // verifies the result with inverse_probe (M^-1 (M v) = v for a fixed
