@@ -731,9 +731,37 @@ __global__ void __launch_bounds__(kRegThreads, 1) panel_lu_reg_kernel(int m, int
   }
 }
 
+__device__ __forceinline__ double2 crecip_pivot(double2 p);
+__device__ __forceinline__ float2 crecip_pivot(float2 p);
+// 1 / pivot, 0 for a zero or NaN pivot; the division for magnitudes whose scale
+// would leave the exponent range
+__device__ __forceinline__ double2 panel_recip(double2 p) {
+  if (!(cabs1(p) > 0)) return czero<double2>();
+  return cabs1(p) < 1e300 ? crecip_pivot(p) : cdiv(make_double2(1.0, 0.0), p);
+}
+__device__ __forceinline__ float2 panel_recip(float2 p) {
+  return cabs1(p) > 0 ? cdiv(make_float2(1.f, 0.f), p) : czero<float2>();
+}
+
+// The same maximum by three warp reductions of 32-bit words (the high and low
+// words of 1 + the bits of b, which are monotonic for b >= 0, then the lowest
+// row), about 80 cycles instead of five rounds of three shuffles (200).
+// b = -1 marks a lane without a candidate.
+template <typename R>
+__device__ __forceinline__ void warp_argmax_redux(R& b, int& br) {
+  const unsigned long long key = b >= R(0) ? 1ull + (unsigned long long)__double_as_longlong((double)b) : 0ull;
+  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  const bool first = hi == mh && lo == ml;
+  br = (int)__reduce_min_sync(0xffffffffu, first ? (unsigned)br : (unsigned)INT_MAX);
+  const unsigned long long top = ((unsigned long long)mh << 32) | ml;
+  b = top ? (R)__longlong_as_double((long long)(top - 1ull)) : R(-1);
+}
+
 // ----------------------------------------------------------------------------
-// Push panel: one panel row per thread, held in registers (32 complex), with
-// the column loop fully unrolled so every register index is static.  Per
+// Push panel: one panel row per thread, held in registers (32 complex)
+// that rotate one place per column, so every register index is static.  Per
 // column: warp argmax -> the winning lane parks its row in shared memory ->
 // warp 0 picks the CTA's best row and PUSHES it (value, index, 32 elements)
 // into the candidate slot of every CTA of the cluster with DSMEM stores ->
@@ -742,6 +770,9 @@ __global__ void __launch_bounds__(kRegThreads, 1) panel_lu_reg_kernel(int m, int
 // remotely, so the barrier is the only cluster-wide latency per column.
 // Candidate slots are double buffered: slot t & 1 is rewritten at column t + 2,
 // after every CTA has passed barrier t + 1 and thus finished reading it.
+// Latency bound: the LU of 1537 complex128 rows takes 5.6 ms; with five-round
+// shuffle reductions, a division per column and a select chain over the row's
+// registers (89 us per panel) it took 6.6.
 constexpr int kPushThreads = 384;
 constexpr int kPushWarps = kPushThreads / 32;
 constexpr int kPushMaxCluster = 16;
@@ -782,22 +813,24 @@ __global__ void __launch_bounds__(kPushThreads, 1) panel_lu_push_kernel(int m, i
   const unsigned kFull = 0xffffffffu;
 
   // The column loop stays rolled (a fully unrolled one overflows the
-  // instruction cache); column t of the register row is read with a select
-  // chain and updated with predicated FMAs, so every register index is static.
+  // instruction cache) and the row rotates through the registers: at column t
+  // register c holds column (t + c) mod 32, so column t is v[0], an update
+  // writes one place to the left and the multiplier goes to the end.
 #pragma unroll 1
   for (int t = 0; t < w; ++t) {
     const int buf = t & 1;
-    C vt = v[0];
-#pragma unroll
-    for (int c = 1; c < kPanelNB; ++c)
-      if (c == t) vt = v[c];
+    const C vt = v[0];
     // warp candidate; the winning lane parks its row in shared memory
     Real wb = act ? pmag(vt) : (Real)-1;
     int wi = act ? prow_id : INT_MAX;
-    warp_argmax<C>(wb, wi);
+    warp_argmax_redux(wb, wi);
     if (act && wi == prow_id) {
 #pragma unroll
-      for (int c = 0; c < kPanelNB; ++c) sh.wrow[wid][c] = v[c];
+      for (int g = 0; g < kPanelNB; g += 8)
+        if (g + t < kPanelNB) {  // columns t .. 31 only
+#pragma unroll
+          for (int c = g; c < g + 8; ++c) sh.wrow[wid][c] = v[c];
+        }
     }
     if (lane == 0) {
       sh.wval[wid] = wb;
@@ -809,7 +842,7 @@ __global__ void __launch_bounds__(kPushThreads, 1) panel_lu_push_kernel(int m, i
       int bi = lane < nwarps ? sh.widx[lane] : INT_MAX;
       const Real b0 = b;
       const int i0 = bi;
-      warp_argmax<C>(b, bi);
+      warp_argmax_redux(b, bi);
       const unsigned msk = __ballot_sync(kFull, lane < nwarps && i0 == bi && b0 == b);
       const int ww = msk ? __ffs(msk) - 1 : 0;
       const C e = sh.wrow[ww][lane];
@@ -829,7 +862,7 @@ __global__ void __launch_bounds__(kPushThreads, 1) panel_lu_push_kernel(int m, i
     int bi = lane < cs ? sh.crow[buf][lane] : INT_MAX;
     const Real b0 = b;
     const int i0 = bi;
-    warp_argmax<C>(b, bi);
+    warp_argmax_redux(b, bi);
     const unsigned msk = __ballot_sync(kFull, lane < cs && i0 == bi && b0 == b);
     const int wc = msk ? __ffs(msk) - 1 : 0;
     const int p = min(bi, m - 1);  // an unused row always exists: bi < m
@@ -838,30 +871,34 @@ __global__ void __launch_bounds__(kPushThreads, 1) panel_lu_push_kernel(int m, i
       if (!(b > 0) && !sh.singular) sh.singular = t + 1;
     }
     const C* prow = sh.cand[buf][wc];
-    const C piv = prow[t];
+    const C piv = prow[0];
     // multipliers use the reciprocal of the pivot, as LAPACK's scaling does
-    const C inv = cabs1(piv) > 0 ? cdiv(cmake<C>(1.0, 0.0), piv) : czero<C>();
+    const C inv = panel_recip(piv);
     if (prow_id == p) act = false;  // the pivot row becomes a row of U
-    if (act) {
-      const C l = cmul(vt, inv);
+    const C l = act ? cmul(vt, inv) : vt;  // a finished row rotates unchanged
 #pragma unroll
-      for (int g = 0; g < kPanelNB; g += 8) {
-        if (g + 7 >= t) {  // uniform: skip groups left of the pivot column
+    for (int g = 0; g < kPanelNB; g += 8) {
+      if (act && g + t < kPanelNB) {
 #pragma unroll
-          for (int c = g; c < g + 8; ++c) {
-            const C u = csub(v[c], cmul(l, prow[c]));
-            v[c] = (c > t) ? u : ((c == t) ? l : v[c]);
-          }
+        for (int c = max(g, 1); c < g + 8; ++c) {
+          const C u = csub(v[c], cmul(l, prow[c]));
+          v[c - 1] = c + t < kPanelNB ? u : v[c];
         }
+      } else {
+#pragma unroll
+        for (int c = max(g, 1); c < g + 8; ++c) v[c - 1] = v[c];
       }
     }
+    v[kPanelNB - 1] = l;
   }
   // every remote store happened before the last barrier: no CTA touches
   // another's shared memory from here on
   if (tid < rcount) {
 #pragma unroll
-    for (int c = 0; c < kPanelNB; ++c)
-      if (c < w) A[phys * ld + col + c] = v[c];
+    for (int c = 0; c < kPanelNB; ++c) {
+      const int cc = (c + w) & (kPanelNB - 1);
+      if (cc < w) A[phys * ld + col + cc] = v[c];
+    }
   }
   __syncthreads();
   if (rank == 0 && wid == 0) {

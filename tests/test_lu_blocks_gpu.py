@@ -115,3 +115,33 @@ def test_inverse_in_place_products(cuda, n, part):
     X = At.cpu().numpy().astype(np.complex128)
     r = np.abs(X @ A.astype(np.complex128) - np.eye(n)).max()
     assert r < 16 * n * 2.0 ** -24, r
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 127, 129, 200, 513])
+@pytest.mark.parametrize("scale", [0, 500, -500])
+def test_pivoted_panel_c128(cuda, n, scale):
+    """Partially pivoted complex128 panels (rows rotating through registers):
+    ragged last panels, one to several CTAs, ties in the first column (the
+    first maximum wins), entries near 2^+-500.  The pivots are scipy's, and
+    |P A - L U| <= 8 n eps |L| |U| elementwise, the bound of complex Gaussian
+    elimination."""
+    import torch
+    from scipy.linalg import lu_factor
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    A[:, 0] = np.array([1, -1, 1j, -1j])[rng.integers(0, 4, n)]
+    A *= 2.0 ** scale
+    L = nat.lib()
+    At = torch.as_tensor(A, device="cuda").clone()
+    rowmap, ipiv = (torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2))
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    wsb = int(L.bem200_getrf_workspace_size(nat.C128, 0, n))
+    ws = torch.empty(wsb, dtype=torch.uint8, device="cuda")
+    nat.call("bem200_getrf_ex", nat.C128, 0, n, nat.ptr(At), n, nat.ptr(rowmap), nat.ptr(ipiv), nat.ptr(info),
+             nat.ptr(ws), wsb, 0, 0, nat.stream_ptr())
+    assert int(info.item()) == 0
+    assert np.array_equal(ipiv.cpu().numpy(), lu_factor(A)[1])
+    P = rowmap.cpu().numpy()
+    F = At.cpu().numpy()[P]
+    Lo, U = np.tril(F, -1) + np.eye(n), np.triu(F)
+    assert np.all(np.abs(A[P] - Lo @ U) <= 8 * n * 2.0 ** -53 * (np.abs(Lo) @ np.abs(U)))
