@@ -3050,9 +3050,9 @@ __global__ void __launch_bounds__(kInvLeafThreads, 1) inv_leaf_kernel(int nb, C*
 // 384 203 -> 188, 512 296 -> 244, 704 441 -> 379, 768 483 -> 461, 1024 617 (with
 // two halves by this) -> 697; 1325 1186 -> 901, 2884 2927 -> 2749.
 constexpr int kGjMin = 256, kGjMax = 768;
+static size_t gj_scratch(int n) { return 128 * (size_t)(ceil_div(n, 64) * 64) + 2; }
 template <typename C>
 static bool gj_takes(int n) { return sizeof(C) == 8 && n > kGjMin && n <= kGjMax; }
-static size_t gj_scratch(int n) { return 128 * (size_t)(ceil_div(n, 64) * 64) + 2; }
 
 template <typename C>
 __global__ void __launch_bounds__(kInvLeafThreads, 1) gj_pivot_kernel(int n, int k0, C* __restrict__ M, long long ld,
@@ -3206,9 +3206,9 @@ static size_t inverse_nopiv_scratch(int n) {
   // the inverse of A runs first, from the start of the scratch; then T1, T2
   // stay live while the inverse of S uses what follows them
   if (n <= kInvLeaf) return 0;
-  if (gj_takes<C>(n)) return gj_scratch(n);
   const int n1 = min(n - 1, ceil_div(n / 2, kInvLeaf) * kInvLeaf), n2 = n - n1;
-  return max(inverse_nopiv_scratch<C>(n1), 2 * (size_t)n1 * n2 + inverse_nopiv_scratch<C>(n2));
+  const size_t rec = max(inverse_nopiv_scratch<C>(n1), 2 * (size_t)n1 * n2 + inverse_nopiv_scratch<C>(n2));
+  return n > kGjMin && n <= kGjMax ? max(rec, gj_scratch(n)) : rec;  // the same count for both types
 }
 
 // A side stream and two events of the recording thread: in a recorded graph
