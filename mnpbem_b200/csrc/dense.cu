@@ -1514,7 +1514,7 @@ __global__ void __launch_bounds__(kCaluThreads, 1) panel_calu_kernel(int m, int 
 // that property, so their panels can skip the column-wide pivot search that
 // bounds the pivoted panels.  Two launches per 64 columns: one CTA factors the
 // 64 x 64 diagonal block in registers (panel_diag_kernel), then the rows below
-// it are multiplied by U11^-1 (trsm_leaf with the check).  Column j fails the
+// it are solved with U11 by substitution (trsm_leaf with the check).  Column j fails the
 // check when some row has |a_ij^(j)|_1 > tau |a_jj^(j)|_1; a failing panel
 // raises ctx.vflag and the caller factors the matrix again with partial
 // pivoting.  With tau = 1 a passing matrix gets LAPACK's partial-pivoting
@@ -1658,7 +1658,7 @@ static int panel_lu(const LaContext& ctx, int m, int w, C* A, long long ld, int 
                                                     (R_t<C>)ctx.pivot_tau);
     BEM_LAUNCH_CHECK();
     const RowView<C> V{A, ld, rowmap, col};
-    return trsm_leaf_rows_checked<C>(ctx, w, m - w, V, V.sub(w, 0));  // L21 = A21 U11^-1
+    return trsm_leaf_rows_checked<C>(ctx, w, m - w, V, V.sub(w, 0));  // L21 U11 = A21
   }
   if constexpr (sizeof(C) == 8) {
     if (ctx.tournament && m > kCaluMinRows && m <= kCaluMaxCluster * kCaluThreads) {
@@ -1824,6 +1824,90 @@ enum LeafKind : int {
   kRightLowerUnit = 3,  // X <- X L^-1
 };
 
+// Blocked substitution, K as above: T x = b for NV right-hand vectors per CTA.
+// Thread (g, v) of G = 256 / NV groups holds rows R g .. R g + R - 1 (R = NV / 4) of
+// vector v in registers.  Step b: group b solves its R x R triangle and publishes
+// x; the groups below take it off their rows (R^2 complex FMAs): one barrier per
+// step.  The order of operations is that of plain substitution, so an element
+// before its division is the eliminated entry a_ie^(e), on which kCheck decides:
+// |a_ie^(e)|_1 > tau |U_ee|_1 (also for U_ee = 0) raises *vflag.
+template <typename C, int K, int NV, bool kCheck>
+__global__ void __launch_bounds__(kLeafThreads) trsm_leaf_kernel(int m, int nvec, RowView<C> T, RowView<C> B,
+                                                                 double tau, int* __restrict__ vflag) {
+  constexpr int NB = LeafNB<C>::value, MP = NB + 1, VP = NV + 1, R = NV / 4;
+  constexpr bool kLeft = (K == kLeftLowerUnit || K == kLeftUpper);
+  constexpr bool kForward = (K == kLeftLowerUnit || K == kRightUpper);
+  constexpr bool kUnit = (K == kLeftLowerUnit || K == kRightLowerUnit);
+  static_assert(R * (kLeafThreads / NV) == NB, "leaf layout");
+  extern __shared__ __align__(16) unsigned char leaf_smem[];
+  using D = double2;  // both types solve in FP64
+  D* M = reinterpret_cast<D*>(leaf_smem);  // [NB][MP]: the triangle
+  D* V = M + NB * MP;                      // [NB][VP]: element e of vector v
+  __shared__ D rinv[NB];
+  const int tid = threadIdx.x;
+  const int v0 = blockIdx.x * NV;
+  const int nv = min(NV, nvec - v0);
+  // canonical lower triangle: element e of a backward kind is row m - 1 - e
+  for (int idx = tid; idx < NB * NB; idx += kLeafThreads) {
+    const int e = kLeft ? idx / NB : idx % NB, r = kLeft ? idx % NB : idx / NB;
+    D t = make_double2(e == r ? 1.0 : 0.0, 0.0);
+    if (e < m && r <= e && !(kUnit && e == r)) {
+      const int fe = kForward ? e : m - 1 - e, fr = kForward ? r : m - 1 - r;
+      const C g = kLeft ? T.at(fe, fr) : T.at(fr, fe);
+      t = make_double2(g.x, g.y);
+    }
+    M[e * MP + r] = t;
+    if (!kUnit && e == r) rinv[e] = kCheck ? crecip_scaled(t) : cdiv(make_double2(1.0, 0.0), t);
+  }
+  for (int idx = tid; idx < NB * NV; idx += kLeafThreads) {
+    const int e = kLeft ? idx / NV : idx % NB, v = kLeft ? idx % NV : idx / NB;
+    const int fe = kForward ? e : m - 1 - e;
+    const C g = (e < m && v < nv) ? (kLeft ? B.at(fe, v0 + v) : B.at(v0 + v, fe)) : czero<C>();
+    V[e * VP + v] = make_double2(g.x, g.y);
+  }
+  __syncthreads();
+  const int v = tid % NV, g = tid / NV, e0 = R * g;
+  D x[R];
+#pragma unroll
+  for (int i = 0; i < R; ++i) x[i] = V[(e0 + i) * VP + v];
+  bool bad = false;
+#pragma unroll 1
+  for (int b = 0; R * b < m; ++b) {
+    if (g == b) {
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const D* col = M + e0 * MP + e0 + i;
+        if (kCheck && pmag(x[i]) > tau * pmag(col[i * MP])) bad = true;
+        if (!kUnit) x[i] = cmul(x[i], rinv[e0 + i]);
+        V[(e0 + i) * VP + v] = x[i];
+#pragma unroll
+        for (int k = i + 1; k < R; ++k) cmsub(x[k], col[k * MP], x[i]);
+      }
+    }
+    __syncthreads();
+    if (g > b && e0 < m) {
+      const D* blk = M + e0 * MP + R * b;
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const D xj = V[(R * b + j) * VP + v];
+#pragma unroll
+        for (int i = 0; i < R; ++i) cmsub(x[i], blk[i * MP + j], xj);
+      }
+    }
+  }
+  for (int idx = tid; idx < NB * NV; idx += kLeafThreads) {
+    const int e = kLeft ? idx / NV : idx % NB, w = kLeft ? idx % NV : idx / NB;
+    if (w >= nv || e >= m) continue;
+    const int fe = kForward ? e : m - 1 - e;
+    const D r = V[e * VP + w];
+    const C o = cmake<C>(r.x, r.y);
+    if constexpr (kLeft) B.at(fe, v0 + w) = o; else B.at(v0 + w, fe) = o;
+  }
+  if constexpr (kCheck) {
+    if (__syncthreads_or(bad) && tid == 0 && vflag) atomicExch(vflag, 1);
+  }
+}
+
 // acc[p][v] += sum_{r < 32} M[row0 + ty + 16 p][r0 + r] V[r0 + r][tx + 16 v] for the 2 x NV / 16 block of a thread
 template <int NVT, int MP, int VP>
 __device__ __forceinline__ void leaf_product(const double2* M, const double2* V, int row0, int r0, int ty, int tx,
@@ -1842,9 +1926,8 @@ __device__ __forceinline__ void leaf_product(const double2* M, const double2* V,
   }
 }
 
-template <typename C, int K, int NV, bool kCheck>
-__global__ void __launch_bounds__(kLeafThreads) trsm_leaf_kernel(int m, int nvec, RowView<C> T, RowView<C> B,
-                                                                 double tau, int* __restrict__ vflag) {
+template <typename C, int K, int NV>
+__global__ void __launch_bounds__(kLeafThreads) trsm_leaf_inv_kernel(int m, int nvec, RowView<C> T, RowView<C> B) {
   constexpr int NB = LeafNB<C>::value, MP = NB + 1, VP = NV + 1, NVT = NV / 16;
   constexpr bool kLeft = (K == kLeftLowerUnit || K == kLeftUpper);
   constexpr bool kForward = (K == kLeftLowerUnit || K == kRightUpper);
@@ -1853,7 +1936,7 @@ __global__ void __launch_bounds__(kLeafThreads) trsm_leaf_kernel(int m, int nvec
   using D = double2;  // both types solve in FP64: the inverses lose nothing against substitution
   D* M = reinterpret_cast<D*>(leaf_smem);  // [NB][MP]: the triangle, then the inverses of its diagonal blocks
   D* V = M + NB * MP;                      // [NB][VP]: element e of vector v
-  __shared__ D rinv[NB], diag[NB], tmp[512];
+  __shared__ D rinv[NB], tmp[512];
   const int tid = threadIdx.x;
   const int v0 = blockIdx.x * NV;
   const int nv = min(NV, nvec - v0);
@@ -1868,8 +1951,7 @@ __global__ void __launch_bounds__(kLeafThreads) trsm_leaf_kernel(int m, int nvec
     }
     M[e * MP + r] = t;
     if (e == r) {
-      diag[e] = t;
-      rinv[e] = kUnit ? t : crecip_newton<kCheck>(t);
+      rinv[e] = kUnit ? t : crecip_newton<false>(t);
     }
   }
   for (int idx = tid; idx < NB * NV; idx += kLeafThreads) {
@@ -1955,20 +2037,13 @@ __global__ void __launch_bounds__(kLeafThreads) trsm_leaf_kernel(int m, int nvec
     put(32, acc);
     __syncthreads();
   }
-  bool bad = false;
   for (int idx = tid; idx < NB * NV; idx += kLeafThreads) {
     const int e = kLeft ? idx / NV : idx % NB, v = kLeft ? idx % NV : idx / NB;
     if (v >= nv || e >= m) continue;
     const int fe = kForward ? e : m - 1 - e;
     const D r = V[e * VP + v];
-    if constexpr (kCheck) {  // the multiplier times the pivot is the eliminated entry a_ie^(e)
-      if (pmag(cmul(r, diag[e])) > tau * pmag(diag[e])) bad = true;
-    }
     const C g = cmake<C>(r.x, r.y);
     if constexpr (kLeft) B.at(fe, v0 + v) = g; else B.at(v0 + v, fe) = g;
-  }
-  if constexpr (kCheck) {
-    if (__syncthreads_or(bad) && tid == 0 && vflag) atomicExch(vflag, 1);
   }
 }
 
@@ -2074,6 +2149,13 @@ static constexpr size_t leaf_smem_bytes() {
 
 template <typename C, int K, int NV, bool kCheck>
 static int trsm_leaf_launch(const LaContext& ctx, int m, int nvec, RowView<C> T, RowView<C> B) {
+  if constexpr (!kCheck) {
+    auto kern = trsm_leaf_inv_kernel<C, K, NV>;
+    BEM_CUDA_CHECK(set_kernel_attrs_once(kern, (int)leaf_smem_bytes<C, NV>(), false));
+    kern<<<ceil_div(nvec, NV), kLeafThreads, leaf_smem_bytes<C, NV>(), ctx.stream>>>(m, nvec, T, B);
+    BEM_LAUNCH_CHECK();
+    return BEM200_OK;
+  }
   auto kern = trsm_leaf_kernel<C, K, NV, kCheck>;
   BEM_CUDA_CHECK(set_kernel_attrs_once(kern, (int)leaf_smem_bytes<C, NV>(), false));
   kern<<<ceil_div(nvec, NV), kLeafThreads, leaf_smem_bytes<C, NV>(), ctx.stream>>>(m, nvec, T, B, (double)ctx.pivot_tau,
