@@ -1807,13 +1807,9 @@ static int panel_lu(const LaContext& ctx, int m, int w, C* A, long long ld, int 
 // ===================================================================== TRSM leaves
 // A leaf solves with a triangle of m <= NB = 64 rows; larger triangles recurse,
 // so the work above the leaves runs as GEMMs with k >= 64 (tensor cores for the
-// large ones).  Every CTA holds the triangle in shared memory in a canonical
-// form (lower, the backward kinds with reversed indices), inverts its two 32 x
-// 32 diagonal blocks (8 x 8 by substitution, then block merges) and applies
-// X1 = D1^-1 B1, X2 = D2^-1 (B2 - T21 X1) to NV right-hand vectors (columns of B
-// for left solves, rows of X for right solves) as small products.  The
-// substitution it replaces was a chain of 64 shuffles per vector: complex128
-// 64 x 64 x 2884 vectors 35 us, now about 8.  FP64 (FP32) pipe bound.
+// large ones).  complex128 (and the checked rows of both types): blocked
+// substitution with one vector per thread column (trsm_leaf_kernel); complex64:
+// a warp per vector (trsm_leaf_subst_kernel).
 template <typename C> struct LeafNB { static constexpr int value = 64; };
 constexpr int kLeafThreads = 256;
 
@@ -1905,145 +1901,6 @@ __global__ void __launch_bounds__(kLeafThreads) trsm_leaf_kernel(int m, int nvec
   }
   if constexpr (kCheck) {
     if (__syncthreads_or(bad) && tid == 0 && vflag) atomicExch(vflag, 1);
-  }
-}
-
-// acc[p][v] += sum_{r < 32} M[row0 + ty + 16 p][r0 + r] V[r0 + r][tx + 16 v] for the 2 x NV / 16 block of a thread
-template <int NVT, int MP, int VP>
-__device__ __forceinline__ void leaf_product(const double2* M, const double2* V, int row0, int r0, int ty, int tx,
-                                             double2 (&acc)[2][NVT]) {
-#pragma unroll 8
-  for (int r = 0; r < 32; ++r) {
-    double2 m[2], v[NVT];
-#pragma unroll
-    for (int p = 0; p < 2; ++p) m[p] = M[(row0 + ty + 16 * p) * MP + r0 + r];
-#pragma unroll
-    for (int q = 0; q < NVT; ++q) v[q] = V[(r0 + r) * VP + tx + 16 * q];
-#pragma unroll
-    for (int p = 0; p < 2; ++p)
-#pragma unroll
-      for (int q = 0; q < NVT; ++q) cmac(acc[p][q], m[p], v[q]);
-  }
-}
-
-template <typename C, int K, int NV>
-__global__ void __launch_bounds__(kLeafThreads) trsm_leaf_inv_kernel(int m, int nvec, RowView<C> T, RowView<C> B) {
-  constexpr int NB = LeafNB<C>::value, MP = NB + 1, VP = NV + 1, NVT = NV / 16;
-  constexpr bool kLeft = (K == kLeftLowerUnit || K == kLeftUpper);
-  constexpr bool kForward = (K == kLeftLowerUnit || K == kRightUpper);
-  constexpr bool kUnit = (K == kLeftLowerUnit || K == kRightLowerUnit);
-  extern __shared__ __align__(16) unsigned char leaf_smem[];
-  using D = double2;  // both types solve in FP64: the inverses lose nothing against substitution
-  D* M = reinterpret_cast<D*>(leaf_smem);  // [NB][MP]: the triangle, then the inverses of its diagonal blocks
-  D* V = M + NB * MP;                      // [NB][VP]: element e of vector v
-  __shared__ D rinv[NB], tmp[512];
-  const int tid = threadIdx.x;
-  const int v0 = blockIdx.x * NV;
-  const int nv = min(NV, nvec - v0);
-  // canonical lower triangle: element e of a backward kind is row m - 1 - e
-  for (int idx = tid; idx < NB * NB; idx += kLeafThreads) {
-    const int e = kLeft ? idx / NB : idx % NB, r = kLeft ? idx % NB : idx / NB;
-    D t = make_double2(e == r ? 1.0 : 0.0, 0.0);
-    if (e < m && r <= e && !(kUnit && e == r)) {
-      const int fe = kForward ? e : m - 1 - e, fr = kForward ? r : m - 1 - r;
-      const C g = kLeft ? T.at(fe, fr) : T.at(fr, fe);
-      t = make_double2(g.x, g.y);
-    }
-    M[e * MP + r] = t;
-    if (e == r) {
-      rinv[e] = kUnit ? t : crecip_newton<false>(t);
-    }
-  }
-  for (int idx = tid; idx < NB * NV; idx += kLeafThreads) {
-    const int e = kLeft ? idx / NV : idx % NB, v = kLeft ? idx % NV : idx / NB;
-    const int fe = kForward ? e : m - 1 - e;
-    const C g = (e < m && v < nv) ? (kLeft ? B.at(fe, v0 + v) : B.at(v0 + v, fe)) : czero<C>();
-    V[e * VP + v] = make_double2(g.x, g.y);
-  }
-  __syncthreads();
-  // inverses of the 8 x 8 diagonal blocks: thread 8 b + c takes column c of block b
-  D x[8];
-  if (tid < NB) {
-    const int b0 = tid & ~7, c = tid & 7;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      D s = make_double2(0.0, 0.0);
-#pragma unroll
-      for (int j = 0; j < i; ++j) cmsub(s, M[(b0 + i) * MP + b0 + j], x[j]);
-      const D ri = rinv[b0 + i];
-      x[i] = i < c ? make_double2(0.0, 0.0) : (i == c ? ri : cmul(s, ri));
-    }
-  }
-  __syncthreads();
-  if (tid < NB) {
-    const int b0 = tid & ~7, c = tid & 7;
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (i >= c) M[(b0 + i) * MP + b0 + c] = x[i];
-  }
-  __syncthreads();
-  // merges 8 -> 16 -> 32: the off-diagonal block becomes -D2^-1 T21 D1^-1
-#pragma unroll
-  for (int h = 8; h <= 16; h *= 2) {
-    const int per = h * h, total = (NB / (2 * h)) * per;
-    for (int idx = tid; idx < total; idx += kLeafThreads) {
-      const int b = (idx / per) * 2 * h, i = (idx % per) / h, j = idx % h;
-      D s = make_double2(0.0, 0.0);
-#pragma unroll
-      for (int r = 0; r < h; ++r) cmac(s, M[(b + h + i) * MP + b + r], M[(b + r) * MP + b + j]);
-      tmp[idx] = s;
-    }
-    __syncthreads();
-    for (int idx = tid; idx < total; idx += kLeafThreads) {
-      const int b = (idx / per) * 2 * h, i = (idx % per) / h, j = idx % h;
-      D s = make_double2(0.0, 0.0);
-#pragma unroll
-      for (int r = 0; r < h; ++r) cmsub(s, M[(b + h + i) * MP + b + h + r], tmp[(idx / per) * per + r * h + j]);
-      M[(b + h + i) * MP + b + j] = s;
-    }
-    __syncthreads();
-  }
-  const int tx = tid & 15, ty = tid >> 4;
-  auto put = [&](int row0, const D(&acc)[2][NVT]) {
-#pragma unroll
-    for (int p = 0; p < 2; ++p)
-#pragma unroll
-      for (int q = 0; q < NVT; ++q) V[(row0 + ty + 16 * p) * VP + tx + 16 * q] = acc[p][q];
-  };
-  D acc[2][NVT];
-  auto clear = [&]() {
-#pragma unroll
-    for (int p = 0; p < 2; ++p)
-#pragma unroll
-      for (int q = 0; q < NVT; ++q) acc[p][q] = make_double2(0.0, 0.0);
-  };
-  clear();
-  leaf_product<NVT, MP, VP>(M, V, 0, 0, ty, tx, acc);  // X1 = D1^-1 B1
-  __syncthreads();
-  put(0, acc);
-  __syncthreads();
-  if (m > 32) {
-    clear();
-    leaf_product<NVT, MP, VP>(M, V, 32, 0, ty, tx, acc);  // T21 X1
-#pragma unroll
-    for (int p = 0; p < 2; ++p)
-#pragma unroll
-      for (int q = 0; q < NVT; ++q) acc[p][q] = csub(V[(32 + ty + 16 * p) * VP + tx + 16 * q], acc[p][q]);
-    put(32, acc);  // B2 - T21 X1 (each thread rewrites the entries that it read)
-    __syncthreads();
-    clear();
-    leaf_product<NVT, MP, VP>(M, V, 32, 32, ty, tx, acc);
-    __syncthreads();
-    put(32, acc);
-    __syncthreads();
-  }
-  for (int idx = tid; idx < NB * NV; idx += kLeafThreads) {
-    const int e = kLeft ? idx / NV : idx % NB, v = kLeft ? idx % NV : idx / NB;
-    if (v >= nv || e >= m) continue;
-    const int fe = kForward ? e : m - 1 - e;
-    const D r = V[e * VP + v];
-    const C g = cmake<C>(r.x, r.y);
-    if constexpr (kLeft) B.at(fe, v0 + v) = g; else B.at(v0 + v, fe) = g;
   }
 }
 
@@ -2149,13 +2006,6 @@ static constexpr size_t leaf_smem_bytes() {
 
 template <typename C, int K, int NV, bool kCheck>
 static int trsm_leaf_launch(const LaContext& ctx, int m, int nvec, RowView<C> T, RowView<C> B) {
-  if constexpr (!kCheck) {
-    auto kern = trsm_leaf_inv_kernel<C, K, NV>;
-    BEM_CUDA_CHECK(set_kernel_attrs_once(kern, (int)leaf_smem_bytes<C, NV>(), false));
-    kern<<<ceil_div(nvec, NV), kLeafThreads, leaf_smem_bytes<C, NV>(), ctx.stream>>>(m, nvec, T, B);
-    BEM_LAUNCH_CHECK();
-    return BEM200_OK;
-  }
   auto kern = trsm_leaf_kernel<C, K, NV, kCheck>;
   BEM_CUDA_CHECK(set_kernel_attrs_once(kern, (int)leaf_smem_bytes<C, NV>(), false));
   kern<<<ceil_div(nvec, NV), kLeafThreads, leaf_smem_bytes<C, NV>(), ctx.stream>>>(m, nvec, T, B, (double)ctx.pivot_tau,
