@@ -279,7 +279,7 @@ def run_ours(args):
             "workload": "5768-face Au sphere dimer, 2 nm gap, water, Drude Au, x-pol +z, lambda = 650 + 0.05 s nm",
             "faces": cp.n,
             "precision": args.precision,
-            "engine": args.engine if args.precision == "mixed" else "simt",
+            "engine": args.engine,
             "ir_iterations": ir[0] if ir else None,
             "ir_relres": ir[1] if ir else None,
             "ir_relres_max": ir_max,

@@ -242,7 +242,8 @@ int bem200_getrf_ex(int dtype, int engine, int n, void* A, int64_t ld, int32_t* 
 /* ws of this size lets bem200_getrf run its look-ahead schedule: panels on a
  * high-priority stream, trailing updates on a low-priority one, both forked
  * from and joined back into `stream` (same pivots and factors).  A smaller
- * (or NULL) ws selects the single-stream schedule. */
+ * (or NULL) ws selects the single-stream schedule; for complex128 on engine 1
+ * it also selects the CUDA cores. */
 size_t bem200_getrf_workspace_size(int dtype, int engine, int n);
 /* B <- A^-1 B from the getrf factors (nrhs columns, row-major B).  scratch:
  * bem200_getrs_workspace_size bytes.  *status (device int) is set to
@@ -295,7 +296,8 @@ int bem200_getrs_noalloc(int dtype, int n, int nrhs, const void* LU, int64_t ld,
                          int64_t ldb, int32_t* status, void* stream);
 
 /* ------------------------------------------------------------- dense BEM
- * precision 0 = complex128 throughout (the drop-in FP64 path);
+ * precision 0 = complex128 throughout (the drop-in FP64 path; large products
+ * of the factorisation on `engine`);
  * precision 1 = mixed: complex64 factors (GEMMs on `engine`) with FP64
  * residuals and iterative refinement (bem200_bem_solve_ir).
  * precision 2 = mixed with explicit complex64 inverses G1^-1, G2^-1,
@@ -315,6 +317,10 @@ int bem200_getrs_noalloc(int dtype, int n, int nrhs, const void* LU, int64_t ld,
  * Replaces BEMRet.init (mnpbem/bem/bem_ret.py:293-525). */
 size_t bem200_bem_workspace_size(int precision, int n);
 int bem200_bem_slots(int precision, int n, void* ws, void** G1, void** G2, void** H1, void** H2);
+/* gemm_ws of bem200_bem_init: operand space of its tensor-core products
+ * (engine 1; 0 bytes otherwise).  precision 0: engine 0, or a smaller gemm_ws,
+ * computes every product in FP64 on the CUDA cores. */
+size_t bem200_bem_gemm_workspace_size(int precision, int engine, int n);
 int bem200_bem_init(int precision, int engine, int n, void* ws, int eps_per_face, const double* eps1,
                     const double* eps2, const double* nvec, double k0, void* gemm_ws, size_t gemm_ws_bytes,
                     int32_t* info_host, void* stream);

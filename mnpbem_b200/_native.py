@@ -119,6 +119,7 @@ _SIGS = {
     "bem200_hmat_matvec_items": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _vp, ctypes.c_int, _vp, _vp, _vp, _vp,
                                                 _vp, _vp, _vp, _vp, _vp, ctypes.c_int64, ctypes.c_int, _vp, _vp, _vp,
                                                 ctypes.c_int, _vp, ctypes.c_int, _vp, _vp, _vp]),
+    "bem200_bem_gemm_workspace_size": (_sz, [ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     "bem200_hmat_operator_workspace_size": (_sz, [ctypes.c_int, ctypes.c_int, _i64]),
     "bem200_hmat_operator": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _vp, ctypes.c_int, _vp, _vp, _vp, _dbl, _vp, _vp,
                                             ctypes.c_int, _vp, _vp, _vp, _vp, _vp, _i64, ctypes.c_int, _vp, _vp, _vp,

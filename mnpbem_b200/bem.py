@@ -5,7 +5,10 @@ h2`` as host numpy arrays, exactly like mnpbem/bem/bem_ret.py:1569-1831.
 Everything per wavelength runs in libbem200 on the GPU:
 
 * ``precision='fp64'`` (default): complex128 assembly, LU factors, Sigma /
-  Delta build and the Eq. (19, 20) solve -- the drop-in path;
+  Delta build and the Eq. (19, 20) solve -- the drop-in path.  The large
+  products of the factorisation run on the tcgen05 int8 tensor cores with
+  operands of 58 bits below their row or column norm; ``engine='simt'``
+  computes them in FP64 on the CUDA cores;
 * ``precision='mixed'``: complex64 factors built with tcgen05 tensor-core
   GEMMs (``engine='bf16x3'``, the name of an earlier operand split, runs
   the int8 residue products; ``'simt'`` uses CUDA cores),
@@ -102,7 +105,9 @@ class BEMRet:
             raise RuntimeError("BEMRet: a CUDA device is required (no CPU fallback)")
         self.p = p
         self.precision = precision
-        self.engine = engine if precision == "mixed" else "simt"
+        self.engine = engine
+        # the solves with complex128 factors are FP64 on the CUDA cores on any engine
+        self._solve_engine = _ENGINES[engine] if precision == "mixed" else 0
         self.ir_tol = float(ir_tol)
         self.ir_maxit = int(ir_maxit)
         self.gmres_ir = bool(gmres_ir)
@@ -156,9 +161,8 @@ class BEMRet:
         slots = [ctypes.c_void_p() for _ in range(4)]
         nat.call("bem200_bem_slots", prec, n, nat.ptr(self._ws), *[ctypes.byref(s) for s in slots])
         self._slots = [s.value for s in slots]
-        # operand space of the largest GEMM for each of the two factor chains
-        # that run beside each other
-        gbytes = int(L.bem200_gemm_workspace_size(_ENGINES[self.engine], n, n, n) * 2)
+        # operand space of the tensor-core products of the factor chains
+        gbytes = int(L.bem200_bem_gemm_workspace_size(prec, _ENGINES[self.engine], n))
         self._gws = torch.empty(max(gbytes, 1), dtype=torch.uint8, device=self.dev)
         self._gws_bytes = gbytes
         if prec == 1:
@@ -290,7 +294,7 @@ class BEMRet:
             it = ctypes.c_int32(0)
             rr = ctypes.c_double(0)
             G = self._G128
-            st = L.bem200_bem_solve_ir_ex(self._cprec, _ENGINES[self.engine], n, npol, nat.ptr(self._ws),
+            st = L.bem200_bem_solve_ir_ex(self._cprec, self._solve_engine, n, npol, nat.ptr(self._ws),
                                           nat.ptr(G[0]), nat.ptr(G[1]), nat.ptr(G[2]), nat.ptr(G[3]), nat.ptr(bt),
                                           self._eps_mode, self._e1p, self._e2p, nat.ptr(self._nvec), self.k,
                                           self.ir_tol, self.ir_maxit, nat.ptr(W1), nat.ptr(W2), nat.ptr(scratch),
@@ -325,7 +329,7 @@ class BEMRet:
                      ctypes.c_void_p(v.data_ptr() + 16 * 4 * np_), nat.ptr(b), nat.ptr(out), nat.ptr(ascr), s)
 
         def apply_M(v, out):
-            nat.call("bem200_bem_precond", self._cprec, _ENGINES[self.engine], n, npol, nat.ptr(self._ws), nat.ptr(v),
+            nat.call("bem200_bem_precond", self._cprec, self._solve_engine, n, npol, nat.ptr(self._ws), nat.ptr(v),
                      self._eps_mode, self._e1p, self._e2p, nat.ptr(self._nvec), self.k, nat.ptr(out),
                      nat.ptr(pscr), nat.ptr(self._gws), self._gws_bytes, s)
 

@@ -32,19 +32,17 @@ struct BemState {
   int* info;      // verdict of the init: 0, first zero pivot, or -BEM200_ERR_*
   int* status;
   int* verdict;   // the same of each factorisation: G1, G2, Delta, Sigma
-  void* gws;         // complex128: operand space of the tensor-core products of the init
-  size_t gws_bytes;
 };
 
 static size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
-// complex128 operand space: the two factor chains of the init run
-// concurrently and each solves two halves of its right-hand sides at a time
-template <typename C>
-static size_t state_operand_bytes(int n) {
-  if (sizeof(C) == 8) return 0;  // the caller's GEMM workspace
+// Operand space of the init's tensor-core products: two factor chains run
+// concurrently; in complex128 each solves two halves of its right-hand sides at a
+// time, in complex64 a product of any size of the chain fits.
+static size_t init_operand_bytes(int precision, int n) {
   const int half = n / 2 + 64;
-  return align256(4 * gemm_tc_workspace<C>(n, half, half, GemmEngine::kTc) + 4096);
+  if (precision == 0) return align256(4 * gemm_tc_workspace<double2>(n, half, half, GemmEngine::kTc) + 4096);
+  return 2 * gemm_tc_workspace<float2>(n, n, n, GemmEngine::kTc);
 }
 
 template <typename C>
@@ -52,7 +50,7 @@ static size_t state_bytes(int n) {
   size_t mat = align256(sizeof(C) * (size_t)n * n);
   return kSlots * mat + 8 * align256(sizeof(int32_t) * n) +
          2 * (align256(sizeof(int32_t) * 2 * (size_t)n) + kPanelGridScratch) + 6 * align256(trsv_diag_inverse_bytes<C>(n)) +
-         256 + state_operand_bytes<C>(n);
+         256;
 }
 
 template <typename C>
@@ -80,8 +78,6 @@ static BemState<C> state_view(int n, void* ws) {
   s.info = reinterpret_cast<int*>(p);
   s.status = s.info + 1;
   s.verdict = s.info + 2;
-  s.gws = p + 256;
-  s.gws_bytes = state_operand_bytes<C>(n);
   return s;
 }
 
@@ -1064,12 +1060,9 @@ int bem200_bem_init_ex(int precision, int engine, int n, void* ws, int eps_per_f
   ctx.diag_pivots = (lu_flags & BEM200_GETRF_DIAGONAL_PIVOTS) != 0;
   ctx.la_nb = lookahead_nb;
   EpsArg eps = make_eps(eps_per_face, eps1, eps2);
-  if (precision == 0) {  // complex128 products: the operand space of the workspace itself
-    const BemState<double2> s = state_view<double2>(n, ws);
-    ctx.engine = GemmEngine::kTc;
-    ctx.ws = s.gws;
-    ctx.ws_bytes = s.gws_bytes;
-  }
+  // complex128: the tensor cores only on engine 1 with their operand space
+  if (precision == 0 && !(ctx.engine == GemmEngine::kTc && ctx.ws && ctx.ws_bytes >= init_operand_bytes(0, n)))
+    ctx.engine = GemmEngine::kSimt;
   StageTimer tm;
   if (phase_ms)
     for (cudaEvent_t& e : tm.ev) BEM_CUDA_CHECK(cudaEventCreate(&e));
@@ -1104,6 +1097,10 @@ int bem200_bem_init_ex(int precision, int engine, int n, void* ws, int eps_per_f
     BEM_REQUIRE(*info_host == 0, BEM200_ERR_SINGULAR, "bem_init: exactly singular pivot at column %d", *info_host);
   }
   return BEM200_OK;
+}
+
+size_t bem200_bem_gemm_workspace_size(int precision, int engine, int n) {
+  return n > 0 && engine_from(engine) == GemmEngine::kTc ? init_operand_bytes(precision, n) : 0;
 }
 
 int bem200_bem_init(int precision, int engine, int n, void* ws, int eps_per_face, const double* eps1,

@@ -3478,11 +3478,14 @@ static size_t getrf_snap_bytes(int n) {
   return (((size_t)2 * n * sizeof(int32_t) + 255) & ~size_t(255)) + kPanelGridScratch;
 }
 
-// operand space of getrf: complex64 for any product of the factorisation,
-// complex128 for the two concurrent updates of the look-ahead schedule
+// operand space of getrf on a tensor-core engine: complex64 for any product of
+// the factorisation, complex128 for the two concurrent updates of the look-ahead
+// schedule (engine 1 only)
 static size_t getrf_operand_bytes(int dtype, int engine, int n) {
-  const size_t b = dtype == BEM200_C128 ? 2 * gemm_tc_workspace<double2>(n, n, min(n, 512), GemmEngine::kTc) + 512
-                                        : gemm_tc_workspace<float2>(n, n, n, engine_of(engine));
+  const GemmEngine e = engine_of(engine);
+  size_t b = 0;
+  if (dtype != BEM200_C128) b = gemm_tc_workspace<float2>(n, n, n, e);
+  else if (e == GemmEngine::kTc) b = 2 * gemm_tc_workspace<double2>(n, n, min(n, 512), e) + 512;
   return (b + 255) & ~size_t(255);
 }
 
@@ -3508,15 +3511,16 @@ int bem200_getrf_ex(int dtype, int engine, int n, void* A, int64_t ld, int32_t* 
   ctx.diag_pivots = (flags & BEM200_GETRF_DIAGONAL_PIVOTS) != 0;
   ctx.la_nb = lookahead_nb;
   int32_t* snap = nullptr;
-  // complex128 needs only the snapshots for the look-ahead schedule; its
-  // products go to the tensor cores when the operand space is there too
+  // complex128 needs only the snapshots for the look-ahead schedule; on engine
+  // 1 its products go to the tensor cores when the operand space is there too
   const bool z = dtype == BEM200_C128;
   const size_t sb = n > 0 ? getrf_snap_bytes(n) : 0;
   if (ws && n > 0 && ws_bytes >= (z ? sb : bem200_getrf_workspace_size(dtype, engine, n))) {
     ctx.ws_bytes = (ws_bytes - sb) & ~size_t(255);
     snap = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(ws) + ctx.ws_bytes);
   }
-  if (z) ctx.engine = snap && ctx.ws_bytes >= getrf_operand_bytes(dtype, engine, n) ? GemmEngine::kTc : GemmEngine::kSimt;
+  if (z && !(ctx.engine == GemmEngine::kTc && snap && ctx.ws_bytes >= getrf_operand_bytes(dtype, engine, n)))
+    ctx.engine = GemmEngine::kSimt;
   if (dtype == BEM200_C128) return getrf<double2>(ctx, n, (double2*)A, ld, rowmap, ipiv, snap);
   if (dtype == BEM200_C64) return getrf<float2>(ctx, n, (float2*)A, ld, rowmap, ipiv, snap);
   set_error("getrf: bad dtype %d", dtype);

@@ -424,8 +424,7 @@ def _transposed_solve(bem, w, npol, tol=1e-12, maxit=30):
 
 
 def _engine(bem):
-    from .bem import _ENGINES
-    return _ENGINES[bem.engine]
+    return bem._solve_engine
 
 
 def extinction_vertex_vjp(bem, exc, enei, weights=None):
