@@ -191,8 +191,13 @@ int bem200_green_field(int n, int npart, const int32_t* pid, const int32_t* blk0
  * calls of mnpbem/bem/bem_ret.py:437-523, dispatched through
  * mnpbem/utils/gpu.py:145-279).  dtype BEM200_C128 or BEM200_C64; engine 0 =
  * CUDA cores, 1 = large products on the tcgen05 int8 tensor cores in residue
- * arithmetic (rows of A and columns of B rounded to fixed point, 26 bits
- * (complex64) or 58 bits (complex128) below their 2-norm, then exact); 2 is
+ * arithmetic: rows of A and columns of B, balanced along the summation index
+ * by powers of two, are rounded to fixed point 26 bits (complex64) or 58 bits
+ * (complex128) below their 2-norm, the rest is exact.  The error is bounded
+ * in norms, sqrt(2 k) 2^-25 (2^-57) |a_i| |b_j| (about 2^-26, 2^-58 typically),
+ * not entry by entry: an entry far below its vector's norm keeps fewer bits
+ * than FP64 products (engine 0) would use, and an operand row or column with
+ * an infinity makes its row or column of C NaN; 2 is
  * reserved for a tcgen05 TF32 engine that is not built: a complex64 product
  * that would run on the tensor cores returns BEM200_ERR_UNSUPPORTED with it.
  * alpha, beta: HOST pointers to (re, im).

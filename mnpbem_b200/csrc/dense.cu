@@ -284,18 +284,18 @@ static int gemm_skinny(const LaContext& ctx, int m, int n, int k, C alpha, RowVi
 // Whether gemm_v runs an m x n x k product on the tensor cores (the only path
 // that uses the operand workspace ctx.ws).  That path pays three launches and
 // 2 N residue bytes written and read per entry of C whatever k is.  Measured
-// against the CUDA-core tiles: complex64 360^3 23 vs 24 us, 512^3 30 vs 44 us
+// against the CUDA-core tiles: complex64 448^3 38 vs 37 us, 512^3 37 vs 42 us
 // (from 2^26 multiply-adds), but with k = 128 only the large updates gain
 // (5768 x 5768 x 128: 451 vs 751 us; updates of 1500 rows slow a sweep on four
-// streams by 4 %); complex128 256^3 25 vs 23 us, 360^3 33 vs 38 us,
-// 5768 x 5768 x 128 1140 vs 1780 us.
+// streams by 4 %); complex128 360^3 35 vs 35 us, 408^3 44 vs
+// 60 us, 5768 x 5768 x 128 1240 vs 1780 us (from 2^26).
 template <typename C>
 static bool gemm_takes_tc(const LaContext& ctx, int m, int n, int k) {
   if (m <= 0 || n <= 0 || (n <= 16 && k >= 256)) return false;  // empty, or the skinny path
   if (ctx.engine == GemmEngine::kSimt || k < 64 || m < 64 || n < 64) return false;
   const double macs = (double)m * n * k;
   if (sizeof(C) == 16)  // without room for the operands: CUDA cores
-    return ctx.engine == GemmEngine::kTc && macs >= 33554432.0 && gemm_tc_fits<C>(ctx, m, n, k);
+    return ctx.engine == GemmEngine::kTc && macs >= 67108864.0 && gemm_tc_fits<C>(ctx, m, n, k);
   return macs >= (k >= 256 ? 67108864.0 : 1073741824.0);
 }
 

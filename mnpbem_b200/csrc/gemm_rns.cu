@@ -15,18 +15,26 @@
 // So a product takes 2 N int8 products with int32 accumulation, all exact:
 //   complex64 : N = 7,  2 alpha = 53 (26-bit operands relative to the row norm)
 //   complex128: N = 16, 2 alpha = 116 (58 bits: more than a double's 53)
-// The rounding of the operands is the only error before the final rounding:
-// |dC_ij| <= about 2^(1 - alpha) |a_i| |b_j| (complex64 2^-25, complex128
-// 2^-57), below the error of the FP32- / FP64-accumulated products it
-// replaces, and the result does not depend on any summation order.
+// The rounding of the operands is the only error before the final rounding, and
+// the result does not depend on any summation order.  The scaled norms lie in
+// [2^(alpha - 1), 2^alpha] and every real component is rounded by at most half a
+// unit, so |dC_ij| <= sqrt(2 k) 2^(1 - alpha) |a_i| |b_j| in the worst case, about
+// 2^-alpha |a_i| |b_j| for roundings of random sign.  That is a bound in norms; an
+// FMA product is bounded by sum_k |a_ik| |b_kj| instead, which is smaller where the
+// large entries of a_i meet small ones of b_j.  A scaling of the operands does not
+// blow the norms up: rows of A and columns of B have their own scales, and one
+// along the summation index, (A D)(D^-1 B), is undone by powers of two
+// (rns_balance).  Within a balanced vector, entries below 2^-4 (complex128; 2^-2
+// complex64) of its norm still keep fewer bits than the type holds.
 //
-// Launches per product: rns_split (scales and residue planes, K-major, of A
-// and B), rns_gemm (2 N int8 products, residues of the accumulators),
-// rns_merge (CRT, alpha, beta).
+// Launches per product: rns_balance (powers of two along k), rns_split (scales
+// and residue planes, K-major, of A and B), rns_gemm (2 N int8 products, residues
+// of the accumulators), rns_merge (CRT, alpha, beta).
 #include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cuda.h>
+#include <type_traits>
 
 #include "dense.cuh"
 
@@ -46,6 +54,7 @@ template <> struct Traits<float2> {
   static constexpr int kWords = 1;      // 32-bit words of an operand's base-256 digits
   static constexpr int kFrac = 2;       // 32-bit words of the CRT fractions
   static constexpr int kBlock = 6144;   // largest block of m and n per pass (workspace bound)
+  static constexpr int kExpMax = 250;   // entries are scaled by at most 2^+-kExpMax, in two factors
 };
 template <> struct Traits<double2> {
   static constexpr int N = 16;          // log2 P = 117.68
@@ -53,6 +62,7 @@ template <> struct Traits<double2> {
   static constexpr int kWords = 2;
   static constexpr int kFrac = 3;
   static constexpr int kBlock = 3072;
+  static constexpr int kExpMax = 2040;
 };
 // Largest k per pass: accumulators stay below 121^2 x 3072 < 2^25.5, where the
 // FP32 quotient of the epilogue leaves residues of at most 126 (see there).
@@ -164,22 +174,37 @@ static const Tables& tables() {
 // its row or column of the product becomes NaN.
 constexpr int kNonFinite = INT_MIN;
 
-__device__ __forceinline__ int scale_exponent(double mx, double ss, int k, int two_alpha) {
+// norm^2 = ss of the vector times 2^d per entry
+__device__ __forceinline__ int scale_exponent(double ss, int two_alpha) {
+  if (!(ss < INFINITY)) return kNonFinite;
+  return ss > 0.0 ? (two_alpha - 1 - ilogb(ss * (1.0 + 1e-12))) >> 1 : 0;  // floor; norm^2 < 2^(ilogb + 1)
+}
+// complex64: squares and their sums stay in the range of doubles
+__device__ __forceinline__ void norm_add(float2 v, int d, double& ss) {
+  const double x = v.x, y = v.y;
+  ss = fma(fma(x, x, y * y), __hiloint2double((2 * d + 1023) << 20, 0), ss);  // a NaN entry stays in ss
+}
+__device__ __forceinline__ void norm_add(double2 v, int d, double& ss) {
+  const double f = __hiloint2double((d + 1023) << 20, 0), x = v.x * f, y = v.y * f;
+  ss = fma(x, x, fma(y, y, ss));
+}
+// complex128 squares out of range (or a vector of zeros): the norm taken again, kLowShift powers of two
+// lower if the sum overflowed; where squares vanish, norm^2 <= 2 k max^2
+constexpr int kLowShift = 600;
+__device__ __forceinline__ bool norm_unsafe(float2*, double) { return false; }
+__device__ __forceinline__ bool norm_unsafe(double2*, double ss) { return !(ss > 1e-270 && ss < 1e290); }
+template <typename C>
+__device__ __forceinline__ void norm_add_wide(C v, int d, bool low, double& mx, double& ss) {
+  const double g = low ? __hiloint2double((1023 - kLowShift) << 20, 0) : 1.0, f = __hiloint2double((d + 1023) << 20, 0);
+  const double x = fabs((double)v.x) * g * f, y = fabs((double)v.y) * g * f;
+  mx = fmax(mx, fmax(x, y));
+  ss = fma(x, x, fma(y, y, ss));
+}
+__device__ __forceinline__ int scale_exponent_wide(double mx, double ss, int k, bool low, int two_alpha) {
   if (!(ss >= 0.0) || !(mx < INFINITY)) return kNonFinite;
   if (!(mx > 0.0)) return 0;
-  int e2;  // norm^2 < 2^(e2 + 1)
-  if (mx > 1e-140 && mx < 1e140)
-    e2 = ilogb(ss * (1.0 + 1e-12));
-  else  // squares out of range: norm^2 <= 2 k max^2
-    e2 = 2 * (ilogb(mx) + 1) + ilogb((double)(2 * k));
-  return (two_alpha - 1 - e2) >> 1;  // floor
-}
-
-template <typename C>
-__device__ __forceinline__ void norm_add(C v, double& mx, double& ss) {
-  const double x = fabs((double)v.x), y = fabs((double)v.y);
-  mx = fmax(mx, fmax(x, y));
-  ss = fma(x, x, fma(y, y, ss));  // a NaN entry stays in ss
+  const int e2 = mx > 1e-140 && mx < 1e140 ? ilogb(ss * (1.0 + 1e-12)) : 2 * (ilogb(mx) + 1) + ilogb((double)(2 * k));
+  return ((two_alpha - 1 - e2) >> 1) - (low ? kLowShift : 0);
 }
 
 // ------------------------------------------------------------------ residue planes
@@ -197,6 +222,98 @@ __device__ __forceinline__ void digits(double x, int e, int32_t (&d)[2]) {
   const long long v = (__double2ll_rn(s) + 0x0080808080808080LL) ^ 0x0080808080808080LL;
   d[0] = (int32_t)v;
   d[1] = (int32_t)(v >> 32);
+}
+
+// ------------------------------------------------------------------ balance
+// (A D)(D^-1 B) = A B for any diagonal D, but with D far from constant the large
+// columns of A meet small rows of B, and scales taken from the norms leave few
+// bits for the entries that make up the product.  So column k of A is multiplied
+// by 2^d[k] and row k of B by 2^-d[k], d[k] half the difference of their mean
+// exponents over 32 rows of A and 32 columns of B (evenly spaced over all of
+// them; zeros and non-finite entries do not count).  A diagonal scaling of
+// either operand shows in every row and column and shifts these means exactly;
+// the means are little moved by the peaks of single entries, so that operands
+// without a grading stay as they are to within a bit.  A k without an entry in
+// the sample takes the mean over 32 other k.  One CTA per 32 k; 3 to 4 us, latency
+// bound.  (Exact column and row maxima recorded by the split, and a second split
+// where they differ, cost 9 - 25 % of a solve: the maxima of BEM blocks differ by
+// 5 to 10 bits along k through single entries.)
+constexpr int kSample = 32;
+
+// exponent of the larger component; false for zeros and non-finite entries
+__device__ __forceinline__ bool entry_exponent(float2 v, int& e) {
+  const int b = max(__float_as_int(v.x) & INT_MAX, __float_as_int(v.y) & INT_MAX);
+  e = b >> 23;
+  if (e == 0) e = 9 - __clz(b);  // subnormal
+  e -= 127;
+  return b != 0 && b < 0x7f800000;
+}
+__device__ __forceinline__ bool entry_exponent(double2 v, int& e) {
+  const double m = fmax(fabs(v.x), fabs(v.y));
+  const bool ok = m > 0.0 && m < INFINITY && v.x == v.x && v.y == v.y;
+  e = ok ? ilogb(m) : 0;
+  return ok;
+}
+
+template <typename C>
+__global__ void __launch_bounds__(256) rns_balance_kernel(int m, int n, int k, RowView<C> A, RowView<C> B,
+                                                          int* __restrict__ d) {
+  __shared__ int as[8][32], ac[8][32], bs[32], bc[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, k0 = 32 * blockIdx.x;
+  const int na = min(kSample, m), nb = min(kSample, n);
+  // mean exponents of 32 columns of A (k from col(0..31), along the lanes) and of the same rows of B, into
+  // warp 0's lanes; false where either has no entry
+  auto difference = [&](auto col, float& v) -> bool {
+    int sum = 0, cnt = 0;
+    C va[4], vb[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int r = 4 * wid + j, ca = col(lane), cb = col(r);
+      va[j] = r < na && ca < k ? A.at((int)((2LL * r + 1) * m / (2 * na)), ca) : czero<C>();
+      vb[j] = lane < nb && cb < k ? B.at(cb, (int)((2LL * lane + 1) * n / (2 * nb))) : czero<C>();
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      int e;
+      if (entry_exponent(va[j], e)) {
+        sum += e;
+        ++cnt;
+      }
+      const bool ok = entry_exponent(vb[j], e);
+      const int s = __reduce_add_sync(0xffffffffu, ok ? e : 0), c = __popc(__ballot_sync(0xffffffffu, ok));
+      if (lane == 0) {
+        bs[4 * wid + j] = s;
+        bc[4 * wid + j] = c;
+      }
+    }
+    as[wid][lane] = sum;
+    ac[wid][lane] = cnt;
+    __syncthreads();
+    bool ok = false;
+    if (wid == 0) {
+      for (int w = 1; w < 8; ++w) {
+        sum += as[w][lane];
+        cnt += ac[w][lane];
+      }
+      ok = cnt > 0 && bc[lane] > 0;
+      v = ok ? 0.5f * ((float)bs[lane] / bc[lane] - (float)sum / cnt) : 0.f;
+    }
+    __syncthreads();
+    return ok;
+  };
+  float v = 0.f;
+  const bool ok = difference([&](int i) { return k0 + i; }, v);
+  if (__syncthreads_or(wid == 0 && !ok && k0 + lane < k)) {
+    float t = 0.f;
+    const bool any = difference([&](int i) { return (int)((2LL * i + 1) * k / 64); }, t);
+    if (wid == 0) {
+      const int c = __popc(__ballot_sync(0xffffffffu, any));
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (!ok) v = c ? t / c : 0.f;
+    }
+  }
+  constexpr int lim = sizeof(C) == 8 ? 300 : 1020;  // 2^(2 d) and 2^d are normal doubles
+  if (wid == 0 && k0 + lane < k) d[k0 + lane] = max(-lim, min(lim, __float2int_rn(v)));
 }
 
 __device__ __forceinline__ uint32_t pack4(const uint32_t (&b)[4]) {
@@ -257,11 +374,19 @@ __device__ __forceinline__ void emit(const int4 (&re)[Traits<C>::kWords], const 
 // A's zeros).  Instruction issue (64 % of the slots) and latency at half
 // occupancy bound it: 13 (complex64) / 15 (complex128) instructions per entry
 // and modulus; 2884^3 complex64 operands take 120 us with the moduli unrolled,
-// 133 with a loop over them.  Norms summed in FP32 do not help.
+// 133 with a loop over them.  Norms summed in FP32 do not help.  Entries take the
+// powers of two of rns_balance on top of their vector's scale (2884^3 products:
+// complex64 449 us, 447 without them; complex128 1072 and 1064).
+// exponent of the scale of one entry: 2^e of its vector times 2^d; clamped where the scaled entry is
+// 0 or rounds to 0 anyway
+template <typename C>
+__device__ __forceinline__ int entry_scale(int e, int d) {
+  return e == kNonFinite ? 0 : max(-Traits<C>::kExpMax, min(Traits<C>::kExpMax, e + d));
+}
 constexpr int kRowChunks = kBlockK / 128 / 8;  // chunks per warp of the longest row
 template <typename C>
-__global__ void __launch_bounds__(256) rns_split_kernel(int m, int n, int k, RowView<C> A, RowView<C> B, int Mp, int Np,
-                                                        int Kp, int ablocks, int wpr, int* __restrict__ sa,
+__global__ void __launch_bounds__(256, sizeof(C) == 16 ? 3 : 4) rns_split_kernel(int m, int n, int k, RowView<C> A, RowView<C> B, int Mp, int Np,
+                                                        int Kp, int ablocks, int wpr, const int* __restrict__ pw, int* __restrict__ sa,
                                                         int* __restrict__ sb, uint8_t* __restrict__ pa,
                                                         uint8_t* __restrict__ pb,
                                                         const __grid_constant__ SplitTab tab) {
@@ -273,50 +398,71 @@ __global__ void __launch_bounds__(256) rns_split_kernel(int m, int n, int k, Row
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int4 re[W], im[W];
   if ((int)blockIdx.x < ablocks) {
-    const int chunks = Kp / 128, part = wid % wpr;
+    const int chunks = Kp / 128, share = wid % wpr;
     const int i = blockIdx.x * (8 / wpr) + wid / wpr;
     C v[kRowChunks][4];
+    int d[kRowChunks][4];
     double mx = 0.0, ss = 0.0;
+    // sum over the lanes and the row's warps
+    auto row_sum = [&](int buf) {
+      for (int o = 16; o > 0; o >>= 1) {
+        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      }
+      if (lane == 0) {
+        rmx[buf][wid] = mx;
+        rss[buf][wid] = ss;
+      }
+      __syncthreads();
+      mx = ss = 0.0;
+      for (int w = 0; w < wpr; ++w) {
+        mx = fmax(mx, rmx[buf][wid - share + w]);
+        ss += rss[buf][wid - share + w];
+      }
+    };
     if (i < m) {
       const C* row = &A.at(i, 0);
 #pragma unroll
       for (int g = 0; g < kRowChunks; ++g)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int c = (part + g * wpr) * 128 + lane + 32 * j;
+          const int c = (share + g * wpr) * 128 + lane + 32 * j;
           v[g][j] = c < k ? row[c] : czero<C>();
+          d[g][j] = c < k ? pw[c] : 0;
         }
 #pragma unroll
       for (int g = 0; g < kRowChunks; ++g)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) norm_add(v[g][j], mx, ss);
-      for (int o = 16; o > 0; o >>= 1) {
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        for (int j = 0; j < 4; ++j) norm_add(v[g][j], d[g][j], ss);
+    }
+    row_sum(0);
+    int e = scale_exponent(ss, T::kTwoAlpha);
+    if constexpr (sizeof(C) == 16) {
+      const bool redo = i < m && norm_unsafe((C*)nullptr, ss), low = ss >= 1e290;
+      if (__syncthreads_or(redo)) {
+        mx = ss = 0.0;
+        if (redo) {
+#pragma unroll
+          for (int g = 0; g < kRowChunks; ++g)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) norm_add_wide(v[g][j], d[g][j], low, mx, ss);
+        }
+        row_sum(1);
+        if (redo) e = scale_exponent_wide(mx, ss, k, low, T::kTwoAlpha);
       }
     }
-    if (lane == 0) {
-      rmx[0][wid] = mx;
-      rss[0][wid] = ss;
-    }
-    __syncthreads();
     if (i >= m) return;
-    mx = ss = 0.0;
-    for (int w = 0; w < wpr; ++w) {
-      mx = fmax(mx, rmx[0][wid - part + w]);
-      ss += rss[0][wid - part + w];
-    }
-    const int e = scale_exponent(mx, ss, k, T::kTwoAlpha);
-    if (part == 0 && lane == 0) sa[i] = e;
+    if (share == 0 && lane == 0) sa[i] = e;
 #pragma unroll
     for (int g = 0; g < kRowChunks; ++g) {
-      const int ch = part + g * wpr;
+      const int ch = share + g * wpr;
       if (ch >= chunks) break;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         int32_t dr[W], di[W];
-        digits(v[g][j].x, e == kNonFinite ? 0 : e, dr);
-        digits(v[g][j].y, e == kNonFinite ? 0 : e, di);
+        const int t = entry_scale<C>(e, d[g][j]);
+        digits(v[g][j].x, t, dr);
+        digits(v[g][j].y, t, di);
 #pragma unroll
         for (int l = 0; l < W; ++l) {
           sh[wid][l][lane + 32 * j] = e == kNonFinite ? 0 : dr[l];
@@ -338,39 +484,56 @@ __global__ void __launch_bounds__(256) rns_split_kernel(int m, int n, int k, Row
   const int c = threadIdx.x & 7, rg = threadIdx.x >> 3, q = q0 + c;  // column, row group (0..31)
   {
     double mx = 0.0, ss = 0.0;
-    if (q < n) {
-#pragma unroll 8
-      for (int p = rg; p < k; p += 32) norm_add(B.at(p, q), mx, ss);
-    }
-    for (int o = 16; o >= 8; o >>= 1) {
-      mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    }
-    if (lane < 8) {
-      rmx[wid][lane] = mx;
-      rss[wid][lane] = ss;
-    }
-    __syncthreads();
-    if (threadIdx.x < 8) {
+    // sum over the row groups, to threads 0 .. 7
+    auto column_sum = [&]() {
+      for (int o = 16; o >= 8; o >>= 1) {
+        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      }
+      if (lane < 8) {
+        rmx[wid][lane] = mx;
+        rss[wid][lane] = ss;
+      }
+      __syncthreads();
       mx = ss = 0.0;
       for (int w = 0; w < 8; ++w) {
-        mx = fmax(mx, rmx[w][threadIdx.x]);
-        ss += rss[w][threadIdx.x];
+        mx = fmax(mx, rmx[w][c]);
+        ss += rss[w][c];
       }
-      const int e = scale_exponent(mx, ss, k, T::kTwoAlpha);
-      esh[threadIdx.x] = e;
-      if (q0 + (int)threadIdx.x < n) sb[q0 + threadIdx.x] = e;
+      __syncthreads();
+    };
+    if (q < n) {
+#pragma unroll 8
+      for (int p = rg; p < k; p += 32) norm_add(B.at(p, q), -pw[p], ss);
+    }
+    column_sum();
+    int e = scale_exponent(ss, T::kTwoAlpha);
+    if constexpr (sizeof(C) == 16) {
+      const bool redo = q < n && norm_unsafe((C*)nullptr, ss), low = ss >= 1e290;
+      if (__syncthreads_or(redo)) {
+        mx = ss = 0.0;
+        if (redo)
+          for (int p = rg; p < k; p += 32) norm_add_wide(B.at(p, q), -pw[p], low, mx, ss);
+        column_sum();
+        if (redo) e = scale_exponent_wide(mx, ss, k, low, T::kTwoAlpha);
+      }
+    }
+    if (threadIdx.x < 8) {
+      esh[c] = e;
+      if (q < n) sb[q] = e;
     }
     __syncthreads();
   }
   const int e = esh[c];
   const size_t plane = (size_t)Np * Kp;
   C v[4];
+  int d[4];
   auto fetch = [&](int p0) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int p = p0 + 4 * rg + j;
       v[j] = (p < k && q < n) ? B.at(p, q) : czero<C>();
+      d[j] = p < k ? -pw[p] : 0;
     }
   };
   fetch(0);
@@ -379,8 +542,9 @@ __global__ void __launch_bounds__(256) rns_split_kernel(int m, int n, int k, Row
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       int32_t r[W], s[W];
-      digits(v[j].x, e == kNonFinite ? 0 : e, r);
-      digits(v[j].y, e == kNonFinite ? 0 : e, s);
+      const int t = entry_scale<C>(e, d[j]);
+      digits(v[j].x, t, r);
+      digits(v[j].y, t, s);
 #pragma unroll
       for (int l = 0; l < W; ++l) {
         (&dr[l].x)[j] = e == kNonFinite ? 0 : r[l];
@@ -793,6 +957,9 @@ static int make_map(CUtensorMap* m, void* ptr, long long rows, int cols, int box
 
 static size_t up256(size_t b) { return (b + 255) & ~size_t(255); }
 
+constexpr size_t kBalanceBytes = sizeof(int) * kBlockK;
+static_assert(kBalanceBytes % 256 == 0, "workspace layout");
+
 struct Plan {
   int Mp, Np, Kp;
   size_t a, b, c, sa, sb, total;
@@ -810,7 +977,7 @@ static Plan plan(int m, int n, int k) {
   p.c = up256(planes * m * (size_t)p.Np);
   p.sa = up256(sizeof(int) * (size_t)m);
   p.sb = up256(sizeof(int) * (size_t)n);
-  p.total = p.a + p.b + p.c + p.sa + p.sb + 256;
+  p.total = kBalanceBytes + p.a + p.b + p.c + p.sa + p.sb + 256;
   return p;
 }
 
@@ -878,22 +1045,24 @@ int gemm_tc(const LaContext& ctx, int m, int n, int k, C alpha, RowView<C> A, Ro
       for (int n0 = 0; n0 < n; n0 += nb) {
         const int mm = std::min(mb, m - m0), nn = std::min(nb, n - n0), kk = std::min(kb, k - k0);
         const Plan p = plan<C>(mm, nn, kk);
-        // A's scales and planes come first: they stay for the other blocks of n
-        int* sa = reinterpret_cast<int*>(w);
-        uint8_t* pa = reinterpret_cast<uint8_t*>(w) + p.sa;
+        // the powers of two stay for all blocks of this k, A's scales and planes for the other blocks of n
+        int* pw = reinterpret_cast<int*>(w);
+        int* sa = reinterpret_cast<int*>(w + kBalanceBytes);
+        uint8_t* pa = reinterpret_cast<uint8_t*>(w) + kBalanceBytes + p.sa;
         uint8_t* pb = pa + p.a;
         uint8_t* pc = pb + p.b;
         int* sb = reinterpret_cast<int*>(pc + p.c);
-        int* status = ctx.dstatus;
-        if (!status) {
-          status = reinterpret_cast<int*>(pc + p.c + p.sb);
-          BEM_CUDA_CHECK(cudaMemsetAsync(status, 0, sizeof(int), ctx.stream));
-        }
+        // without a status of the caller's, a place that is written on a timeout and never read
+        int* status = ctx.dstatus ? ctx.dstatus : reinterpret_cast<int*>(pc + p.c + p.sb);
         const RowView<C> Ab = A.sub(m0, k0), Bb = B.sub(k0, n0), Cb = Cv.sub(m0, n0);
         const int chunks = p.Kp / 128, wpr = chunks >= 8 ? 8 : (chunks >= 4 ? 4 : (chunks >= 2 ? 2 : 1));
         const int ablocks = n0 == 0 ? ceil_div(mm, 8 / wpr) : 0;
+        if (m0 == 0 && n0 == 0) {
+          rns_balance_kernel<C><<<ceil_div(kk, 32), 256, 0, ctx.stream>>>(m, n, kk, A.sub(0, k0), B.sub(k0, 0), pw);
+          BEM_LAUNCH_CHECK();
+        }
         rns_split_kernel<C><<<ablocks + ceil_div(nn, 8), 256, 0, ctx.stream>>>(
-            mm, nn, kk, Ab, Bb, p.Mp, p.Np, p.Kp, ablocks, wpr, sa, sb, pa, pb, tab.split);
+            mm, nn, kk, Ab, Bb, p.Mp, p.Np, p.Kp, ablocks, wpr, pw, sa, sb, pa, pb, tab.split);
         BEM_LAUNCH_CHECK();
         CUtensorMap ma, mbm;
         int st;
