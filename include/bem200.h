@@ -201,7 +201,9 @@ int bem200_green_field(int n, int npart, const int32_t* pid, const int32_t* blk0
  * reserved for a tcgen05 TF32 engine that is not built: a complex64 product
  * that would run on the tensor cores returns BEM200_ERR_UNSUPPORTED with it.
  * alpha, beta: HOST pointers to (re, im).
- * ws/ws_bytes: scratch for the tensor-core engine, may be NULL/0 for engine 0.
+ * ws/ws_bytes: scratch for the tensor-core engine (any address), may be NULL/0
+ * for engine 0.  complex64 on engine 1 needs it from 128 rows, 64 columns, k = 64
+ * and 2^26 multiply-adds (engine 2 refuses these products).
  * bem200_gemm_workspace_size: complex64 in one pass (complex128 takes 2.3 times
  * that); a smaller ws is used in smaller blocks, and a complex128 product that
  * no block fits runs on the CUDA cores. */

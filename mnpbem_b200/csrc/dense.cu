@@ -289,13 +289,20 @@ static int gemm_skinny(const LaContext& ctx, int m, int n, int k, C alpha, RowVi
 // (5768 x 5768 x 128: 451 vs 751 us; updates of 1500 rows slow a sweep on four
 // streams by 4 %); complex128 360^3 35 vs 35 us, 408^3 44 vs
 // 60 us, 5768 x 5768 x 128 1240 vs 1780 us (from 2^26).
+// What a call is owed whatever the thresholds: complex64 products of at least
+// 128 rows, 64 columns, k = 64 and 2^26 multiply-adds need the tensor-core engine's
+// workspace (engine 1) or that engine (2) and are refused without; smaller
+// ones, and all complex128 ones, run on the CUDA cores then.
 template <typename C>
 static bool gemm_takes_tc(const LaContext& ctx, int m, int n, int k) {
   if (m <= 0 || n <= 0 || (n <= 16 && k >= 256)) return false;  // empty, or the skinny path
   if (ctx.engine == GemmEngine::kSimt || k < 64 || m < 64 || n < 64) return false;
   const double macs = (double)m * n * k;
-  if (sizeof(C) == 16)  // without room for the operands: CUDA cores
-    return ctx.engine == GemmEngine::kTc && macs >= 67108864.0 && gemm_tc_fits<C>(ctx, m, n, k);
+  if (sizeof(C) == 16) return ctx.engine == GemmEngine::kTc && macs >= 67108864.0 && gemm_tc_fits<C>(ctx, m, n, k);
+  const bool demands = m >= 128 && macs >= 67108864.0;
+  if (ctx.engine != GemmEngine::kTc) return demands;
+  if (!demands && (k < 256 || macs < 67108864.0)) return false;
+  if (!gemm_tc_fits<C>(ctx, m, n, k)) return demands;
   return macs >= (k >= 256 ? 67108864.0 : 1073741824.0);
 }
 

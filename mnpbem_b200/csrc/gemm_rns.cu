@@ -1015,16 +1015,27 @@ size_t gemm_tc_workspace(int m, int n, int k, GemmEngine e) {
   return rns::plan<C>(mb, nb, kb).total;
 }
 
+// the caller's workspace from its first 256-byte boundary on
+static char* operand_space(const LaContext& ctx, size_t& bytes) {
+  const uintptr_t p = reinterpret_cast<uintptr_t>(ctx.ws), a = (p + 255) & ~uintptr_t(255);
+  bytes = ctx.ws && ctx.ws_bytes > a - p ? ctx.ws_bytes - (a - p) : 0;
+  return reinterpret_cast<char*>(a);
+}
+
 template <typename C>
 bool gemm_tc_fits(const LaContext& ctx, int m, int n, int k) {
   int mb, nb, kb;
-  return ctx.ws && rns::fit_blocks<C>(m, n, k, ctx.ws_bytes, mb, nb, kb);
+  size_t bytes;
+  operand_space(ctx, bytes);
+  return rns::fit_blocks<C>(m, n, k, bytes, mb, nb, kb);
 }
 
 template <typename C>
 bool gemm_tc_in_place(const LaContext& ctx, int m, int n, int k) {
   int mb, nb, kb;
-  return ctx.ws && rns::fit_blocks<C>(m, n, k, ctx.ws_bytes, mb, nb, kb) && mb == m && kb == k;
+  size_t bytes;
+  operand_space(ctx, bytes);
+  return rns::fit_blocks<C>(m, n, k, bytes, mb, nb, kb) && mb == m && kb == k;
 }
 
 template <typename C>
@@ -1034,12 +1045,13 @@ int gemm_tc(const LaContext& ctx, int m, int n, int k, C alpha, RowView<C> A, Ro
   using T = Traits<C>;
   BEM_REQUIRE(ctx.engine == GemmEngine::kTc, BEM200_ERR_UNSUPPORTED, "gemm: the TF32 tensor-core engine is not built");
   int mb, nb, kb;
-  BEM_REQUIRE(ctx.ws && fit_blocks<C>(m, n, k, ctx.ws_bytes, mb, nb, kb), BEM200_ERR_ARG,
+  size_t bytes;
+  char* w = operand_space(ctx, bytes);
+  BEM_REQUIRE(fit_blocks<C>(m, n, k, bytes, mb, nb, kb), BEM200_ERR_ARG,
               "gemm: workspace of %zu bytes needed for %d x %d x %d (have %zu)", plan<C>(m, n, k).total, m, n, k,
               ctx.ws_bytes);
   const Tables& tab = tables<C>();
   BEM_CUDA_CHECK(set_kernel_attrs_once(rns_gemm_kernel, SMEM_BYTES, false));
-  char* w = reinterpret_cast<char*>(ctx.ws);
   for (int k0 = 0; k0 < k; k0 += kb)
     for (int m0 = 0; m0 < m; m0 += mb)
       for (int n0 = 0; n0 < n; n0 += nb) {
