@@ -19,7 +19,8 @@ Everything per wavelength runs in libbem200 on the GPU:
   or diverging sweep is the condition estimate that the factors are not good
   enough) continues as GMRES-IR: restarted GMRES on the FP64 operator,
   right-preconditioned by the same complex64 factors (``gmres_ir=True``).
-  A solve that still misses ``ir_tol`` raises ``RuntimeError``.
+  A solve that still misses ``ir_tol`` is repeated with LU factors if the
+  factors were explicit inverses, and raises ``RuntimeError`` otherwise.
 
 There is no CPU fallback: without a GPU or the library, construction raises.
 """
@@ -193,10 +194,8 @@ class BEMRet:
         if self.enei is not None and np.isclose(self.enei, enei):
             return self
         self._alloc()
-        n = self.n
         self.k = 2 * np.pi / enei
         self._eps(enei)
-        s = nat.stream_ptr()
         if self._prec == 1:
             self.g.bem_matrices(enei, dtype="c128", out=self._G128)
         if self.pivoting == "partial":
@@ -205,6 +204,17 @@ class BEMRet:
             modes = ["inverse", "diagonal", "partial"]
         else:
             modes = ["diagonal", "partial"]
+        self._factor(enei, modes)
+        if self._phase_buf is not None:
+            self.last_init_phases_ms = list(self._phase_buf)
+        self.enei = enei
+        return self
+
+    def _factor(self, enei, modes):
+        """The factors by the first of ``modes`` whose checks pass, from the Green
+        matrices (mixed: the assembled ones)."""
+        n = self.n
+        s = nat.stream_ptr()
         for mode in modes:
             cprec = 2 if mode == "inverse" else self._prec
             if self._prec == 0:
@@ -225,10 +235,15 @@ class BEMRet:
             self.last_pivoting = "partial" if info.value == -nat.ERR_PIVOTING else mode
             self._cprec = cprec
             break
-        if self._phase_buf is not None:
-            self.last_init_phases_ms = list(self._phase_buf)
-        self.enei = enei
-        return self
+
+    def refactor(self):
+        """LU factors in place of the explicit inverses of the current wavelength
+        (whose probe is coarse: solves that miss their tolerance with them call
+        this and try again).  False when the factors are no inverses."""
+        if self._cprec != 2:
+            return False
+        self._factor(self.enei, ["diagonal", "partial"])
+        return True
 
     def _lookahead(self):
         """Look-ahead block width of the LU factorisations (0: the library's
@@ -300,10 +315,15 @@ class BEMRet:
                                           self.ir_tol, self.ir_maxit, nat.ptr(W1), nat.ptr(W2), nat.ptr(scratch),
                                           nat.ptr(self._gws), self._gws_bytes, ctypes.byref(it), ctypes.byref(rr), s)
             self.last_ir = (int(it.value), float(rr.value), "ir")
-            if st == nat.ERR_NOCONV and self.gmres_ir:
-                W1, W2 = self._gmres_refine(bt, npol, W1, W2, int(it.value))
-            else:
-                nat.check(st, "bem200_bem_solve_ir")
+            try:
+                if st == nat.ERR_NOCONV and self.gmres_ir:
+                    W1, W2 = self._gmres_refine(bt, npol, W1, W2, int(it.value))
+                else:
+                    nat.check(st, "bem200_bem_solve_ir")
+            except RuntimeError:
+                if st == nat.ERR_NOCONV and self.refactor():
+                    return self.solve_device(bt, npol)
+                raise
         return W1, W2
 
     def _gmres_refine(self, bt, npol, W1, W2, sweeps):

@@ -392,7 +392,8 @@ def _planewave_terms(cp, exc, enei, pos, nvec, area):
 def _transposed_solve(bem, w, npol, tol=1e-12, maxit=30):
     """lambda = A^-T w for the current wavelength's factors: one transposed
     solve with the complex128 factors (fp64), or refinement of the complex64
-    transposed solve against the FP64 transposed operator (mixed)."""
+    transposed solve against the FP64 transposed operator (mixed), with LU
+    factors where the explicit inverses are not good enough."""
     import torch
     L = nat.lib()
     n = bem.n
@@ -420,6 +421,8 @@ def _transposed_solve(bem, w, npol, tol=1e-12, maxit=30):
             return lam, it
         sT(r, d)
         lam += d
+    if bem.refactor():
+        return _transposed_solve(bem, w, npol, tol, maxit)
     raise RuntimeError("transposed solve: refinement left the residual at {:.3e} (tol {:.1e})".format(rn / wn, tol))
 
 
