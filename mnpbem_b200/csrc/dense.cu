@@ -13,11 +13,13 @@
 //     tensor cores for large ones (gemm_rns.cu).
 // Pivot choice follows LAPACK izamax: largest |re| + |im|.
 #include <cooperative_groups.h>
+#include <cuda.h>
 
 #include <climits>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "dense.cuh"
@@ -29,40 +31,74 @@ namespace bem200 {
 // ------------------------------------------------------------- stream pool
 namespace {
 struct PooledBundle {
-  int dev, kind;
-  cudaStream_t stream;
-  cudaEvent_t ev[3];
+  unsigned long long ctx = 0;  // 0: an empty place
+  int kind = 0;
+  cudaStream_t main = nullptr, stream = nullptr;
+  cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+  unsigned long long returned = 0;
 };
-constexpr int kPoolCap = 32;  // idle bundles kept per device and kind
+constexpr int kPoolCap = 32;     // idle bundles kept per context and kind
+constexpr int kPoolFresh = 4;     // a stream without a bundle of its own takes another's from here on
+constexpr int kPoolPlaces = 256;
 std::mutex g_pool_mu;
-// never destroyed: streams must not be released after the runtime has shut down
-std::vector<PooledBundle>& pool() {
-  static auto* p = new std::vector<PooledBundle>;
-  return *p;
+// plain storage: nothing to allocate, nothing released after the runtime has shut down
+PooledBundle g_pool[kPoolPlaces];
+unsigned long long g_pool_tick = 0;
+
+// Unique number of the calling thread's context, 0 if it cannot be told.  (A
+// device's handles die with cudaDeviceReset, and each context has its own.)
+unsigned long long context_id() {
+  using GetCurrent = CUresult (*)(CUcontext*);
+  using GetId = CUresult (*)(CUcontext, unsigned long long*);
+  static const auto fns = [] {
+    std::pair<GetCurrent, GetId> f{nullptr, nullptr};
+    void *a = nullptr, *b = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &a, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess && cudaGetDriverEntryPoint("cuCtxGetId", &b, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      f = {reinterpret_cast<GetCurrent>(a), reinterpret_cast<GetId>(b)};
+    else
+      (void)cudaGetLastError();
+    return f;
+  }();
+  CUcontext c = nullptr;
+  unsigned long long id = 0;
+  if (!fns.first || fns.first(&c) != CUDA_SUCCESS || !c || fns.second(c, &id) != CUDA_SUCCESS) return 0;
+  return id + 1;
 }
 }  // namespace
 
 cudaError_t StreamLease::acquire(cudaStream_t main, Kind kind) {
-  cudaError_t e = cudaGetDevice(&dev_);
-  if (e != cudaSuccess) return e;
   kind_ = kind;
+  main_ = main;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(main, &cs) != cudaSuccess) {
     (void)cudaGetLastError();
     cs = cudaStreamCaptureStatusActive;
   }
-  pooled_ = cs == cudaStreamCaptureStatusNone;
-  if (pooled_) {
+  ctx_ = cs == cudaStreamCaptureStatusNone ? context_id() : 0;
+  if (ctx_) {
     std::lock_guard<std::mutex> lock(g_pool_mu);
-    std::vector<PooledBundle>& v = pool();
-    for (size_t i = v.size(); i-- > 0;)
-      if (v[i].dev == dev_ && v[i].kind == kind) {
-        stream = v[i].stream;
-        for (int k = 0; k < 3; ++k) ev[k] = v[i].ev[k];
-        v.erase(v.begin() + i);
-        return cudaSuccess;
-      }
+    // the bundle that last served `main`: its work is joined into `main` already.  Else, when
+    // there are enough idle ones, the one that was returned first.
+    PooledBundle *own = nullptr, *oldest = nullptr;
+    int idle = 0;
+    for (PooledBundle& b : g_pool) {
+      if (b.ctx != ctx_ || b.kind != kind) continue;
+      ++idle;
+      if (b.main == main && (!own || b.returned > own->returned)) own = &b;
+      if (!oldest || b.returned < oldest->returned) oldest = &b;
+    }
+    PooledBundle* b = own ? own : (idle >= kPoolFresh ? oldest : nullptr);
+    if (b) {
+      stream = b->stream;
+      for (int k = 0; k < 3; ++k) ev[k] = b->ev[k];
+      *b = PooledBundle{};
+      return cudaSuccess;
+    }
   }
+  cudaError_t e;
   int prio = 0, lo = 0, hi = 0;
   if (kind != kNormal) {
     if ((e = cudaDeviceGetStreamPriorityRange(&lo, &hi)) != cudaSuccess) return e;
@@ -76,13 +112,16 @@ cudaError_t StreamLease::acquire(cudaStream_t main, Kind kind) {
 
 void StreamLease::release() {
   if (!stream) return;
-  if (pooled_ && ev[2]) {
+  if (ctx_ && ev[2]) {
     std::lock_guard<std::mutex> lock(g_pool_mu);
-    std::vector<PooledBundle>& v = pool();
+    PooledBundle* place = nullptr;
     int idle = 0;
-    for (const PooledBundle& b : v) idle += b.dev == dev_ && b.kind == kind_;
-    if (idle < kPoolCap) {
-      v.push_back(PooledBundle{dev_, kind_, stream, {ev[0], ev[1], ev[2]}});
+    for (PooledBundle& b : g_pool) {
+      idle += b.ctx == ctx_ && b.kind == kind_;
+      if (!b.ctx) place = &b;
+    }
+    if (place && idle < kPoolCap) {
+      *place = PooledBundle{ctx_, kind_, main_, stream, {ev[0], ev[1], ev[2]}, ++g_pool_tick};
       stream = nullptr;
       return;
     }

@@ -73,12 +73,14 @@ constexpr size_t kPanelGridScratch = 176u * 1024u;
 
 // A side stream with three events, leased from a pool shared by all threads
 // (creating and destroying a stream and its events costs 70 - 180 us per call,
-// more than the work of a small solve).  At most 32 idle bundles per device
-// and kind are kept, the rest is destroyed on return.  A returned stream may
-// still have queued work: the next user's work runs after it, which is an
-// ordering only (every lease is joined into its caller's stream).  While
-// `main` is being captured a bundle is created for the call and destroyed with
-// it, so that no stream of the pool ever belongs to a capture.
+// more than the work of a small solve).  At most 32 idle bundles per context and
+// kind are kept, the rest is destroyed on return.  A bundle goes back to the
+// caller's stream it last served, whose later work is behind the bundle's
+// anyway; a stream without one gets a new bundle, or from 4 idle ones on the
+// one that was returned first: that one may still be working for another stream,
+// which orders the new work behind it and nothing more.  While `main` is being
+// captured a bundle is created for the call and destroyed with it, so that no
+// stream of the pool ever belongs to a capture.
 struct StreamLease {
   enum Kind { kNormal = 0, kHigh = 1, kLow = 2 };  // stream priority
   cudaStream_t stream = nullptr;
@@ -91,8 +93,9 @@ struct StreamLease {
 
  private:
   void release();
-  int dev_ = -1, kind_ = 0;
-  bool pooled_ = false;
+  unsigned long long ctx_ = 0;  // 0: not of the pool
+  int kind_ = 0;
+  cudaStream_t main_ = nullptr;
 };
 
 // A side stream forked from ctx.stream (fork()) and joined back into it
