@@ -445,12 +445,17 @@ class BEMHMatrices:
             # blocks (one CTA per block, 1.1 ms at 3600 faces)
             cur = torch.cuda.current_stream()
             sides = [torch.cuda.Stream() for _ in range(4)]
-            for w, (h, s) in enumerate(zip(self.H, sides)):
-                s.wait_stream(cur)
-                with torch.cuda.stream(s):
-                    h.compress_green(self.g, enei, w, fetch=False)
-            for s in sides:
-                cur.wait_stream(s)
+            try:
+                for w, (h, s) in enumerate(zip(self.H, sides)):
+                    s.wait_stream(cur)
+                    with torch.cuda.stream(s):
+                        h.compress_green(self.g, enei, w, fetch=False)
+            except BaseException:
+                self.H = None  # its memory is free for work behind the fills already queued
+                raise
+            finally:
+                for s in sides:
+                    cur.wait_stream(s)
             for h in self.H:
                 h.fetch_ranks()
             self.enei = enei
