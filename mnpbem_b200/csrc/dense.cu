@@ -3172,8 +3172,6 @@ static int inverse_gj(const LaContext& ctx, int n, float2* M, long long ld, floa
     BEM_LAUNCH_CHECK();
     gj_step_kernel<<<dim3(2 * blocks, ceil_div(blocks, kGjCluster) * kGjCluster), 256, kGjSmem, ctx.stream>>>(n, k0, M, ld, nn, rowk, colt);
     BEM_LAUNCH_CHECK();
-    count_launch();
-    count_launch();
   }
   return BEM200_OK;
 }
@@ -3224,7 +3222,6 @@ static int inverse_nopiv_rec(const LaContext& ctx, int n, C* M, long long ld, C*
   if (n <= kInvLeaf) {
     inv_leaf_kernel<C><<<1, kInvLeafThreads, 0, ctx.stream>>>(n, M, ld, (R_t<C>)ctx.pivot_tau, vflag);
     BEM_LAUNCH_CHECK();
-    count_launch();
     return BEM200_OK;
   }
   if constexpr (sizeof(C) == 8)
