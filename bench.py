@@ -362,7 +362,7 @@ def roofline_gemm(dev):
     # bytes the three kernels move once: operands read, 14 residue planes of A, B and C written and
     # read, C written
     traffic = 8.0 * (m * k + k * n + m * n) + 28.0 * (m * k + k * n + m * n)
-    return {"kernel": "rns_gemm_kernel (+ rns_split, rns_merge)", "bound": "tensor", "achieved": round(achieved, 2),
+    return {"kernel": "rns_gemm_kernel (+ rns_balance, rns_split, rns_merge)", "bound": "tensor", "achieved": round(achieved, 2),
             "peak": peak, "peak_source": src, "unit": "TFLOP/s", "frac": round(achieved / peak, 4),
             "traffic": traffic, "traffic_source": "operand, residue-plane and result bytes, each written and read once",
             "algorithmic_flops_per_launch": 8.0 * m * n * k, "shape": [m, n, k], "ms_per_launch": round(1e3 * t, 3),

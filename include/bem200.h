@@ -342,8 +342,9 @@ int bem200_bem_init(int precision, int engine, int n, void* ws, int eps_per_face
  * BEM200_INIT_REPAIR (with DIAGONAL_PIVOTS, precision 0 or 1, info_host given):
  * when G1 and G2 passed their checks and only Delta or Sigma needs row
  * exchanges, that part alone is built again with partial pivoting inside the
- * call, which then returns BEM200_OK with *info_host = -BEM200_ERR_PIVOTING
- * (the factors are partial pivoting's throughout).
+ * call, which then returns BEM200_OK with *info_host = -BEM200_ERR_PIVOTING.
+ * The LU factors are partial pivoting's throughout; precision 1 keeps a
+ * Delta^-1 that passed its probe.
  * phase_ms (HOST, 4 floats, or NULL): stage timer (CUDA events on the
  * stream; the call then synchronises): LU(G1) || LU(G2) with Sigma1 || Sigma2,
  * LU(Delta), Delta^-1, Sigma build + LU(Sigma). */
